@@ -552,7 +552,7 @@ int jfli_power_spectrum(void* stream, const float* mesh, const float* kedges, in
   const float box[3] = {lx, ly, lz};
   const float norm = 1.0f / ((float)nx * (float)ny * (float)nz);
   cudaError_t e = jfli::power_partials(mesh, spec, partials, d, kedges, nedges, box, norm, s);
-  if (e == cudaSuccess) e = jfli::power_finalize(partials, jfli::x_pass_ctas(d), nedges + 1, out, batch, s);
+  if (e == cudaSuccess) e = jfli::power_finalize(partials, jfli::pk_ctas(d), nedges + 1, out, batch, s);
   return cuda_status(e, err, errlen, "jfli_power_spectrum");
 }
 
@@ -930,7 +930,7 @@ int jfli_power_spectrum_noalloc(void* stream, const float* mesh, const float* ke
   if (!(lx > 0 && ly > 0 && lz > 0)) return fail(err, errlen, JFLI_EINVAL, "box sizes must be positive");
   const MeshDims d{nx, ny, nz, batch};
   const size_t spec = spec_bytes(d);
-  const size_t partials = align256((size_t)jfli::noalloc_pk_ctas(d) * batch * 3 * (nedges + 1) * sizeof(double));
+  const size_t partials = align256((size_t)jfli::noalloc_x_pass_ctas(d) * batch * 3 * (nedges + 1) * sizeof(double));
   const size_t cap = jfli::noalloc_scratch_bytes();
   if (spec + partials > cap)
     return fail(err, errlen, JFLI_EUNSUPPORTED,

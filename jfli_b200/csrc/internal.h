@@ -19,7 +19,8 @@ struct MeshDims {
 // ---- fft.cu ----
 bool fft_axis_supported(int n);
 bool mesh_fft_supported(int nx, int ny, int nz);
-int x_pass_ctas(const MeshDims& d);
+int x_pass_ctas(const MeshDims& d);  // tiles of the x pass (sizes the P(k) workspace)
+int pk_ctas(const MeshDims& d);      // rows of P(k) partials: CTAs of the x pass that feeds the histogram
 cudaError_t rfft3d_forward(const float* in, float2* spec, const MeshDims& d, float sub, cudaStream_t s);
 cudaError_t rfft3d_inverse(float2* spec, float* out, const MeshDims& d, float scale, cudaStream_t s);
 cudaError_t rfft2d_forward(const float* in, float2* spec, const MeshDims& d, cudaStream_t s);  // d.nx == 1
@@ -156,6 +157,7 @@ cudaError_t adjoint_position(const float* disp, const float* u, const float* rho
 // P(k) whose scratch is a file-scope device array (no allocation).
 cudaError_t noalloc_scratch(void** out);
 size_t noalloc_scratch_bytes();
+int noalloc_x_pass_ctas(const MeshDims& d);
 int noalloc_pk_ctas(const MeshDims& d);
 cudaError_t power_partials_noalloc(const float* mesh, float2* spec, double* partials, const MeshDims& d,
                                    const float* kedges, int nedges, const float* box, float norm, cudaStream_t s);

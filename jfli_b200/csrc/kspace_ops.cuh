@@ -6,6 +6,7 @@
 // h/Mpc) for P(k) and initial conditions.
 #pragma once
 
+#include "binning.cuh"
 #include "common.cuh"
 
 namespace jfli {
@@ -159,77 +160,146 @@ struct IcOp {
 // ortho normalisation binned by digitize(|k|, kedges) over the full grid. The half
 // spectrum stores each mode with 0 < kz < nz/2 once for itself and its conjugate
 // partner, so those modes count twice. Sums are kept in FP64.
-struct PkOp {
-  static constexpr bool kInverse = false;
-  static constexpr bool kStore = false;
+struct PkArgs {
   int nx, ny, nz;
   const float* kedges;
   int nedges;
   float cx, cy, cz;  // 2*pi / L_i
   float norm;        // 1 / M for norm="ortho"
   double* partials;  // [batch][nctas][3][nedges+1]
-  static size_t smem_bytes(const PkOp& op) {
-    return sizeof(double) * 3 * (op.nedges + 1) + sizeof(float) * (op.nedges + 1);
+};
+
+constexpr size_t kPkHistBudget = 24u << 10;  // bytes of histogram columns (one column always fits)
+
+__host__ __device__ inline int pk_hist_columns(int nedges) {
+  return histogram_columns((size_t)(nedges + 1) * 20, kPkHistBudget);
+}
+// shared memory of the histogram, the edges and the tile's column constants
+__host__ __device__ inline size_t pk_smem_bytes(int nedges, int columns) {
+  return (size_t)pk_hist_columns(nedges) * (nedges + 1) * 20 + sizeof(float) * ((size_t)nedges + 3 * (size_t)columns) + 8;
+}
+
+// A CTA's part of the histogram: [nedges + 1][cols] sums of power and of |k| (FP64) and mode
+// counts (32 bits: a mesh has fewer than 2^32 modes), the edges, and per column of the tile
+// (ky^2, kz^2, weight).
+struct PkTile {
+  double *power, *ksum;
+  unsigned* count;
+  float *edges, *column;
+  int cols;
+
+  __device__ PkTile(const PkArgs& a, void* sm) {
+    cols = pk_hist_columns(a.nedges);
+    const size_t n = (size_t)cols * (a.nedges + 1);
+    power = reinterpret_cast<double*>(sm);
+    ksum = power + n;
+    count = reinterpret_cast<unsigned*>(ksum + n);
+    edges = reinterpret_cast<float*>(count + n);
+    column = edges + a.nedges;
   }
-  __device__ void prologue(float* smf, int) const {
-    double* bins = reinterpret_cast<double*>(smf);
-    float* edges = reinterpret_cast<float*>(bins + 3 * (nedges + 1));
-    for (int i = threadIdx.x; i < 3 * (nedges + 1); i += blockDim.x) bins[i] = 0.0;
-    for (int i = threadIdx.x; i < nedges; i += blockDim.x) edges[i] = kedges[i];
-    __syncthreads();
+  __device__ void clear(const PkArgs& a) {
+    for (int i = threadIdx.x; i < cols * (a.nedges + 1); i += blockDim.x) {
+      power[i] = 0.0;
+      ksum[i] = 0.0;
+      count[i] = 0;
+    }
+    for (int i = threadIdx.x; i < a.nedges; i += blockDim.x) edges[i] = a.kedges[i];
   }
-  __device__ float2 apply(float2 v, int kx, int ky, int kz, float* smf, int) const {
-    double* bins = reinterpret_cast<double*>(smf);
-    const float* edges = reinterpret_cast<const float*>(bins + 3 * (nedges + 1));
-    // |k| with the rounding of the reference's float32 grid: no FMA contraction, sum in
-    // x, y, z order, correctly rounded sqrt (decides the bin of modes on an edge)
-    const float ax = __fmul_rn(cx, (float)signed_freq(kx, nx));
-    const float ay = __fmul_rn(cy, (float)signed_freq(ky, ny));
-    const float az = __fmul_rn(cz, (float)signed_freq(kz, nz));
-    const float kmag = __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(ax, ax), __fmul_rn(ay, ay)), __fmul_rn(az, az)));
-    // digitize(right=False): number of edges <= kmag
-    int lo = 0, hi = nedges;
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (edges[mid] <= kmag)
-        lo = mid + 1;
-      else
-        hi = mid;
+  // tile columns c0 .. c0 + w - 1, column = ky hz + kz (one past the last has weight 0)
+  __device__ void set_columns(const PkArgs& a, int c0, int w, int ncols, int hz) {
+    for (int c = threadIdx.x; c < w; c += blockDim.x) {
+      const int col = c0 + c;
+      const int ky = col / hz, kz = col - ky * hz;
+      // |k| with the rounding of the reference's float32 grid: no FMA contraction, sum in
+      // x, y, z order, correctly rounded sqrt (decides the bin of modes on an edge)
+      const float ay = __fmul_rn(a.cy, (float)signed_freq(ky, a.ny));
+      const float az = __fmul_rn(a.cz, (float)signed_freq(kz, a.nz));
+      column[3 * c + 0] = __fmul_rn(ay, ay);
+      column[3 * c + 1] = __fmul_rn(az, az);
+      column[3 * c + 2] = col < ncols ? ((kz == 0 || 2 * kz == a.nz) ? 1.f : 2.f) : 0.f;
     }
-    const int bin = lo;
-    const double w = (kz == 0 || 2 * kz == nz) ? 1.0 : 2.0;
-    const double p = w * ((double)v.x * v.x + (double)v.y * v.y) * (double)norm;
-    const double kw = w * (double)kmag;
-    const unsigned active = __activemask();
-    const unsigned peers = __match_any_sync(active, bin);
-    const int lane = threadIdx.x & 31;
-    const int leader = __ffs(peers) - 1;
-    double sp = 0.0, sw = 0.0, sk = 0.0;
-    unsigned m = peers;
-    while (m) {
-      const int l = __ffs(m) - 1;
-      sp += __shfl_sync(peers, p, l);
-      sw += __shfl_sync(peers, w, l);
-      sk += __shfl_sync(peers, kw, l);
-      m &= m - 1;
-    }
-    if (lane == leader) {
-      atomicAdd(&bins[bin], sp);
-      atomicAdd(&bins[(nedges + 1) + bin], sw);
-      atomicAdd(&bins[2 * (nedges + 1) + bin], sk);
-    }
-    return v;
   }
-  __device__ void epilogue(float* smf, int batch, int cta, int nctas) const {
-    const double* bins = reinterpret_cast<const double*>(smf);
-    const int nb = 3 * (nedges + 1);
-    double* dst = partials + ((long long)batch * nctas + cta) * nb;
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) dst[i] = bins[i];
+  __device__ __forceinline__ float kmag(float ax2, int c) const {
+    return __fsqrt_rn(__fadd_rn(__fadd_rn(ax2, column[3 * c]), column[3 * c + 1]));
+  }
+  __device__ __forceinline__ void flush(int bin, double p, double k, unsigned n) {
+    const int i = bin * cols + ((threadIdx.x & 31) & (cols - 1));
+    atomicAdd(power + i, p);
+    atomicAdd(ksum + i, k);
+    atomicAdd(count + i, n);
+  }
+  // Bins a transformed tile buf[e * pitch + c] (element e < n of column c < w), pitch odd.
+  // The modes e and n - e have the same |k| bit for bit and are taken together. Lanes run
+  // along e (no bank conflicts); a thread walks `span` successive columns. The element
+  // e = n / 2 has no partner and would leave a row of one lane, so the lanes of the last
+  // warps take it, one column each.
+  __device__ __forceinline__ void add(const PkArgs& a, const float2* buf, int pitch, int n, int w) {
+    const int rows = (n + 1) / 2;
+    const int groups = max(1, min(w, (int)blockDim.x / rows));
+    const int span = (w + groups - 1) / groups;
+    for (int i = threadIdx.x; i < rows * groups; i += blockDim.x) {
+      const int grp = i / rows, e = i - grp * rows;
+      const float ax = __fmul_rn(a.cx, (float)e), ax2 = __fmul_rn(ax, ax);
+      const float2* lower = buf + e * pitch;
+      const float2* upper = buf + (n - e) * pitch;  // read only when e > 0
+      BinCursor cur;
+      double p = 0.0, ks = 0.0;
+      unsigned cnt = 0;
+      const int c1 = min(w, (grp + 1) * span);
+      for (int c = grp * span; c < c1; ++c) {
+        const float wt = column[3 * c + 2];
+        if (wt == 0.f) break;
+        const float k = kmag(ax2, c);
+        if (!cur.holds(k)) {
+          if (cnt) flush(cur.bin, p * (double)a.norm, ks, cnt);
+          cur.move(k, edges, a.nedges);
+          p = ks = 0.0;
+          cnt = 0;
+        }
+        const float2 f = lower[c];
+        double q = (double)f.x * f.x + (double)f.y * f.y;
+        float m = wt;
+        if (e > 0) {
+          const float2 g = upper[c];
+          q += (double)g.x * g.x + (double)g.y * g.y;
+          m += wt;
+        }
+        p += (double)wt * q;
+        ks += (double)m * (double)k;
+        cnt += (unsigned)m;
+      }
+      if (cnt) flush(cur.bin, p * (double)a.norm, ks, cnt);
+    }
+    if ((n & 1) == 0) {
+      const int c = (int)blockDim.x - 1 - (int)threadIdx.x;
+      if (c < w && column[3 * c + 2] > 0.f) {
+        const float wt = column[3 * c + 2];
+        const float ax = __fmul_rn(a.cx, (float)(n / 2));
+        const float k = kmag(__fmul_rn(ax, ax), c);
+        const float2 f = buf[(n / 2) * pitch + c];
+        flush(digitize(k, edges, a.nedges), (double)wt * ((double)f.x * f.x + (double)f.y * f.y) * (double)a.norm,
+              (double)wt * (double)k, (unsigned)wt);
+      }
+    }
+  }
+  // the CTA's sums, columns added in order; called after a barrier
+  __device__ void store(const PkArgs& a, int batch, int cta, int nctas) {
+    const int nb = a.nedges + 1;
+    double* dst = a.partials + ((long long)batch * nctas + cta) * 3 * nb;
+    for (int i = threadIdx.x; i < 3 * nb; i += blockDim.x) {
+      const int q = i / nb, bin = i - q * nb;
+      double s = 0.0;
+      for (int c = 0; c < cols; ++c) {
+        const int at = bin * cols + c;
+        s += q == 0 ? power[at] : (q == 1 ? (double)count[at] : ksum[at]);
+      }
+      dst[i] = s;
+    }
   }
 };
 
 // Adjoint of P(k) with respect to the mesh: mode k is scaled by weights[bin(k)] * norm,
-// bin(k) = digitize(|k|, kedges) with the same |k| rounding as PkOp, so that the inverse
+// bin(k) = digitize(|k|, kedges) with the same |k| rounding as the histogram, so that the inverse
 // transform gives dL/dmesh = sum over bins of dL/dP_b * dP_b/dmesh when
 // weights[b] = 2 * dL/dP_b * prod(L/N) / count_b (0 for the dropped under/overflow bins).
 // L_l(mu) by the reference's recurrence, in FP32 (the multipole weights (2l + 1) L_l(mu) of

@@ -7,7 +7,7 @@
 // every element with 0 < kz < nz/2 also adds its conjugate partner (-k; for real meshes
 // F(-k) = conj F(k)) with the partner's own wavevector, so the sums are those of the full
 // grid, odd multipoles and imaginary parts included. |k| and the bin are formed as the
-// monopole kernel forms them (kspace_ops.cuh PkOp); mu with the reference's float32 order
+// monopole kernel forms them (kspace_ops.cuh PkTile); mu with the reference's float32 order
 // (x, y, z products summed, then divided by |k|); L_l by the reference's recurrence in FP32.
 // Per-CTA FP64 sums: [2 nell + 2][nedges + 1] = for each l (Re, Im), then mode count, sum |k|.
 #include "common.cuh"
