@@ -15,6 +15,8 @@ import pytest
 import torch
 
 from jfli_b200 import ops
+from jfli_b200.power import power_poles
+from oracle import pm as opm
 
 pytestmark = pytest.mark.gpu
 
@@ -53,3 +55,27 @@ def test_power_sums_match_full_grid(shape, nedges, batch):
         np.testing.assert_array_equal(got[b, 1], ref[1])
         np.testing.assert_allclose(got[b, 2], ref[2], rtol=1e-12)
         np.testing.assert_allclose(got[b, 0], ref[0], rtol=2e-5)
+
+
+@pytest.mark.parametrize("shape,poles,cross,nedges", [
+    ((32, 24, 36), (0, 1, 2, 3, 4, 5, 6, 7), True, 9), ((27, 18, 16), (3,), False, 5), ((16, 16, 16), (0, 2, 4), True, 60),
+    ((6, 81, 8), (1, 2), True, 4), ((64, 64, 12), (16, 0), False, 12), ((2, 4, 64), (2, 1, 0), True, 500),
+])
+def test_power_poles_match_oracle(shape, poles, cross, nedges):
+    """Every multipole count, odd and Nyquist-plane modes, an oblique line of sight. FP32 mu and
+    L_l weights (up to (2l + 1) |L_l| rounding, 2e-6 at l = 16) on FP32 transforms: 1e-4 of the
+    bin's monopole, the parity tests' bound."""
+    rng = np.random.default_rng(sum(shape))
+    a = rng.standard_normal(shape).astype(np.float32)
+    b = (0.5 * a + rng.standard_normal(shape)).astype(np.float32) if cross else None
+    box = tuple(2.7 * n for n in shape)
+    edges = np.linspace(0.037, 1.9, nedges)
+    los = (0.3, -0.5, 0.8)
+    k, pk = power_poles(torch.as_tensor(a, device="cuda"), None if b is None else torch.as_tensor(b, device="cuda"),
+                           box, edges, poles, los)
+    kr, pr = opm.power_poles(a, b, box, edges, poles, los)
+    scale = np.abs(opm.power_poles(a, None, box, edges, 0)[1])
+    if cross:
+        scale = np.maximum(scale, np.abs(opm.power_poles(b, None, box, edges, 0)[1]))
+    np.testing.assert_allclose(k.cpu().numpy(), kr, rtol=1e-6)
+    assert np.all(np.abs(np.atleast_2d(pk.cpu().numpy()) - np.atleast_2d(pr)) <= 1e-4 * scale)
