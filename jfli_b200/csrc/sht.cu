@@ -1,167 +1,440 @@
-// Legendre stages of the spherical harmonic transform of HEALPix ring maps (FP64), the
-// O(lmax^2 x rings) part of healpy's anafast (reference _src/power/_compute.py:175-191).
-// The ring FFTs along phi run on the host; these kernels take and return per-ring Fourier
-// coefficients F[r][m] (m = 0..lmax, phase e^{-i m phi_0} applied).
+// Spherical harmonic transform of HEALPix ring maps (FP64), the two stages of healpy's
+// anafast (reference _src/power/_compute.py:175-191): the ring transforms along phi, which
+// take a map to per-ring Fourier coefficients F[r][m] (m = 0..lmax, phase e^{-i m phi_0}
+// applied) and back, and the O(lmax^2 x rings) Legendre stages between F and a_lm:
 //
 //   analysis:  a_lm  = w * sum_r lambda_lm(theta_r) F[r][m]
 //   synthesis: G[r][m] = sum_l a_lm lambda_lm(theta_r)
 //
 // lambda_lm are the orthonormal associated Legendre functions with the Condon-Shortley
-// phase: lambda_mm = (-1)^m sqrt((2m+1)/(4 pi) (2m)!/(4^m (m!)^2)) sin^m theta, then the
-// three-term recursion in l. lambda_mm is formed in log space; where it is below FP64
-// range the recursion runs on values scaled by e^s and drops the scale as they grow
-// (factor 1e100 at a time), so that rings where lambda_lm becomes significant before lmax
-// are not lost to underflow. a_lm is packed by m: a[m][l - m], offset m (lmax + 1) - m (m - 1) / 2.
+// phase. a_lm is packed by m: a[m][l - m], offset m (lmax + 1) - m (m - 1) / 2.
+#include <type_traits>
+
 #include "common.cuh"
 #include "internal.h"
 
 namespace jfli {
 
-constexpr int kShtThreads = 128;
-constexpr int kShtLTile = 16;
-// row stride of the per-tile contributions (one row per l): one element of padding so that
-// the reduction's lanes, which read one element per row, fall in different banks
-constexpr int kShtRow = kShtThreads + 1;
-
 __host__ __device__ __forceinline__ long long alm_offset(int m, int lmax) {
   return (long long)m * (lmax + 1) - (long long)m * (m - 1) / 2;
 }
 
-struct LegendreState {
-  double prev, cur, scale, escale;
+__device__ __forceinline__ double2 zadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 zsub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ double2 zmul(double2 a, double2 b) {
+  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+__device__ __forceinline__ double2 zconj(double2 a) { return make_double2(a.x, -a.y); }
+
+// ---- Legendre stages ----------------------------------------------------------------
+//
+// Both are FP64-arithmetic bound (a B200 SM issues 64 FP64 FMAs a clock). Per (l, m) and ring
+// the least is the recursion step and two multiply-adds of the sum, and two properties cut
+// the rings and the step to their least form:
+//   * lambda_lm(pi - theta) = (-1)^(l+m) lambda_lm(theta): a ring and its mirror image take one
+//     recursion, on the sum (l - m even) or difference (odd) of their coefficients.
+//   * with lambda_l = alpha_l mu_l, alpha_l = (a_l / a_(l-1)) alpha_(l-2) and a_l = sqrt((4 l^2
+//     - 1) / (l^2 - m^2)), the three-term recursion lambda_l = a_l (z lambda_(l-1) -
+//     lambda_(l-2) / a_(l-1)) becomes mu_l = (A_l z) mu_(l-1) - mu_(l-2), A_l = a_(l-1)
+//     alpha_(l-1) / alpha_(l-2): one multiplication and one FMA per ring. alpha stays within
+//     about [0.1, 1] and multiplies the finished sums (analysis) or a_lm (synthesis).
+// So a pair of rings costs 4 FP64 instructions per l. A thread keeps RP pairs in registers
+// (independent chains cover the FP64 latency), a CTA holds one m and up to 32 RP pairs per
+// warp, with successive rings in a warp.
+//
+// Where lambda_mm underflows the recursion runs on values scaled by 2^(400 k) and k drops as
+// they grow; a ring adds to the sums only at k = 0 (below, its lambda is under 2^-140). The
+// scale is looked at every 8 l, over which a value grows by less than 2^60.
+//
+// The tables of one m (A_l and alpha_l for 32 l at a time) are made by one warp while the
+// others use the previous ones: a prefix product over lanes of equal parity.
+//
+// 1 B200, nside 1024, lmax 3000 (8190 x 4.5M (ring, l, m)): analysis 31.9 -> 6.9 ms, synthesis
+// 19.4 -> 5.3 ms against one ring per thread with a three-multiplication recursion and, in the
+// analysis, one shared-memory reduction per ring and l; FP64 floor of the form above 2.1 ms.
+constexpr int kLTile = 32;    // l per table
+constexpr int kLChunk = 8;    // l between looks at the scale
+constexpr int kScaleBits = 400;
+
+struct LegendreTables {
+  double A[2][kLTile], alpha[2][kLTile];
 };
 
-// lambda_mm for one ring (scaled), and e^-scale.
-__device__ __forceinline__ LegendreState legendre_start(int m, double z) {
-  const double logc = 0.5 * log((2.0 * m + 1.0) / (4.0 * 3.14159265358979323846)) +
-                      0.5 * (lgamma(2.0 * m + 1.0) - 2.0 * lgamma(m + 1.0) - m * log(4.0));
-  const double s2 = 1.0 - z * z;
-  LegendreState st;
-  const double logv = (m == 0) ? logc : logc + 0.5 * m * log(s2);
-  st.scale = (logv < -600.0) ? (-300.0 - logv) : 0.0;
-  const double sign = (m & 1) ? -1.0 : 1.0;
-  st.cur = sign * exp(logv + st.scale);
-  st.prev = 0.0;
-  st.escale = (st.scale == 0.0) ? 1.0 : (st.scale < 745.0 ? exp(-st.scale) : 0.0);
-  return st;
+// a_l of the recursion (l > m)
+__device__ __forceinline__ double legendre_a(int l, int m) {
+  const double d = (double)l;
+  return sqrt((4.0 * d * d - 1.0) / ((double)(l - m) * (double)(l + m)));
 }
 
-// Advance to l (>= m + 1) with the recursion coefficients of (l, m); returns lambda_lm.
-__device__ __forceinline__ double legendre_step(LegendreState& st, double z, double a, double b) {
-  double nxt = a * (z * st.cur - b * st.prev);
-  if (st.scale > 0.0 && fabs(nxt) > 1e100) {
-    nxt *= 1e-100;
-    st.cur *= 1e-100;
-    st.scale -= 230.25850929940458;  // ln 1e100
-    st.escale = (st.scale < 745.0) ? exp(-st.scale) : 0.0;
+// Tables of l = l0 .. l0 + 31 (one warp, lane = l - l0; l0 - m is a multiple of 32). c0 and c1
+// carry alpha of the last two l across tables.
+__device__ __forceinline__ void legendre_tables(LegendreTables& t, int buf, int l0, int m, double& c0, double& c1) {
+  const int lane = threadIdx.x & 31;
+  const int l = l0 + lane;
+  const double al = l > m ? legendre_a(l, m) : 1.0;
+  const double ap = l > m + 1 ? legendre_a(l - 1, m) : 1.0;
+  // alpha_m = alpha_(m+1) = 1
+  double alpha = l > m + 1 ? al / ap : 1.0;
+  if (lane < 2) alpha *= lane == 0 ? c0 : c1;
+#pragma unroll
+  for (int off = 2; off < 32; off <<= 1) {
+    const double v = __shfl_up_sync(0xffffffffu, alpha, off);
+    if (lane >= off) alpha *= v;
   }
-  st.prev = st.cur;
-  st.cur = nxt;
-  return nxt * st.escale;
-}
-
-// recursion coefficients for l of a tile (a_l, b_l; l = m + 1 uses a = sqrt(2m+3), b = 0)
-__device__ __forceinline__ void legendre_coeffs(int l, int m, double& a, double& b) {
-  if (l == m + 1) {
-    a = sqrt(2.0 * m + 3.0);
-    b = 0.0;
-  } else {
-    const double ll = (double)l, mm = (double)m;
-    a = sqrt((4.0 * ll * ll - 1.0) / (ll * ll - mm * mm));
-    b = sqrt(((ll - 1.0) * (ll - 1.0) - mm * mm) / (4.0 * (ll - 1.0) * (ll - 1.0) - 1.0));
+  double p1 = __shfl_up_sync(0xffffffffu, alpha, 1), p2 = __shfl_up_sync(0xffffffffu, alpha, 2);
+  if (lane == 0) {
+    p1 = c1;
+    p2 = c0;
+  } else if (lane == 1) {
+    p2 = c1;
   }
+  t.A[buf][lane] = l > m + 1 ? ap * p1 / p2 : al;  // lambda_(m+1) = a_(m+1) z lambda_mm
+  t.alpha[buf][lane] = alpha;
+  c0 = __shfl_sync(0xffffffffu, alpha, 30);
+  c1 = __shfl_sync(0xffffffffu, alpha, 31);
 }
 
-__global__ void __launch_bounds__(kShtThreads) k_sht_analysis(const double2* __restrict__ F, const double* __restrict__ z,
-                                                               int nrings, int lmax, double w, double2* __restrict__ alm) {
-  extern __shared__ double2 contrib[];  // [kShtLTile][kShtRow]
-  __shared__ double coef[2][kShtLTile];
-  __shared__ double2 part[kShtThreads / kShtLTile][kShtLTile];
-  const int m = blockIdx.y;
-  const int r = blockIdx.x * kShtThreads + threadIdx.x;
-  const bool active = r < nrings;
-  const double zr = active ? z[r] : 0.0;
-  const double2 f = active ? F[(long long)r * (lmax + 1) + m] : make_double2(0.0, 0.0);
-  LegendreState st = legendre_start(m, active ? zr : 0.0);
+// ln of the normalisation of lambda_mm without its sign: ln sqrt((1 / 4 pi) prod_(k=1..m) (2k
+// + 1) / 2k), summed over the CTA's threads in a fixed order.
+__device__ __forceinline__ double legendre_lognorm(int m, double* scratch) {
+  double s = 0.0;
+  for (int k = 1 + threadIdx.x; k <= m; k += blockDim.x) s += log1p(0.5 / (double)k);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
+  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = s;
+  __syncthreads();
+  s = 0.0;
+  for (int w = 0; w < (int)blockDim.x / 32; ++w) s += scratch[w];
+  __syncthreads();
+  return 0.5 * (s - 2.5310242469692907);  // ln 4 pi
+}
+
+// One ring (pair) of a thread: z, the last two mu, and the scale k (see above).
+struct LegendreRing {
+  double z, prev, cur;
+  int k;
+
+  __device__ __forceinline__ void start(int m, double zr, double lognorm) {
+    z = zr;
+    prev = 0.0;
+    const double s2 = (1.0 - zr) * (1.0 + zr);
+    const double v = m == 0 ? lognorm : lognorm + 0.5 * m * log(s2);  // s2 = 0: -inf, lambda = 0
+    const double step = kScaleBits * 0.69314718055994530942;
+    k = v < -0.5 * step ? (int)fmin(1e6, ceil((-0.5 * step - v) / step)) : 0;
+    cur = exp(v + k * step);
+    if (m & 1) cur = -cur;
+  }
+  __device__ __forceinline__ void rescale() {
+    if (k > 0 && fabs(cur) > 0x1p200) {
+      cur *= 0x1p-400;
+      prev *= 0x1p-400;
+      --k;
+    }
+  }
+  // (cur, prev) <- (A z cur - prev, cur)
+  __device__ __forceinline__ void step(double A) {
+    const double n = fma(A * z, cur, -prev);
+    prev = cur;
+    cur = n;
+  }
+};
+
+// Ring pairs of a CTA: pair p is rings p and nrings - 1 - p (the same ring in the middle).
+// z need not be mirror symmetric: a CTA that finds a pair whose z differ from mirror images by
+// more than rounding takes the two hemispheres one after the other instead.
+struct RingPairs {
+  int nrings, pairs;
+  __device__ __forceinline__ bool mirrored(const double* z, int first, int n) const {
+    bool ok = true;
+    for (int p = first + threadIdx.x; p < min(pairs, first + n); p += blockDim.x)
+      ok = ok && fabs(z[p] + z[nrings - 1 - p]) <= 4e-16;
+    return __syncthreads_and(ok);
+  }
+};
+
+constexpr int kLegendreThreads = 256;  // at most
+
+// Analysis: a thread's sums over its pairs of one l go through shared memory: the lanes of a
+// warp first halve (re in lanes 0..15, im in 16..31), 32 l are collected per warp and lane j
+// adds up row j, so the reduction over a warp's rings costs a few instructions per l.
+template <int RP>
+__global__ void __launch_bounds__(kLegendreThreads) k_sht_analysis(const double2* __restrict__ F,
+                                                                   const double* __restrict__ z, int nrings, int lmax,
+                                                                   double w, double2* __restrict__ alm) {
+  __shared__ LegendreTables tab;
+  __shared__ double2 part[kLegendreThreads / 32][kLTile];
+  extern __shared__ double rows[];  // per warp [32 l][33]
+  const int m = blockIdx.x;
+  const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double* row = rows + (size_t)warp * kLTile * 33;
+  const RingPairs rp{nrings, (nrings + 1) / 2};
+  const int first = blockIdx.y * (blockDim.x * RP);
+  const bool mirror = rp.mirrored(z, first, blockDim.x * RP);
+  const double lognorm = legendre_lognorm(m, &part[0][0].x);
   const long long off = alm_offset(m, lmax);
-  for (int l0 = m; l0 <= lmax; l0 += kShtLTile) {
-    if (threadIdx.x < kShtLTile) {
-      const int l = l0 + threadIdx.x;
-      double a = 0.0, b = 0.0;
-      if (l > m && l <= lmax) legendre_coeffs(l, m, a, b);
-      coef[0][threadIdx.x] = a;
-      coef[1][threadIdx.x] = b;
-    }
-    __syncthreads();
-    for (int t = 0; t < kShtLTile; ++t) {
-      const int l = l0 + t;
-      double lam = 0.0;
-      if (l == m)
-        lam = st.cur * st.escale;
-      else if (l <= lmax)
-        lam = legendre_step(st, zr, coef[0][t], coef[1][t]);
-      contrib[t * kShtRow + threadIdx.x] = active ? make_double2(lam * f.x, lam * f.y) : make_double2(0.0, 0.0);
-    }
-    __syncthreads();
-    {  // thread (q, row): sum of kShtLTile rings of one l
-      const int row = threadIdx.x & (kShtLTile - 1), q = threadIdx.x / kShtLTile;
-      double sx = 0.0, sy = 0.0;
-      for (int i = 0; i < kShtLTile; ++i) {
-        const double2 c = contrib[row * kShtRow + q * kShtLTile + i];
-        sx += c.x;
-        sy += c.y;
-      }
-      part[q][row] = make_double2(sx, sy);
-    }
-    __syncthreads();
-    if (threadIdx.x < kShtLTile) {
-      const int l = l0 + threadIdx.x;
-      if (l <= lmax) {
-        double sx = 0.0, sy = 0.0;
-        for (int q = 0; q < kShtThreads / kShtLTile; ++q) {
-          sx += part[q][threadIdx.x].x;
-          sy += part[q][threadIdx.x].y;
+  const long long fs = lmax + 1;
+  for (int hemi = 0; hemi < (mirror ? 1 : 2); ++hemi) {
+    LegendreRing r[RP];
+    double2 even[RP], odd[RP];
+#pragma unroll
+    for (int j = 0; j < RP; ++j) {
+      const int p = first + warp * (32 * RP) + 32 * j + lane;
+      const int q = nrings - 1 - p;
+      even[j] = odd[j] = make_double2(0.0, 0.0);
+      double zr = 0.0;
+      if (p < rp.pairs && !(hemi == 1 && p == q)) {
+        if (mirror) {
+          const double2 a = F[p * fs + m], b = p == q ? make_double2(0.0, 0.0) : F[q * fs + m];
+          even[j] = zadd(a, b);
+          odd[j] = zsub(a, b);
+          zr = p == q ? z[p] : 0.5 * (z[p] - z[q]);
+        } else {
+          const int ring = hemi == 0 ? p : q;
+          even[j] = odd[j] = F[ring * fs + m];
+          zr = z[ring];
         }
-        atomicAdd(&alm[off + (l - m)].x, w * sx);
-        atomicAdd(&alm[off + (l - m)].y, w * sy);
+      }
+      r[j].start(m, zr, lognorm);
+    }
+    // 0, or NaN where a ring's coefficients are not finite: what a ring adds before its lambda counts
+    double poison = 0.0;
+    {
+      double px = 0.0, py = 0.0;
+#pragma unroll
+      for (int j = 0; j < RP; ++j) {
+        px += 0.0 * even[j].x + 0.0 * odd[j].x;
+        py += 0.0 * even[j].y + 0.0 * odd[j].y;
+      }
+      poison = (lane < 16 ? px : py) + __shfl_xor_sync(0xffffffffu, lane < 16 ? py : px, 16);
+    }
+    const bool poisoned = __any_sync(0xffffffffu, !(poison == 0.0));
+    double c0 = 1.0, c1 = 1.0;  // used by the warp whose turn it is; handed on through shared memory
+    __shared__ double carry[2];
+    if (warp == 0) {
+      legendre_tables(tab, 0, m, m, c0, c1);
+      if (lane == 0) {
+        carry[0] = c0;
+        carry[1] = c1;
       }
     }
     __syncthreads();
+    int buf = 0;
+    for (int l0 = m; l0 <= lmax; l0 += kLTile, buf ^= 1) {
+      // the next table, by a warp that changes with the table
+      if (l0 + kLTile <= lmax && warp == ((l0 - m) / kLTile + 1) % warps) {
+        c0 = carry[0];
+        c1 = carry[1];
+        __syncwarp();
+        legendre_tables(tab, buf ^ 1, l0 + kLTile, m, c0, c1);
+        if (lane == 0) {
+          carry[0] = c0;
+          carry[1] = c1;
+        }
+      }
+      bool any = poisoned;
+      for (int t0 = 0; t0 < kLTile; t0 += kLChunk) {
+        int scaled = 0;
+#pragma unroll
+        for (int j = 0; j < RP; ++j) {
+          r[j].rescale();
+          scaled += r[j].k > 0;
+        }
+        const bool all_on = __all_sync(0xffffffffu, scaled == 0);
+        const bool none_on = __all_sync(0xffffffffu, scaled == RP);
+        if (!none_on) any = true;
+        auto chunk = [&](auto masked) {
+          double on[RP];
+          if constexpr (masked) {
+#pragma unroll
+            for (int j = 0; j < RP; ++j) on[j] = r[j].k == 0 ? 1.0 : 0.0;
+          }
+#pragma unroll
+          for (int t = 0; t < kLChunk; ++t) {
+            const int l = l0 + t0 + t;
+            double re = 0.0, im = 0.0;
+#pragma unroll
+            for (int j = 0; j < RP; ++j) {
+              if (l > m) r[j].step(tab.A[buf][t0 + t]);
+              double v = r[j].cur;
+              if constexpr (masked) v *= on[j];
+              const double2 f = (t & 1) ? odd[j] : even[j];
+              re = fma(v, f.x, re);
+              im = fma(v, f.y, im);
+            }
+            // lanes 0..15 take re, 16..31 im
+            const double give = lane < 16 ? im : re, keep = lane < 16 ? re : im;
+            row[(t0 + t) * 33 + lane] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+          }
+        };
+        if (all_on) {
+          chunk(std::false_type{});
+        } else if (!none_on) {
+          chunk(std::true_type{});
+        } else {  // nothing to add yet
+#pragma unroll
+          for (int t = 0; t < kLChunk; ++t) {
+#pragma unroll
+            for (int j = 0; j < RP; ++j)
+              if (l0 + t0 + t > m) r[j].step(tab.A[buf][t0 + t]);
+            row[(t0 + t) * 33 + lane] = poison;
+          }
+        }
+      }
+      __syncwarp();
+      double sx = 0.0, sy = 0.0;
+      if (any) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          sx += row[lane * 33 + i];
+          sy += row[lane * 33 + 16 + i];
+        }
+      }
+      part[warp][lane] = make_double2(sx, sy);
+      __syncthreads();
+      if (threadIdx.x < kLTile) {
+        const int l = l0 + threadIdx.x;
+        if (l <= lmax) {
+          double2 s = make_double2(0.0, 0.0);
+          for (int i = 0; i < warps; ++i) s = zadd(s, part[i][threadIdx.x]);
+          const double f = w * tab.alpha[buf][threadIdx.x];
+          double2* dst = alm + off + (l - m);
+          if (gridDim.y > 1) {
+            atomicAdd(&dst->x, f * s.x);
+            atomicAdd(&dst->y, f * s.y);
+          } else if (hemi == 0) {
+            *dst = make_double2(f * s.x, f * s.y);
+          } else {
+            *dst = make_double2(dst->x + f * s.x, dst->y + f * s.y);
+          }
+        }
+      }
+      __syncthreads();
+    }
   }
 }
 
-__global__ void __launch_bounds__(kShtThreads) k_sht_synthesis(const double2* __restrict__ alm,
-                                                                const double* __restrict__ z, int nrings, int lmax,
-                                                                double2* __restrict__ G) {
-  __shared__ double coef[2][kShtLTile];
-  __shared__ double2 a_tile[kShtLTile];
-  const int m = blockIdx.y;
-  const int r = blockIdx.x * kShtThreads + threadIdx.x;
-  const bool active = r < nrings;
-  const double zr = active ? z[r] : 0.0;
-  LegendreState st = legendre_start(m, zr);
-  const long long off = alm_offset(m, lmax);
-  double gx = 0.0, gy = 0.0;
-  for (int l0 = m; l0 <= lmax; l0 += kShtLTile) {
-    if (threadIdx.x < kShtLTile) {
-      const int l = l0 + threadIdx.x;
-      double a = 0.0, b = 0.0;
-      if (l > m && l <= lmax) legendre_coeffs(l, m, a, b);
-      coef[0][threadIdx.x] = a;
-      coef[1][threadIdx.x] = b;
-      a_tile[threadIdx.x] = (l <= lmax) ? alm[off + (l - m)] : make_double2(0.0, 0.0);
+template <int RP>
+__global__ void __launch_bounds__(kLegendreThreads) k_sht_synthesis(const double2* __restrict__ alm,
+                                                                    const double* __restrict__ z, int nrings, int lmax,
+                                                                    double2* __restrict__ G) {
+  __shared__ LegendreTables tab;
+  __shared__ double2 a_tile[2][kLTile];  // alpha_l a_lm
+  __shared__ double scratch[kLegendreThreads / 32];
+  const int m = blockIdx.x;
+  const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const RingPairs rp{nrings, (nrings + 1) / 2};
+  const int first = blockIdx.y * (blockDim.x * RP);
+  const bool mirror = rp.mirrored(z, first, blockDim.x * RP);
+  const double lognorm = legendre_lognorm(m, scratch);
+  const double2* a = alm + alm_offset(m, lmax);
+  const long long fs = lmax + 1;
+  for (int hemi = 0; hemi < (mirror ? 1 : 2); ++hemi) {
+    LegendreRing r[RP];
+    double2 even[RP], odd[RP];
+#pragma unroll
+    for (int j = 0; j < RP; ++j) {
+      const int p = first + warp * (32 * RP) + 32 * j + lane;
+      const int q = nrings - 1 - p;
+      double zr = 0.0;
+      if (p < rp.pairs) zr = mirror ? (p == q ? z[p] : 0.5 * (z[p] - z[q])) : z[hemi == 0 ? p : q];
+      even[j] = odd[j] = make_double2(0.0, 0.0);
+      r[j].start(m, zr, lognorm);
     }
+    __shared__ double carry[2];
+    auto table = [&](int buf, int l0) {
+      double c0 = l0 == m ? 1.0 : carry[0], c1 = l0 == m ? 1.0 : carry[1];
+      __syncwarp();
+      legendre_tables(tab, buf, l0, m, c0, c1);
+      const int l = l0 + lane;
+      const double2 v = l <= lmax ? a[l - m] : make_double2(0.0, 0.0);
+      const double f = tab.alpha[buf][lane];
+      a_tile[buf][lane] = make_double2(f * v.x, f * v.y);
+      if (lane == 0) {
+        carry[0] = c0;
+        carry[1] = c1;
+      }
+    };
+    if (warp == 0) table(0, m);
     __syncthreads();
-    for (int t = 0; t < kShtLTile; ++t) {
-      const int l = l0 + t;
-      if (l > lmax) break;
-      const double lam = (l == m) ? st.cur * st.escale : legendre_step(st, zr, coef[0][t], coef[1][t]);
-      gx += lam * a_tile[t].x;
-      gy += lam * a_tile[t].y;
+    int buf = 0;
+    for (int l0 = m; l0 <= lmax; l0 += kLTile, buf ^= 1) {
+      if (l0 + kLTile <= lmax && warp == ((l0 - m) / kLTile + 1) % warps) table(buf ^ 1, l0 + kLTile);
+      for (int t0 = 0; t0 < kLTile; t0 += kLChunk) {
+        int scaled = 0;
+#pragma unroll
+        for (int j = 0; j < RP; ++j) {
+          r[j].rescale();
+          scaled += r[j].k > 0;
+        }
+        const bool all_on = __all_sync(0xffffffffu, scaled == 0);
+        const bool none_on = __all_sync(0xffffffffu, scaled == RP);
+        auto chunk = [&](auto masked) {
+          double on[RP];
+          if constexpr (masked) {
+#pragma unroll
+            for (int j = 0; j < RP; ++j) on[j] = r[j].k == 0 ? 1.0 : 0.0;
+          }
+#pragma unroll
+          for (int t = 0; t < kLChunk; ++t) {
+            const double2 c = a_tile[buf][t0 + t];
+#pragma unroll
+            for (int j = 0; j < RP; ++j) {
+              if (l0 + t0 + t > m) r[j].step(tab.A[buf][t0 + t]);
+              double v = r[j].cur;
+              if constexpr (masked) v *= on[j];
+              double2& s = (t & 1) ? odd[j] : even[j];
+              s.x = fma(v, c.x, s.x);
+              s.y = fma(v, c.y, s.y);
+            }
+          }
+        };
+        if (all_on) {
+          chunk(std::false_type{});
+        } else if (!none_on) {
+          chunk(std::true_type{});
+        } else {
+#pragma unroll
+          for (int t = 0; t < kLChunk; ++t)
+#pragma unroll
+            for (int j = 0; j < RP; ++j)
+              if (l0 + t0 + t > m) r[j].step(tab.A[buf][t0 + t]);
+        }
+      }
+      __syncthreads();
     }
-    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < RP; ++j) {
+      const int p = first + warp * (32 * RP) + 32 * j + lane;
+      const int q = nrings - 1 - p;
+      if (p >= rp.pairs) continue;
+      const double2 sum = zadd(even[j], odd[j]);
+      if (mirror) {
+        G[p * fs + m] = sum;
+        if (q != p) G[q * fs + m] = zsub(even[j], odd[j]);
+      } else {
+        G[(hemi == 0 ? p : q) * fs + m] = sum;
+      }
+    }
   }
-  if (active) G[(long long)r * (lmax + 1) + m] = make_double2(gx, gy);
+}
+
+// Pairs per thread and threads of a CTA: a thread takes 8 pairs (8 independent recursions)
+// when that still leaves four warps, fewer for small maps, whose 3 nside CTAs would otherwise
+// hold one or two warps each.
+struct LegendreShape {
+  int rp, threads, blocks;
+};
+
+static LegendreShape legendre_shape(int nrings) {
+  const int pairs = (nrings + 1) / 2;
+  LegendreShape s;
+  s.rp = pairs >= 1024 ? 8 : (pairs >= 256 ? 4 : 2);
+  int warps = (pairs + 32 * s.rp - 1) / (32 * s.rp);
+  const int most = kLegendreThreads / 32;
+  s.blocks = (warps + most - 1) / most;
+  warps = (warps + s.blocks - 1) / s.blocks;
+  s.threads = 32 * warps;
+  return s;
 }
 
 // ---- ring transforms along phi ------------------------------------------------------
@@ -206,6 +479,7 @@ __device__ __forceinline__ double2 phase(int m, int j, int n, double phi0, doubl
   return make_double2(cs, sign * sn);
 }
 
+// Direct sums (nside > kRingFftMax):
 // F[r][m] = sum_j f_j e^{-i m phi_j}, m = 0..lmax (aliasing for m >= n is the DFT's own).
 // One block per (ring, 128 m); the ring's values staged in shared memory.
 __global__ void __launch_bounds__(kRingThreads) k_ring_analysis(const double* __restrict__ map, int nside, int lmax,
@@ -268,72 +542,396 @@ __global__ void __launch_bounds__(kRingThreads) k_ring_synthesis(const double2* 
   map[g.start + j] = coef[0].x + 2.0 * acc;
 }
 
+// Rings with 4 nside pixels or fewer, nside <= kRingFftMax, are transformed by an FP64 FFT in
+// shared memory, one CTA per ring. A ring has n = 4 i pixels; its 2 i complex pairs (f_2j +
+// i f_2j+1) split into two interleaved transforms of length i, which are plain radix-4 ones
+// when i is a power of two and Bluestein convolutions of length M = 2^c >= 2 i - 1 otherwise
+// (x_j c_j convolved with conj(c_j), c_j = e^{-i pi j^2 / i}, the chirp's index reduced
+// exactly: j^2 mod 2 i). The transforms are decimation in frequency (natural -> digit
+// reversed) and back in time, so nothing is permuted; the pointwise product does not see the
+// order and a plain transform's outputs are picked up by their digit-reversed position.
+// A ring is never mixed with another one: a NaN or a huge value stays in its ring.
+//
+// 1 B200, nside 1024, lmax 3000: analysis 19.4 -> 0.44 ms, synthesis 20.0 -> 0.42 ms against direct
+// sums (npix x lmax terms), which still serve larger nside, whose convolutions (M = 4096 and
+// more, three arrays) do not fit two CTAs per SM.
+constexpr int kRingFftMax = 1024;
+constexpr int kRingFftThreads = 256;
+
+struct RingFft {
+  int i, M, lg;   // sub-transform length, its FFT length 2^lg
+  bool plain;     // M == i
+  double2 *arr;   // [2][M]
+  double2 *filt;  // [M + 1]: the chirp filter's spectrum (before that, free)
+  double2 *tw;    // [M / 4]: e^{-2 pi i j / M}
+  double2 *part;  // [kRingFftThreads]: the synthesis's partial sums of short rings
+};
+
+__host__ __device__ inline int ring_fft_length(int i) {
+  if ((i & (i - 1)) == 0) return i;
+  int M = 1;
+  while (M < 2 * i - 1) M <<= 1;
+  return M;
+}
+// shared memory for rings of up to 4 nside pixels
+inline size_t ring_fft_smem(int nside) {
+  int M = 1;
+  for (int i = nside; i >= 1 && i > nside - 2; --i) {  // nside and nside - 1 cover the largest of both kinds
+    const int L = ring_fft_length(i);
+    if (L > M) M = L;
+  }
+  // the synthesis keeps the ring's 2 i + 1 folded coefficients in filt, whatever the kind
+  const size_t filt = (size_t)(M > 2 * nside ? M : 2 * nside) + 1;
+  return sizeof(double2) * ((size_t)2 * M + filt + M / 4 + kRingFftThreads);
+}
+
+__device__ __forceinline__ double2 cispi(double x) {  // e^{i pi x}
+  double s, c;
+  sincospi(x, &s, &c);
+  return make_double2(c, s);
+}
+
+__device__ __forceinline__ double2 chirp(int j, int i) { return zconj(cispi((double)((j * j) % (2 * i)) / (double)i)); }
+
+__device__ __forceinline__ RingFft ring_fft_setup(int i, double2* sm) {
+  RingFft f;
+  f.i = i;
+  f.M = ring_fft_length(i);
+  f.plain = f.M == i;
+  f.lg = 31 - __clz(f.M);
+  f.arr = sm;
+  f.filt = sm + 2 * f.M;
+  f.tw = f.filt + (max(f.M, 2 * i) + 1);
+  f.part = f.tw + f.M / 4;
+  for (int j = threadIdx.x; j < f.M / 4; j += blockDim.x) f.tw[j] = cispi(-2.0 * j / (double)f.M);
+  return f;
+}
+
+// Forward DIF transforms of `count` consecutive arrays of length M = 2^lg, in place; ends with
+// a barrier.
+__device__ __forceinline__ void ring_fft_forward(double2* x, int count, int lg, const double2* tw) {
+  int lq = lg - 2, step = 0;  // quarter 2^lq, twiddle stride 2^step
+  for (; lq >= 0; lq -= 2, step += 2) {
+    const int total = count << (lg - 2);
+    for (int t = threadIdx.x; t < total; t += blockDim.x) {
+      const int j = t & ((1 << lq) - 1);
+      double2* p = x + (((t >> lq) << (lq + 2)) + j);
+      const double2 a0 = p[0], a1 = p[1 << lq], a2 = p[2 << lq], a3 = p[3 << lq];
+      const double2 s02 = zadd(a0, a2), d02 = zsub(a0, a2), s13 = zadd(a1, a3), d13 = zsub(a1, a3);
+      const double2 w1 = tw[j << step], w2 = zmul(w1, w1);
+      p[0] = zadd(s02, s13);
+      p[1 << lq] = zmul(make_double2(d02.x + d13.y, d02.y - d13.x), w1);  // (d02 - i d13) w
+      p[2 << lq] = zmul(zsub(s02, s13), w2);
+      p[3 << lq] = zmul(make_double2(d02.x - d13.y, d02.y + d13.x), zmul(w2, w1));
+    }
+    __syncthreads();
+  }
+  if (lg & 1) {
+    const int total = count << (lg - 1);
+    for (int t = threadIdx.x; t < total; t += blockDim.x) {
+      const double2 a = x[2 * t], b = x[2 * t + 1];
+      x[2 * t] = zadd(a, b);
+      x[2 * t + 1] = zsub(a, b);
+    }
+    __syncthreads();
+  }
+}
+
+// The inverse of ring_fft_forward (unnormalised), digit reversed -> natural.
+__device__ __forceinline__ void ring_fft_inverse(double2* x, int count, int lg, const double2* tw) {
+  if (lg & 1) {
+    const int total = count << (lg - 1);
+    for (int t = threadIdx.x; t < total; t += blockDim.x) {
+      const double2 a = x[2 * t], b = x[2 * t + 1];
+      x[2 * t] = zadd(a, b);
+      x[2 * t + 1] = zsub(a, b);
+    }
+    __syncthreads();
+  }
+  for (int lq = lg & 1; lq <= lg - 2; lq += 2) {
+    const int step = lg - 2 - lq;
+    const int total = count << (lg - 2);
+    for (int t = threadIdx.x; t < total; t += blockDim.x) {
+      const int j = t & ((1 << lq) - 1);
+      double2* p = x + (((t >> lq) << (lq + 2)) + j);
+      const double2 w1 = zconj(tw[j << step]), w2 = zmul(w1, w1);
+      const double2 y0 = p[0], y1 = zmul(p[1 << lq], w1), y2 = zmul(p[2 << lq], w2), y3 = zmul(p[3 << lq], zmul(w2, w1));
+      const double2 s02 = zadd(y0, y2), d02 = zsub(y0, y2), s13 = zadd(y1, y3), d13 = zsub(y1, y3);
+      p[0] = zadd(s02, s13);
+      p[1 << lq] = make_double2(d02.x - d13.y, d02.y + d13.x);  // d02 + i d13
+      p[2 << lq] = zsub(s02, s13);
+      p[3 << lq] = make_double2(d02.x + d13.y, d02.y - d13.x);
+    }
+    __syncthreads();
+  }
+}
+
+// Where ring_fft_forward leaves frequency k.
+__device__ __forceinline__ int digit_reversed(int k, int lg) {
+  int pos = 0, left = lg;
+  while (left >= 2) {
+    left -= 2;
+    pos |= (k & 3) << left;
+    k >>= 2;
+  }
+  if (left == 1) pos |= k & 1;
+  return pos;
+}
+
+// DFT of length 2 i of the values whose pairs (s_2j, s_2j+1) the caller put in (arr[0][j],
+// arr[1][j]), j < i. Afterwards frequency k is at ring_fft_at(f, k). Starts and ends with a
+// barrier; filt is overwritten.
+__device__ __forceinline__ void ring_fft_run(const RingFft& f) {
+  const int i = f.i, M = f.M;
+  __syncthreads();
+  if (f.plain) {
+    ring_fft_forward(f.arr, 2, f.lg, f.tw);
+  } else {
+    for (int j = threadIdx.x; j < M; j += blockDim.x) {
+      const bool in = j < i;
+      const double2 c = chirp(in ? j : 0, i);
+      f.arr[j] = in ? zmul(f.arr[j], c) : make_double2(0.0, 0.0);
+      f.arr[M + j] = in ? zmul(f.arr[M + j], c) : make_double2(0.0, 0.0);
+      const int b = in ? j : (M - j < i ? M - j : -1);
+      f.filt[j] = b < 0 ? make_double2(0.0, 0.0) : zconj(chirp(b, i));
+    }
+    __syncthreads();
+    ring_fft_forward(f.arr, 3, f.lg, f.tw);  // filt follows arr: transformed with it
+    for (int j = threadIdx.x; j < M; j += blockDim.x) {
+      const double2 b = f.filt[j];
+      f.arr[j] = zmul(f.arr[j], b);
+      f.arr[M + j] = zmul(f.arr[M + j], b);
+    }
+    __syncthreads();
+    ring_fft_inverse(f.arr, 2, f.lg, f.tw);
+  }
+  const double scale = 1.0 / (double)M;
+  for (int k = threadIdx.x; k < i; k += blockDim.x) {
+    const int at = f.plain ? digit_reversed(k, f.lg) : k;
+    double2 s0 = f.arr[at], s1 = f.arr[M + at];
+    const double2 w = cispi(-(double)k / (double)i);  // e^{-2 pi i k / 2i}
+    if (f.plain) {
+      s1 = zmul(s1, w);
+    } else {
+      double2 c = chirp(k, i);
+      c.x *= scale;
+      c.y *= scale;
+      s0 = zmul(s0, c);
+      s1 = zmul(s1, zmul(c, w));
+    }
+    f.arr[at] = zadd(s0, s1);
+    f.arr[M + at] = zsub(s0, s1);
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ double2 ring_fft_at(const RingFft& f, int k) {
+  const int half = k >= f.i;
+  const int q = k - (half ? f.i : 0);
+  return f.arr[half * f.M + (f.plain ? digit_reversed(q, f.lg) : q)];
+}
+
+// e^{-i m phi0}, phi0 = pi / n or 0
+__device__ __forceinline__ double2 ring_phase(int m, const RingPhi& g) {
+  if (g.phi0 == 0.0) return make_double2(1.0, 0.0);
+  return cispi(-(double)(m % (2 * g.n)) / (double)g.n);
+}
+
+__global__ void __launch_bounds__(kRingFftThreads) k_ring_fft_analysis(const double* __restrict__ map, int nside,
+                                                                       int lmax, double2* __restrict__ F) {
+  extern __shared__ double2 sm2[];
+  const int r = blockIdx.x;
+  const RingPhi g = ring_phi(r, nside);
+  const int n = g.n, h = n / 2;
+  const RingFft f = ring_fft_setup(n / 4, sm2);
+  const double* src = map + g.start;
+  for (int j = threadIdx.x; j < h; j += blockDim.x)  // (f_2j, f_2j+1): ring starts and n are even
+    f.arr[(j & 1) * f.M + (j >> 1)] = make_double2(src[2 * j], src[2 * j + 1]);
+  ring_fft_run(f);
+  double2* out = F + (long long)r * (lmax + 1);
+  for (int m = threadIdx.x; m <= lmax; m += blockDim.x) {
+    int k = m % n;
+    const bool mirror = k > h;  // X[k] = conj X[n - k]
+    if (mirror) k = n - k;
+    const double2 a = ring_fft_at(f, k == h ? 0 : k), b = zconj(ring_fft_at(f, k == 0 ? 0 : h - k));
+    const double2 e = make_double2(0.5 * (a.x + b.x), 0.5 * (a.y + b.y));
+    const double2 o = make_double2(0.5 * (a.y - b.y), -0.5 * (a.x - b.x));  // (a - b) / 2i
+    double2 x = zadd(e, zmul(o, cispi(-2.0 * k / (double)n)));
+    if (mirror) x = zconj(x);
+    out[m] = zmul(x, ring_phase(m, g));
+  }
+}
+
+__global__ void __launch_bounds__(kRingFftThreads) k_ring_fft_synthesis(const double2* __restrict__ G, int nside,
+                                                                        int lmax, double* __restrict__ map) {
+  extern __shared__ double2 sm2[];
+  const int r = blockIdx.x;
+  const RingPhi g = ring_phi(r, nside);
+  const int n = g.n, h = n / 2;
+  const RingFft f = ring_fft_setup(n / 4, sm2);
+  const double2* src = G + (long long)r * (lmax + 1);
+  // E[k], k = 0..h: the Hermitian part of the folded spectrum, (H[k] + conj H[n - k]) / 2 with
+  // H[k] = sum over m = k, k + n, ... of c_m G[m] e^{i m phi0}, c_0 = 1 (real part), c_m = 2.
+  // A ring with fewer frequencies than the CTA has threads gives each several threads, which
+  // take every `groups`-th m and are added in order.
+  const int nk = h + 1;
+  const int groups = max(1, (int)blockDim.x / nk);
+  double2* E = f.filt;
+  double2* partial = f.part;  // [groups][nk]
+  for (int t = threadIdx.x; t < groups * nk; t += blockDim.x) {
+    const int grp = t / nk, k = t - grp * nk;
+    double2 s = make_double2(0.0, 0.0);
+    for (int m = k + grp * n; m <= lmax; m += groups * n) {
+      double2 v = zmul(src[m], zconj(ring_phase(m, g)));
+      if (m == 0) v = make_double2(0.5 * src[0].x, 0.0);
+      s = zadd(s, v);
+    }
+    for (int m = (k == 0 ? n : n - k) + grp * n; m <= lmax; m += groups * n)
+      s = zadd(s, zconj(zmul(src[m], zconj(ring_phase(m, g)))));
+    if (k == 0 && grp == 0) s = zadd(s, make_double2(0.5 * src[0].x, 0.0));  // conj H[0]'s m = 0
+    if (groups == 1)
+      E[k] = s;
+    else
+      partial[t] = s;
+  }
+  __syncthreads();
+  if (groups > 1) {
+    for (int k = threadIdx.x; k < nk; k += blockDim.x) {
+      double2 s = partial[k];
+      for (int grp = 1; grp < groups; ++grp) s = zadd(s, partial[grp * nk + k]);
+      E[k] = s;
+    }
+    __syncthreads();
+  }
+  // f_2j + i f_2j+1 = sum_k Z[k] e^{2 pi i j k / h}, Z[k] = (E[k] + conj E[h-k]) + i (E[k] - conj
+  // E[h-k]) e^{2 pi i k / n}; the inverse transform as the conjugate of a forward one
+  for (int k = threadIdx.x; k < h; k += blockDim.x) {
+    const double2 a = E[k], b = zconj(E[h - k]);
+    const double2 e = zadd(a, b), d = zmul(zsub(a, b), cispi(2.0 * k / (double)n));
+    f.arr[(k & 1) * f.M + (k >> 1)] = make_double2(e.x - d.y, -(e.y + d.x));
+  }
+  ring_fft_run(f);
+  double* dst = map + g.start;
+  for (int j = threadIdx.x; j < h; j += blockDim.x) {
+    const double2 v = ring_fft_at(f, j);
+    dst[2 * j] = v.x;
+    dst[2 * j + 1] = -v.y;
+  }
+}
+
 cudaError_t sht_ring_analysis(const double* map, int nside, int lmax, double* F, cudaStream_t s) {
   const int nrings = 4 * nside - 1;
-  const size_t smem = sizeof(double) * 4 * (size_t)nside;
-  cudaError_t e = cudaFuncSetAttribute(k_ring_analysis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  const dim3 grid((lmax + kRingThreads) / kRingThreads, nrings);
-  k_ring_analysis<<<grid, kRingThreads, smem, s>>>(map, nside, lmax, reinterpret_cast<double2*>(F));
+  double2* out = reinterpret_cast<double2*>(F);
+  cudaError_t e;
+  if (nside <= kRingFftMax) {
+    const size_t smem = ring_fft_smem(nside);
+    e = cudaFuncSetAttribute(k_ring_fft_analysis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k_ring_fft_analysis<<<nrings, kRingFftThreads, smem, s>>>(map, nside, lmax, out);
+  } else {
+    const size_t smem = sizeof(double) * 4 * (size_t)nside;
+    e = cudaFuncSetAttribute(k_ring_analysis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k_ring_analysis<<<dim3((lmax + kRingThreads) / kRingThreads, nrings), kRingThreads, smem, s>>>(map, nside, lmax,
+                                                                                                   out);
+  }
   note_launch();
   return cudaGetLastError();
 }
 
 cudaError_t sht_ring_synthesis(const double* G, int nside, int lmax, double* map, cudaStream_t s) {
   const int nrings = 4 * nside - 1;
-  const size_t smem = sizeof(double2) * (size_t)(lmax + 1);
-  cudaError_t e = cudaFuncSetAttribute(k_ring_synthesis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const double2* in = reinterpret_cast<const double2*>(G);
+  cudaError_t e;
+  if (nside <= kRingFftMax) {
+    const size_t smem = ring_fft_smem(nside);
+    e = cudaFuncSetAttribute(k_ring_fft_synthesis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k_ring_fft_synthesis<<<nrings, kRingFftThreads, smem, s>>>(in, nside, lmax, map);
+  } else {
+    const size_t smem = sizeof(double2) * (size_t)(lmax + 1);
+    e = cudaFuncSetAttribute(k_ring_synthesis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k_ring_synthesis<<<dim3((4 * nside + kRingThreads - 1) / kRingThreads, nrings), kRingThreads, smem, s>>>(
+        in, nside, lmax, map);
+  }
+  note_launch();
+  return cudaGetLastError();
+}
+
+template <int RP>
+static cudaError_t analysis_launch(const LegendreShape& sh, const double* F, const double* z, int nrings, int lmax,
+                                   double weight, double* alm, cudaStream_t s) {
+  const size_t smem = sizeof(double) * (size_t)(sh.threads / 32) * kLTile * 33;
+  cudaError_t e = cudaFuncSetAttribute(k_sht_analysis<RP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  const dim3 grid((4 * nside + kRingThreads - 1) / kRingThreads, nrings);
-  k_ring_synthesis<<<grid, kRingThreads, smem, s>>>(reinterpret_cast<const double2*>(G), nside, lmax, map);
+  k_sht_analysis<RP><<<dim3(lmax + 1, sh.blocks), sh.threads, smem, s>>>(
+      reinterpret_cast<const double2*>(F), z, nrings, lmax, weight, reinterpret_cast<double2*>(alm));
   note_launch();
   return cudaGetLastError();
 }
 
 cudaError_t sht_analysis(const double* F, const double* z, int nrings, int lmax, double weight, double* alm,
                          cudaStream_t s) {
-  const long long nalm = alm_offset(lmax + 1, lmax);
-  cudaError_t e = cudaMemsetAsync(alm, 0, sizeof(double2) * (size_t)nalm, s);
-  if (e != cudaSuccess) return e;
-  const size_t smem = sizeof(double2) * kShtLTile * kShtRow;
-  e = cudaFuncSetAttribute(k_sht_analysis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  const dim3 grid((nrings + kShtThreads - 1) / kShtThreads, lmax + 1);
-  k_sht_analysis<<<grid, kShtThreads, smem, s>>>(reinterpret_cast<const double2*>(F), z, nrings, lmax, weight,
-                                                  reinterpret_cast<double2*>(alm));
-  note_launch();
-  return cudaGetLastError();
+  const LegendreShape sh = legendre_shape(nrings);
+  if (sh.blocks > 1) {  // the blocks of one m add to alm
+    const cudaError_t e = cudaMemsetAsync(alm, 0, sizeof(double2) * (size_t)alm_offset(lmax + 1, lmax), s);
+    if (e != cudaSuccess) return e;
+  }
+  if (sh.rp == 8) return analysis_launch<8>(sh, F, z, nrings, lmax, weight, alm, s);
+  if (sh.rp == 4) return analysis_launch<4>(sh, F, z, nrings, lmax, weight, alm, s);
+  return analysis_launch<2>(sh, F, z, nrings, lmax, weight, alm, s);
 }
 
 cudaError_t sht_synthesis(const double* alm, const double* z, int nrings, int lmax, double* G, cudaStream_t s) {
-  const dim3 grid((nrings + kShtThreads - 1) / kShtThreads, lmax + 1);
-  k_sht_synthesis<<<grid, kShtThreads, 0, s>>>(reinterpret_cast<const double2*>(alm), z, nrings, lmax,
-                                                reinterpret_cast<double2*>(G));
+  const LegendreShape sh = legendre_shape(nrings);
+  const dim3 grid(lmax + 1, sh.blocks);
+  const double2* a = reinterpret_cast<const double2*>(alm);
+  double2* out = reinterpret_cast<double2*>(G);
+  if (sh.rp == 8)
+    k_sht_synthesis<8><<<grid, sh.threads, 0, s>>>(a, z, nrings, lmax, out);
+  else if (sh.rp == 4)
+    k_sht_synthesis<4><<<grid, sh.threads, 0, s>>>(a, z, nrings, lmax, out);
+  else
+    k_sht_synthesis<2><<<grid, sh.threads, 0, s>>>(a, z, nrings, lmax, out);
   note_launch();
   return cudaGetLastError();
 }
 
-// C_l = (Re a_l0 b_l0* + 2 sum_{m=1..l} Re a_lm b_lm*) / (2l + 1) (healpy alm2cl), one
-// thread per l, FP64 sums in increasing m (a fixed order: the result is deterministic).
-__global__ void k_sht_alm2cl(const double2* __restrict__ a, const double2* __restrict__ b, int lmax,
-                             double* __restrict__ cl) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l > lmax) return;
+// C_l = (Re a_l0 b_l0* + 2 sum_{m=1..l} Re a_lm b_lm*) / (2l + 1) (healpy alm2cl), FP64. A
+// block takes 32 l; its 16 rows of threads each sum every 16th m (32 neighbouring l of one m
+// are contiguous) and the rows are added in order, so the result is deterministic. (One
+// thread per l left 3001 chains of dependent loads: 0.67 ms at lmax 3000, 0.05 ms now.)
+constexpr int kClRows = 16;
+
+__global__ void __launch_bounds__(32 * kClRows) k_sht_alm2cl(const double2* __restrict__ a,
+                                                             const double2* __restrict__ b, int lmax,
+                                                             double* __restrict__ cl) {
+  __shared__ double sum[kClRows][33];
+  const int l = blockIdx.x * 32 + threadIdx.x;
   double acc = 0.0;
-  for (int m = 1; m <= l; ++m) {
-    const long long o = alm_offset(m, lmax) + (l - m);
-    const double2 x = a[o], y = b[o];
-    acc += x.x * y.x + x.y * y.y;
+  if (l <= lmax) {
+#pragma unroll 4
+    for (int m = 1 + threadIdx.y; m <= l; m += kClRows) {
+      const long long o = alm_offset(m, lmax) + (l - m);
+      const double2 x = a[o], y = b[o];
+      acc += x.x * y.x + x.y * y.y;
+    }
   }
-  const double2 x0 = a[l], y0 = b[l];
-  cl[l] = (x0.x * y0.x + x0.y * y0.y + 2.0 * acc) / (2.0 * l + 1.0);
+  sum[threadIdx.y][threadIdx.x] = acc;
+  __syncthreads();
+  if (threadIdx.y == 0 && l <= lmax) {
+    acc = 0.0;
+    for (int r = 0; r < kClRows; ++r) acc += sum[r][threadIdx.x];
+    const double2 x0 = a[l], y0 = b[l];
+    cl[l] = (x0.x * y0.x + x0.y * y0.y + 2.0 * acc) / (2.0 * l + 1.0);
+  }
 }
 
 cudaError_t sht_alm2cl(const double* alm1, const double* alm2, int lmax, double* cl, cudaStream_t s) {
-  const int threads = 128;
-  k_sht_alm2cl<<<(lmax + threads) / threads, threads, 0, s>>>(reinterpret_cast<const double2*>(alm1),
-                                                            reinterpret_cast<const double2*>(alm2 ? alm2 : alm1),
-                                                            lmax, cl);
+  k_sht_alm2cl<<<(lmax + 32) / 32, dim3(32, kClRows), 0, s>>>(reinterpret_cast<const double2*>(alm1),
+                                                              reinterpret_cast<const double2*>(alm2 ? alm2 : alm1),
+                                                              lmax, cl);
   note_launch();
   return cudaGetLastError();
 }

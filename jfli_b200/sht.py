@@ -5,8 +5,8 @@ The reference computes angular power spectra with healpy.anafast
 published algorithm with the map, the a_lm and the spectrum on the device, in the
 library's FP64 kernels:
 
-* the ring transforms along phi as direct DFTs (`jfli_sht_ring_analysis`,
-  `jfli_sht_ring_synthesis`): F_r(m) = e^{-i m phi_0} sum_j f_j e^{-2 pi i m j / n_r};
+* the ring transforms along phi (`jfli_sht_ring_analysis`, `jfli_sht_ring_synthesis`):
+  F_r(m) = e^{-i m phi_0} sum_j f_j e^{-2 pi i m j / n_r};
 * the O(lmax^2 x rings) Legendre stages (`jfli_sht_map2alm`, `jfli_sht_alm2map`) with
   uniform quadrature weights 4 pi / npix and a_lm packed by m (a[m][l - m]);
 * healpy's default iterative refinement (iter=3): a += map2alm(map - alm2map(a));
@@ -60,7 +60,7 @@ def packed_offsets(lmax: int) -> np.ndarray:
 
 class _GpuSht:
     """Device tables of one (nside, lmax) and the four device stages: ring transforms along
-    phi (direct FP64 DFTs) and the Legendre stages. Maps and a_lm stay on the device."""
+    phi and the Legendre stages. Maps and a_lm stay on the device."""
 
     def __init__(self, nside: int, lmax: int, device=None):
         self.nside, self.lmax = nside, lmax
