@@ -46,52 +46,73 @@ __device__ __forceinline__ double2 zconj(double2 a) { return make_double2(a.x, -
 // they grow; a ring adds to the sums only at k = 0 (below, its lambda is under 2^-140). The
 // scale is looked at every 8 l, over which a value grows by less than 2^60.
 //
-// The tables of one m (A_l and alpha_l for 32 l at a time) are made by one warp while the
-// others use the previous ones: a prefix product over lanes of equal parity.
+// The tables of one m (A_l and alpha_l) are made for 32 l per warp at a time, all warps at once,
+// and the CTA's sums of those l are finished together: three barriers per super-tile. (One
+// warp making the next 32 l's while the others worked had them wait for it at every table.)
 //
-// 1 B200, nside 1024, lmax 3000 (8190 x 4.5M (ring, l, m)): analysis 31.9 -> 6.9 ms, synthesis
-// 19.4 -> 5.3 ms against one ring per thread with a three-multiplication recursion and, in the
+// 1 B200, nside 1024, lmax 3000 (8190 x 4.5M (ring, l, m)): analysis 31.9 -> 3.6 ms, synthesis
+// 19.4 -> 3.4 ms against one ring per thread with a three-multiplication recursion and, in the
 // analysis, one shared-memory reduction per ring and l; FP64 floor of the form above 2.1 ms.
 constexpr int kLTile = 32;    // l per table
 constexpr int kLChunk = 8;    // l between looks at the scale
+constexpr int kRowTile = 16;  // l between reductions over a warp
 constexpr int kScaleBits = 400;
 
+constexpr int kLegendreWarps = 4;  // at most
+
+// A_l and alpha_l of the super-tile's l, and the products that the warps' tiles end on
 struct LegendreTables {
-  double A[2][kLTile], alpha[2][kLTile];
+  double A[kLegendreWarps * kLTile], alpha[kLegendreWarps * kLTile];
+  double2 ends[kLegendreWarps];
 };
 
-// a_l of the recursion (l > m)
-__device__ __forceinline__ double legendre_a(int l, int m) {
-  const double d = (double)l;
-  return sqrt((4.0 * d * d - 1.0) / ((double)(l - m) * (double)(l + m)));
+// a_l^2 / a_(l-1)^2 (l > m + 1)
+__device__ __forceinline__ double legendre_ratio(int l, int m) {
+  const double d = (double)l, e = d - 1.0;
+  return ((4.0 * d * d - 1.0) * ((double)(l - 1 - m) * (double)(l - 1 + m))) /
+         (((double)(l - m) * (double)(l + m)) * (4.0 * e * e - 1.0));
 }
 
-// Tables of l = l0 .. l0 + 31 (one warp, lane = l - l0; l0 - m is a multiple of 32). c0 and c1
-// carry alpha of the last two l across tables.
-__device__ __forceinline__ void legendre_tables(LegendreTables& t, int buf, int l0, int m, double& c0, double& c1) {
-  const int lane = threadIdx.x & 31;
-  const int l = l0 + lane;
-  const double al = l > m ? legendre_a(l, m) : 1.0;
-  const double ap = l > m + 1 ? legendre_a(l - 1, m) : 1.0;
-  // alpha_m = alpha_(m+1) = 1
-  double alpha = l > m + 1 ? al / ap : 1.0;
-  if (lane < 2) alpha *= lane == 0 ? c0 : c1;
+// Tables of a super-tile of 32 l per warp from s0 (s0 - m a multiple of 32), warp w making those
+// of l = s0 + 32 w + lane: alpha_l^2 is the product of the ratios of equal parity (a scan over
+// lanes of a stride of two, then over the warps' tiles, then the carry of the super-tiles
+// before), A_l = a_(l-1) alpha_(l-1) / alpha_(l-2) from the same products, so that their
+// accumulated rounding cancels in lambda (the closed form A_l = a_(m+1) alpha_(l-1)^2 would
+// need no second division, but lets it in: 1.5e-12 of lambda at l = 700 against 2e-14).
+// carry: alpha^2 of the last two l before s0, the same in every thread. Two barriers inside,
+// the first before the tables are overwritten, the second after they are written.
+__device__ __forceinline__ void legendre_tables(LegendreTables& t, int s0, int m, double2& carry) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int l = s0 + kLTile * warp + lane;
+  double q = l > m + 1 ? legendre_ratio(l, m) : 1.0;  // alpha_m = alpha_(m+1) = 1
 #pragma unroll
   for (int off = 2; off < 32; off <<= 1) {
-    const double v = __shfl_up_sync(0xffffffffu, alpha, off);
-    if (lane >= off) alpha *= v;
+    const double v = __shfl_up_sync(0xffffffffu, q, off);
+    if (lane >= off) q *= v;
   }
-  double p1 = __shfl_up_sync(0xffffffffu, alpha, 1), p2 = __shfl_up_sync(0xffffffffu, alpha, 2);
+  if (lane == 30) t.ends[warp].x = q;
+  if (lane == 31) t.ends[warp].y = q;
+  __syncthreads();
+  double2 c = carry;  // alpha^2 of the last two l before this warp's tile
+  for (int w = 0; w < warps; ++w) {
+    if (w == warp) c = carry;
+    carry.x *= t.ends[w].x;
+    carry.y *= t.ends[w].y;
+  }
+  q *= (lane & 1) ? c.y : c.x;
+  double p1 = __shfl_up_sync(0xffffffffu, q, 1), p2 = __shfl_up_sync(0xffffffffu, q, 2);
   if (lane == 0) {
-    p1 = c1;
-    p2 = c0;
+    p1 = c.y;
+    p2 = c.x;
   } else if (lane == 1) {
-    p2 = c1;
+    p2 = c.y;
   }
-  t.A[buf][lane] = l > m + 1 ? ap * p1 / p2 : al;  // lambda_(m+1) = a_(m+1) z lambda_mm
-  t.alpha[buf][lane] = alpha;
-  c0 = __shfl_sync(0xffffffffu, alpha, 30);
-  c1 = __shfl_sync(0xffffffffu, alpha, 31);
+  const double e = (double)(l - 1);
+  t.A[kLTile * warp + lane] =
+      sqrt(l > m + 1 ? ((4.0 * e * e - 1.0) * p1) / (((double)(l - 1 - m) * (double)(l - 1 + m)) * p2)
+                     : 2.0 * m + 3.0);  // lambda_(m+1) = a_(m+1) z lambda_mm
+  t.alpha[kLTile * warp + lane] = sqrt(q);
+  __syncthreads();
 }
 
 // ln of the normalisation of lambda_mm without its sign: ln sqrt((1 / 4 pi) prod_(k=1..m) (2k
@@ -109,7 +130,8 @@ __device__ __forceinline__ double legendre_lognorm(int m, double* scratch) {
   return 0.5 * (s - 2.5310242469692907);  // ln 4 pi
 }
 
-// One ring (pair) of a thread: z, the last two mu, and the scale k (see above).
+// One ring (pair) of a thread: z, the last two mu, and the scale k (see above). Every l, the
+// first included, is one step: a step that is skipped at l = m costs selects at all others.
 struct LegendreRing {
   double z, prev, cur;
   int k;
@@ -121,8 +143,10 @@ struct LegendreRing {
     const double v = m == 0 ? lognorm : lognorm + 0.5 * m * log(s2);  // s2 = 0: -inf, lambda = 0
     const double step = kScaleBits * 0.69314718055994530942;
     k = v < -0.5 * step ? (int)fmin(1e6, ceil((-0.5 * step - v) / step)) : 0;
-    cur = exp(v + k * step);
-    if (m & 1) cur = -cur;
+    // before l = m: the step to it gives A z 0 - prev = lambda_mm
+    cur = 0.0;
+    prev = exp(v + k * step);
+    if (!(m & 1)) prev = -prev;
   }
   __device__ __forceinline__ void rescale() {
     if (k > 0 && fabs(cur) > 0x1p200) {
@@ -152,21 +176,26 @@ struct RingPairs {
   }
 };
 
-constexpr int kLegendreThreads = 256;  // at most
-
-// Analysis: a thread's sums over its pairs of one l go through shared memory: the lanes of a
-// warp first halve (re in lanes 0..15, im in 16..31), 32 l are collected per warp and lane j
-// adds up row j, so the reduction over a warp's rings costs a few instructions per l.
+// Four warps at most: the warps of a CTA meet at every super-tile, and the pole-side ones have less
+// to do (at nside 1024 one CTA of eight warps per m took 5.7 and 3.9 ms for the two stages,
+// two of four 4.3 and 3.6; with the tables per super-tile 3.6 and 3.4).
+constexpr int kLegendreThreads = 32 * kLegendreWarps;
 template <int RP>
-__global__ void __launch_bounds__(kLegendreThreads) k_sht_analysis(const double2* __restrict__ F,
+constexpr int kLegendreCtas = RP == 8 ? 3 : 6;  // resident per SM (168 and 80 registers)
+
+// Analysis: a thread's sums over its pairs go through shared memory, 16 l at a time per warp: a
+// lane stores one value per l and afterwards adds up half a row (the lanes of one l), so the
+// reduction over a warp's rings costs four instructions per l.
+template <int RP>
+__global__ void __launch_bounds__(kLegendreThreads, kLegendreCtas<RP>) k_sht_analysis(const double2* __restrict__ F,
                                                                    const double* __restrict__ z, int nrings, int lmax,
                                                                    double w, double2* __restrict__ alm) {
   __shared__ LegendreTables tab;
-  __shared__ double2 part[kLegendreThreads / 32][kLTile];
-  extern __shared__ double rows[];  // per warp [32 l][33]
+  __shared__ double2 part[kLegendreWarps][kLegendreWarps * kLTile];
+  extern __shared__ double2 rows[];  // per warp [16 l][33]
   const int m = blockIdx.x;
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double* row = rows + (size_t)warp * kLTile * 33;
+  double2* row = rows + (size_t)warp * kRowTile * 33;
   const RingPairs rp{nrings, (nrings + 1) / 2};
   const int first = blockIdx.y * (blockDim.x * RP);
   const bool mirror = rp.mirrored(z, first, blockDim.x * RP);
@@ -197,129 +226,103 @@ __global__ void __launch_bounds__(kLegendreThreads) k_sht_analysis(const double2
       r[j].start(m, zr, lognorm);
     }
     // 0, or NaN where a ring's coefficients are not finite: what a ring adds before its lambda counts
-    double poison = 0.0;
-    {
-      double px = 0.0, py = 0.0;
+    double2 poison = make_double2(0.0, 0.0);
 #pragma unroll
-      for (int j = 0; j < RP; ++j) {
-        px += 0.0 * even[j].x + 0.0 * odd[j].x;
-        py += 0.0 * even[j].y + 0.0 * odd[j].y;
-      }
-      poison = (lane < 16 ? px : py) + __shfl_xor_sync(0xffffffffu, lane < 16 ? py : px, 16);
+    for (int j = 0; j < RP; ++j) {
+      poison.x += 0.0 * even[j].x + 0.0 * odd[j].x;
+      poison.y += 0.0 * even[j].y + 0.0 * odd[j].y;
     }
-    const bool poisoned = __any_sync(0xffffffffu, !(poison == 0.0));
-    double c0 = 1.0, c1 = 1.0;  // used by the warp whose turn it is; handed on through shared memory
-    __shared__ double carry[2];
-    if (warp == 0) {
-      legendre_tables(tab, 0, m, m, c0, c1);
-      if (lane == 0) {
-        carry[0] = c0;
-        carry[1] = c1;
-      }
-    }
-    __syncthreads();
-    int buf = 0;
-    for (int l0 = m; l0 <= lmax; l0 += kLTile, buf ^= 1) {
-      // the next table, by a warp that changes with the table
-      if (l0 + kLTile <= lmax && warp == ((l0 - m) / kLTile + 1) % warps) {
-        c0 = carry[0];
-        c1 = carry[1];
-        __syncwarp();
-        legendre_tables(tab, buf ^ 1, l0 + kLTile, m, c0, c1);
-        if (lane == 0) {
-          carry[0] = c0;
-          carry[1] = c1;
-        }
-      }
-      bool any = poisoned;
-      for (int t0 = 0; t0 < kLTile; t0 += kLChunk) {
-        int scaled = 0;
+    const bool poisoned = __any_sync(0xffffffffu, !(poison.x == 0.0 && poison.y == 0.0));
+    double2 carry = make_double2(1.0, 1.0);
+    for (int s0 = m; s0 <= lmax; s0 += kLTile * warps) {
+      legendre_tables(tab, s0, m, carry);
+      const int t2 = min(kLTile * warps, lmax + 1 - s0);
+      for (int t1 = 0; t1 < t2; t1 += kRowTile) {
+        bool any = poisoned;
+        for (int t0 = t1; t0 < t1 + kRowTile; t0 += kLChunk) {
+          int scaled = 0;
 #pragma unroll
-        for (int j = 0; j < RP; ++j) {
-          r[j].rescale();
-          scaled += r[j].k > 0;
-        }
-        const bool all_on = __all_sync(0xffffffffu, scaled == 0);
-        const bool none_on = __all_sync(0xffffffffu, scaled == RP);
-        if (!none_on) any = true;
-        auto chunk = [&](auto masked) {
-          double on[RP];
-          if constexpr (masked) {
-#pragma unroll
-            for (int j = 0; j < RP; ++j) on[j] = r[j].k == 0 ? 1.0 : 0.0;
+          for (int j = 0; j < RP; ++j) {
+            r[j].rescale();
+            scaled += r[j].k > 0;
           }
+          const bool all_on = __all_sync(0xffffffffu, scaled == 0);
+          const bool none_on = __all_sync(0xffffffffu, scaled == RP);
+          if (!none_on) any = true;
+          double2* out = row + (t0 - t1) * 33 + lane;
+          auto chunk = [&](auto masked) {
+            bool on[RP];
+            if constexpr (masked) {
 #pragma unroll
-          for (int t = 0; t < kLChunk; ++t) {
-            const int l = l0 + t0 + t;
-            double re = 0.0, im = 0.0;
-#pragma unroll
-            for (int j = 0; j < RP; ++j) {
-              if (l > m) r[j].step(tab.A[buf][t0 + t]);
-              double v = r[j].cur;
-              if constexpr (masked) v *= on[j];
-              const double2 f = (t & 1) ? odd[j] : even[j];
-              re = fma(v, f.x, re);
-              im = fma(v, f.y, im);
+              for (int j = 0; j < RP; ++j) on[j] = r[j].k == 0;
             }
-            // lanes 0..15 take re, 16..31 im
-            const double give = lane < 16 ? im : re, keep = lane < 16 ? re : im;
-            row[(t0 + t) * 33 + lane] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
-          }
-        };
-        if (all_on) {
-          chunk(std::false_type{});
-        } else if (!none_on) {
-          chunk(std::true_type{});
-        } else {  // nothing to add yet
 #pragma unroll
-          for (int t = 0; t < kLChunk; ++t) {
+            for (int t = 0; t < kLChunk; ++t) {
+              double2 sum = make_double2(0.0, 0.0);
 #pragma unroll
-            for (int j = 0; j < RP; ++j)
-              if (l0 + t0 + t > m) r[j].step(tab.A[buf][t0 + t]);
-            row[(t0 + t) * 33 + lane] = poison;
-          }
-        }
-      }
-      __syncwarp();
-      double sx = 0.0, sy = 0.0;
-      if (any) {
+              for (int j = 0; j < RP; ++j) {
+                r[j].step(tab.A[t0 + t]);
+                double v = r[j].cur;
+                if constexpr (masked) v = on[j] ? v : 0.0;
+                const double2 f = (t & 1) ? odd[j] : even[j];
+                sum.x = fma(v, f.x, sum.x);
+                sum.y = fma(v, f.y, sum.y);
+              }
+              out[t * 33] = sum;
+            }
+          };
+          if (all_on) {
+            chunk(std::false_type{});
+          } else if (!none_on) {
+            chunk(std::true_type{});
+          } else {  // nothing to add yet
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          sx += row[lane * 33 + i];
-          sy += row[lane * 33 + 16 + i];
-        }
-      }
-      part[warp][lane] = make_double2(sx, sy);
-      __syncthreads();
-      if (threadIdx.x < kLTile) {
-        const int l = l0 + threadIdx.x;
-        if (l <= lmax) {
-          double2 s = make_double2(0.0, 0.0);
-          for (int i = 0; i < warps; ++i) s = zadd(s, part[i][threadIdx.x]);
-          const double f = w * tab.alpha[buf][threadIdx.x];
-          double2* dst = alm + off + (l - m);
-          if (gridDim.y > 1) {
-            atomicAdd(&dst->x, f * s.x);
-            atomicAdd(&dst->y, f * s.y);
-          } else if (hemi == 0) {
-            *dst = make_double2(f * s.x, f * s.y);
-          } else {
-            *dst = make_double2(dst->x + f * s.x, dst->y + f * s.y);
+            for (int t = 0; t < kLChunk; ++t) {
+#pragma unroll
+              for (int j = 0; j < RP; ++j) r[j].step(tab.A[t0 + t]);
+              out[t * 33] = poison;
+            }
           }
         }
+        __syncwarp();
+        double2 sum = make_double2(0.0, 0.0);
+        if (any) {
+          const double2* in = row + (lane & 15) * 33 + (lane & 16);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) sum = zadd(sum, in[i]);
+        }
+        sum.x += __shfl_xor_sync(0xffffffffu, sum.x, 16);
+        sum.y += __shfl_xor_sync(0xffffffffu, sum.y, 16);
+        if (lane < kRowTile) part[warp][t1 + lane] = sum;
+        __syncwarp();  // row is free again
       }
       __syncthreads();
+      const int l = s0 + threadIdx.x;
+      if (l <= lmax) {
+        double2 s = make_double2(0.0, 0.0);
+        for (int i = 0; i < warps; ++i) s = zadd(s, part[i][threadIdx.x]);
+        const double f = w * tab.alpha[threadIdx.x];
+        double2* dst = alm + off + (l - m);
+        if (gridDim.y > 1) {
+          atomicAdd(&dst->x, f * s.x);
+          atomicAdd(&dst->y, f * s.y);
+        } else if (hemi == 0) {
+          *dst = make_double2(f * s.x, f * s.y);
+        } else {
+          *dst = make_double2(dst->x + f * s.x, dst->y + f * s.y);
+        }
+      }
     }
   }
 }
 
 template <int RP>
-__global__ void __launch_bounds__(kLegendreThreads) k_sht_synthesis(const double2* __restrict__ alm,
+__global__ void __launch_bounds__(kLegendreThreads, kLegendreCtas<RP>) k_sht_synthesis(const double2* __restrict__ alm,
                                                                     const double* __restrict__ z, int nrings, int lmax,
                                                                     double2* __restrict__ G) {
   __shared__ LegendreTables tab;
-  __shared__ double2 a_tile[2][kLTile];  // alpha_l a_lm
-  __shared__ double scratch[kLegendreThreads / 32];
+  __shared__ double2 a_tile[kLegendreWarps * kLTile];  // alpha_l a_lm
+  __shared__ double scratch[kLegendreWarps];
   const int m = blockIdx.x;
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const RingPairs rp{nrings, (nrings + 1) / 2};
@@ -340,26 +343,18 @@ __global__ void __launch_bounds__(kLegendreThreads) k_sht_synthesis(const double
       even[j] = odd[j] = make_double2(0.0, 0.0);
       r[j].start(m, zr, lognorm);
     }
-    __shared__ double carry[2];
-    auto table = [&](int buf, int l0) {
-      double c0 = l0 == m ? 1.0 : carry[0], c1 = l0 == m ? 1.0 : carry[1];
-      __syncwarp();
-      legendre_tables(tab, buf, l0, m, c0, c1);
-      const int l = l0 + lane;
-      const double2 v = l <= lmax ? a[l - m] : make_double2(0.0, 0.0);
-      const double f = tab.alpha[buf][lane];
-      a_tile[buf][lane] = make_double2(f * v.x, f * v.y);
-      if (lane == 0) {
-        carry[0] = c0;
-        carry[1] = c1;
+    double2 carry = make_double2(1.0, 1.0);
+    for (int s0 = m; s0 <= lmax; s0 += kLTile * warps) {
+      legendre_tables(tab, s0, m, carry);
+      {
+        const int l = s0 + threadIdx.x;
+        const double2 v = l <= lmax ? a[l - m] : make_double2(0.0, 0.0);
+        const double f = tab.alpha[threadIdx.x];
+        a_tile[threadIdx.x] = make_double2(f * v.x, f * v.y);
       }
-    };
-    if (warp == 0) table(0, m);
-    __syncthreads();
-    int buf = 0;
-    for (int l0 = m; l0 <= lmax; l0 += kLTile, buf ^= 1) {
-      if (l0 + kLTile <= lmax && warp == ((l0 - m) / kLTile + 1) % warps) table(buf ^ 1, l0 + kLTile);
-      for (int t0 = 0; t0 < kLTile; t0 += kLChunk) {
+      __syncthreads();
+      const int t1 = min(kLTile * warps, lmax + 1 - s0);
+      for (int t0 = 0; t0 < t1; t0 += kLChunk) {
         int scaled = 0;
 #pragma unroll
         for (int j = 0; j < RP; ++j) {
@@ -369,19 +364,19 @@ __global__ void __launch_bounds__(kLegendreThreads) k_sht_synthesis(const double
         const bool all_on = __all_sync(0xffffffffu, scaled == 0);
         const bool none_on = __all_sync(0xffffffffu, scaled == RP);
         auto chunk = [&](auto masked) {
-          double on[RP];
+          bool on[RP];
           if constexpr (masked) {
 #pragma unroll
-            for (int j = 0; j < RP; ++j) on[j] = r[j].k == 0 ? 1.0 : 0.0;
+            for (int j = 0; j < RP; ++j) on[j] = r[j].k == 0;
           }
 #pragma unroll
           for (int t = 0; t < kLChunk; ++t) {
-            const double2 c = a_tile[buf][t0 + t];
+            const double2 c = a_tile[t0 + t];
 #pragma unroll
             for (int j = 0; j < RP; ++j) {
-              if (l0 + t0 + t > m) r[j].step(tab.A[buf][t0 + t]);
+              r[j].step(tab.A[t0 + t]);
               double v = r[j].cur;
-              if constexpr (masked) v *= on[j];
+              if constexpr (masked) v = on[j] ? v : 0.0;
               double2& s = (t & 1) ? odd[j] : even[j];
               s.x = fma(v, c.x, s.x);
               s.y = fma(v, c.y, s.y);
@@ -396,11 +391,9 @@ __global__ void __launch_bounds__(kLegendreThreads) k_sht_synthesis(const double
 #pragma unroll
           for (int t = 0; t < kLChunk; ++t)
 #pragma unroll
-            for (int j = 0; j < RP; ++j)
-              if (l0 + t0 + t > m) r[j].step(tab.A[buf][t0 + t]);
+            for (int j = 0; j < RP; ++j) r[j].step(tab.A[t0 + t]);
         }
       }
-      __syncthreads();
     }
 #pragma unroll
     for (int j = 0; j < RP; ++j) {
@@ -418,9 +411,10 @@ __global__ void __launch_bounds__(kLegendreThreads) k_sht_synthesis(const double
   }
 }
 
-// Pairs per thread and threads of a CTA: a thread takes 8 pairs (8 independent recursions)
-// when that still leaves four warps, fewer for small maps, whose 3 nside CTAs would otherwise
-// hold one or two warps each.
+// Pairs per thread and threads of a CTA. Eight pairs per thread (eight independent chains, the
+// least reduction and table work per pair) for large maps; two for small ones, whose 3 nside
+// CTAs do not fill the SMs for long and end on the serial chain of their first m (four maps of
+// nside 256: 2 pairs 3.6 ms, 4 pairs 4.0, 8 pairs 4.5).
 struct LegendreShape {
   int rp, threads, blocks;
 };
@@ -428,10 +422,9 @@ struct LegendreShape {
 static LegendreShape legendre_shape(int nrings) {
   const int pairs = (nrings + 1) / 2;
   LegendreShape s;
-  s.rp = pairs >= 1024 ? 8 : (pairs >= 256 ? 4 : 2);
+  s.rp = pairs >= 1024 ? 8 : 2;
   int warps = (pairs + 32 * s.rp - 1) / (32 * s.rp);
-  const int most = kLegendreThreads / 32;
-  s.blocks = (warps + most - 1) / most;
+  s.blocks = (warps + kLegendreWarps - 1) / kLegendreWarps;
   warps = (warps + s.blocks - 1) / s.blocks;
   s.threads = 32 * warps;
   return s;
@@ -862,7 +855,7 @@ cudaError_t sht_ring_synthesis(const double* G, int nside, int lmax, double* map
 template <int RP>
 static cudaError_t analysis_launch(const LegendreShape& sh, const double* F, const double* z, int nrings, int lmax,
                                    double weight, double* alm, cudaStream_t s) {
-  const size_t smem = sizeof(double) * (size_t)(sh.threads / 32) * kLTile * 33;
+  const size_t smem = sizeof(double2) * (size_t)(sh.threads / 32) * kRowTile * 33;
   cudaError_t e = cudaFuncSetAttribute(k_sht_analysis<RP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   k_sht_analysis<RP><<<dim3(lmax + 1, sh.blocks), sh.threads, smem, s>>>(
@@ -879,7 +872,6 @@ cudaError_t sht_analysis(const double* F, const double* z, int nrings, int lmax,
     if (e != cudaSuccess) return e;
   }
   if (sh.rp == 8) return analysis_launch<8>(sh, F, z, nrings, lmax, weight, alm, s);
-  if (sh.rp == 4) return analysis_launch<4>(sh, F, z, nrings, lmax, weight, alm, s);
   return analysis_launch<2>(sh, F, z, nrings, lmax, weight, alm, s);
 }
 
@@ -890,8 +882,6 @@ cudaError_t sht_synthesis(const double* alm, const double* z, int nrings, int lm
   double2* out = reinterpret_cast<double2*>(G);
   if (sh.rp == 8)
     k_sht_synthesis<8><<<grid, sh.threads, 0, s>>>(a, z, nrings, lmax, out);
-  else if (sh.rp == 4)
-    k_sht_synthesis<4><<<grid, sh.threads, 0, s>>>(a, z, nrings, lmax, out);
   else
     k_sht_synthesis<2><<<grid, sh.threads, 0, s>>>(a, z, nrings, lmax, out);
   note_launch();
