@@ -446,6 +446,12 @@ __global__ void __launch_bounds__(ColCfg<N>::T) k_x_pk_reg(const float2* __restr
   tile.store(a, blockIdx.y, blockIdx.x, gridDim.x);
 }
 
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* smem, const void* global) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(smem)), "l"(global), "n"(BYTES) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // r2c along z, nh = nz/2 = N complex per row, R rows per CTA.
 // With `clear` (the input mesh itself) each input value is overwritten with 0 by the thread
 // that read it, so a density mesh comes out cleared for the next paint.
@@ -518,7 +524,10 @@ __global__ void __launch_bounds__(RowCfg<N>::T) k_rfft_z_reg(const float* in, fl
   }
 }
 
-// c2r along z (unnormalised times `scale`).
+// c2r along z (unnormalised times `scale`). A CTA's input rows are one contiguous block; its
+// threads bring it into shared memory with asynchronous 16-byte copies, so the whole block is
+// in flight at once (a loop of loads, each waited for before its store, left the pass at 2.0
+// TB/s: 384^3 222 -> 98 us, 256^3 41.5 -> 26.6 us, 64^3 6.0 -> 3.7 us).
 template <int N>
 __global__ void __launch_bounds__(RowCfg<N>::T) k_irfft_z_reg(const float2* __restrict__ in, float* __restrict__ out,
                                                               int nrows, float scale, const float2* __restrict__ twg,
@@ -527,23 +536,27 @@ __global__ void __launch_bounds__(RowCfg<N>::T) k_irfft_z_reg(const float2* __re
   constexpr int P = Split<N>::P, Q = Split<N>::Q, R = RowCfg<N>::R, T = RowCfg<N>::T;
   constexpr int S = P * (Q + 1);
   constexpr int IT = (R * P + T - 1) / T;  // stage-1 items per thread
-  extern __shared__ float2 sm[];
-  float2* tw = sm;
-  float2* tw2 = tw + N;
-  float2* xbuf = tw2 + N + 1;  // R*(N+1) input rows, then (aliased) the R*S exchange buffer
+  extern __shared__ __align__(16) float2 sm[];
+  constexpr int XB = (R * (N + 1) > R * S ? R * (N + 1) : R * S);
+  float2* xbuf = sm;  // R*(N+1) input rows, then (aliased) the R*S exchange buffer
   float2* ybuf = xbuf;
+  float2* tw = sm + XB;
+  float2* tw2 = tw + N;
   in += (long long)blockIdx.y * in_b;
   out += (long long)blockIdx.y * out_b;
   const int tid = threadIdx.x;
+  const int row0 = blockIdx.x * R;
+  const int have = min(R, nrows - row0) * (N + 1);  // rows past the last are not read
+  const float2* src = in + (long long)row0 * (N + 1);
+  if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+    for (int w = tid; w < have / 2; w += T) copy_async<16>(xbuf + 2 * w, src + 2 * w);
+    if ((have & 1) && tid == 0) copy_async<8>(xbuf + have - 1, src + have - 1);
+  } else {
+    for (int w = tid; w < have; w += T) copy_async<8>(xbuf + w, src + w);
+  }
   for (int m = tid; m < N; m += T) tw[m] = twg[m];
   for (int m = tid; m <= N; m += T) tw2[m] = twg2[m];
-  const int row0 = blockIdx.x * R;
-  for (int w = tid; w < R * (N + 1); w += T) {
-    const int rr = w / (N + 1);
-    const int k = w - rr * (N + 1);
-    const int row = row0 + rr;
-    xbuf[w] = (row < nrows) ? in[(long long)row * (N + 1) + k] : make_float2(0.f, 0.f);
-  }
+  copy_async_wait();
   __syncthreads();
   float2 u1[IT][Q];
 #pragma unroll
