@@ -506,6 +506,172 @@ __global__ void __launch_bounds__(kForceMeshThreads) k_force_mesh4(const float* 
   }
 }
 
+// ----------------------------------------------------------------------------------
+// LPT at the grid points, four consecutive z cells per thread (nz % 4 == 0, nz >= 8, 16-byte
+// aligned meshes). Every neighbour along x and y is one aligned 16-byte load, the z
+// neighbours are the adjacent groups.
+//
+// The first-order field goes through memory once, as three meshes F_a = -D_a phi_1 (the
+// second-order source is built from it); the displacements and momenta are formed from the
+// two potentials directly. One scalar thread per cell with an interleaved field that was
+// written, read back by the combination and gathered 24 times per cell by the source took
+// 1.86 of the 3.84 ms of 384^3 initial conditions with 2LPT; this form 0.81.
+// ----------------------------------------------------------------------------------
+struct Quad {
+  int i, j, k0;  // cells (i, j, k0 .. k0 + 3)
+};
+
+__device__ __forceinline__ Quad quad_of(const PGrid& g, unsigned q) {
+  Quad c;
+  particle_ijk(g, 4 * q, c.i, c.j, c.k0);
+  return c;
+}
+
+__device__ __forceinline__ float4 quad_at(const float* __restrict__ f, const PGrid& g, int i, int j, int k0) {
+  return __ldg(reinterpret_cast<const float4*>(f + (i * g.yz + j * g.nz + k0)));
+}
+
+// 12 D along x (AX 0), y (1), z (2) of f at the four cells: 8 (f_+1 - f_-1) - (f_+2 - f_-2)
+template <int AX>
+__device__ __forceinline__ void quad_d12(const float* __restrict__ f, const PGrid& g, const Quad& c, float (&d)[4]) {
+  if constexpr (AX == 2) {
+    const float4 m = quad_at(f, g, c.i, c.j, wrap1(c.k0 - 4, g.nz)), o = quad_at(f, g, c.i, c.j, c.k0),
+                 p = quad_at(f, g, c.i, c.j, wrap1(c.k0 + 4, g.nz));
+    const float v[8] = {m.z, m.w, o.x, o.y, o.z, o.w, p.x, p.y};
+#pragma unroll
+    for (int t = 0; t < 4; ++t) d[t] = 8.0f * (v[t + 3] - v[t + 1]) - (v[t + 4] - v[t]);
+  } else {
+    const auto at = [&](int o) {
+      return AX == 0 ? quad_at(f, g, wrap1(c.i + o, g.nx), c.j, c.k0) : quad_at(f, g, c.i, wrap1(c.j + o, g.ny), c.k0);
+    };
+    const float4 m2 = at(-2), m1 = at(-1), p1 = at(1), p2 = at(2);
+    d[0] = 8.0f * (p1.x - m1.x) - (p2.x - m2.x);
+    d[1] = 8.0f * (p1.y - m1.y) - (p2.y - m2.y);
+    d[2] = 8.0f * (p1.z - m1.z) - (p2.z - m2.z);
+    d[3] = 8.0f * (p1.w - m1.w) - (p2.w - m2.w);
+  }
+}
+
+// three meshes F[3][cells] = -D phi
+__global__ void __launch_bounds__(256) k_grad_meshes4(const float* __restrict__ pot, float* __restrict__ F, PGrid g) {
+  const long long b = blockIdx.y;
+  pot += b * g.np;
+  F += b * g.np * 3;
+  const float s = -1.0f / 12.0f;
+  for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < g.np / 4; q += gridDim.x * blockDim.x) {
+    const Quad c = quad_of(g, q);
+    float d[3][4];
+    quad_d12<0>(pot, g, c, d[0]);
+    quad_d12<1>(pot, g, c, d[1]);
+    quad_d12<2>(pot, g, c, d[2]);
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+      reinterpret_cast<float4*>(F + (size_t)a * g.np)[q] =
+          make_float4(d[a][0] * s, d[a][1] * s, d[a][2] * s, d[a][3] * s);
+  }
+}
+
+// the 2LPT source (see k_lpt2_source_grad) from those meshes: phi_ab = -D_b F_a
+__global__ void __launch_bounds__(256) k_lpt2_source4(const float* __restrict__ F, float* __restrict__ out, PGrid g) {
+  const long long b = blockIdx.y;
+  F += b * g.np * 3;
+  out += b * g.np;
+  const float s = -1.0f / 12.0f;
+  for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < g.np / 4; q += gridDim.x * blockDim.x) {
+    const Quad c = quad_of(g, q);
+    const float *fx = F, *fy = F + g.np, *fz = F + 2 * (size_t)g.np;
+    float xx[4], xy[4], xz[4], yy[4], yz[4], zz[4], r[4];
+    quad_d12<0>(fx, g, c, xx);
+    quad_d12<1>(fx, g, c, xy);
+    quad_d12<2>(fx, g, c, xz);
+    quad_d12<1>(fy, g, c, yy);
+    quad_d12<2>(fy, g, c, yz);
+    quad_d12<2>(fz, g, c, zz);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const float hxx = xx[t] * s, hxy = xy[t] * s, hxz = xz[t] * s, hyy = yy[t] * s, hyz = yz[t] * s, hzz = zz[t] * s;
+      // accumulated in the reference's loop order
+      float v = -hxy * hxy;
+      v -= hxz * hxz;
+      v += hyy * hxx;
+      v -= hyz * hyz;
+      v += hzz * (hxx + hyy);
+      r[t] = v;
+    }
+    reinterpret_cast<float4*>(out)[q] = make_float4(r[0], r[1], r[2], r[3]);
+  }
+}
+
+// Stores the four particles of a thread (v[4][3], 12 floats) of a full warp as 3 x 512
+// contiguous bytes: staged through the warp's 96 float4 (thread L writes float4 3 L .. 3 L + 2,
+// a stride of 48 bytes that covers all banks).
+__device__ __forceinline__ void store_particles4(float* __restrict__ out, unsigned q_first, float4* buf,
+                                                 const float (&v)[12]) {
+  const unsigned lane = threadIdx.x & 31;
+  __syncwarp();
+#pragma unroll
+  for (int t = 0; t < 3; ++t) buf[3 * lane + t] = make_float4(v[4 * t], v[4 * t + 1], v[4 * t + 2], v[4 * t + 3]);
+  __syncwarp();
+  float4* dst = reinterpret_cast<float4*>(out) + 3ull * q_first;
+#pragma unroll
+  for (int t = 0; t < 3; ++t) dst[32 * t + lane] = buf[32 * t + lane];
+}
+
+// dx = c1x F1 + c2x F2, p = c1p (c1x F1) + c2p (c2x F2), F = -D pot; pot2 null for order 1
+template <bool SECOND>
+__global__ void __launch_bounds__(256) k_lpt_apply4(const float* __restrict__ pot1, const float* __restrict__ pot2,
+                                                    float c1x, float c2x, float c1p, float c2p, float* __restrict__ dx,
+                                                    float* __restrict__ pv, PGrid g) {
+  __shared__ float4 stage[8][96];
+  const long long b = blockIdx.y;
+  pot1 += b * g.np;
+  if (SECOND) pot2 += b * g.np;
+  dx += b * g.np * 3;
+  pv += b * g.np * 3;
+  const float s = -1.0f / 12.0f;
+  const unsigned nq = g.np / 4, lane = threadIdx.x & 31;
+  for (unsigned q0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); q0 < nq; q0 += gridDim.x * blockDim.x) {
+    const unsigned q = q0 + lane;
+    float x[12], v[12];  // particle t, component a at 3 t + a
+    if (q < nq) {
+      const Quad c = quad_of(g, q);
+      float d1[3][4], d2[3][4];
+      quad_d12<0>(pot1, g, c, d1[0]);
+      quad_d12<1>(pot1, g, c, d1[1]);
+      quad_d12<2>(pot1, g, c, d1[2]);
+      if (SECOND) {
+        quad_d12<0>(pot2, g, c, d2[0]);
+        quad_d12<1>(pot2, g, c, d2[1]);
+        quad_d12<2>(pot2, g, c, d2[2]);
+      }
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          float xx = c1x * (d1[a][t] * s);
+          float vv = c1p * xx;
+          if (SECOND) {
+            const float x2 = c2x * (d2[a][t] * s);
+            xx += x2;
+            vv += c2p * x2;
+          }
+          x[3 * t + a] = xx;
+          v[3 * t + a] = vv;
+        }
+    }
+    if (q0 + 32 <= nq) {
+      store_particles4(dx, q0, stage[threadIdx.x >> 5], x);
+      store_particles4(pv, q0, stage[threadIdx.x >> 5], v);
+    } else if (q < nq) {
+#pragma unroll
+      for (int t = 0; t < 12; ++t) {
+        dx[12ull * q + t] = x[t];
+        pv[12ull * q + t] = v[t];
+      }
+    }
+  }
+}
+
 // F = scale * (-D pot) at every grid point (particles exactly on the grid), optionally
 // accumulated into `out` (AoS [..,3]).
 __global__ void k_grid_gradient(const float* __restrict__ pot, float* __restrict__ out, float scale, int accumulate,
@@ -804,6 +970,34 @@ cudaError_t lpt2_source_adjoint(const float* pot, const float* sbar, float* q, f
   if (e != cudaSuccess) return e;
   k_lpt2_source_adj_apply<<<particle_grid_dims(d.cells(), d.batch, 256, 16), 256, 0, s>>>(q, out, accumulate,
                                                                                          make_pgrid(d));
+  note_launch();
+  return cudaGetLastError();
+}
+
+bool lpt_quads(const MeshDims& d, const float* pot, const float* src, const float* dx, const float* p) {
+  const uintptr_t all = (uintptr_t)pot | (uintptr_t)src | (uintptr_t)dx | (uintptr_t)p;
+  return d.nz % 4 == 0 && d.nz >= 8 && all % 16 == 0;
+}
+
+cudaError_t grad_meshes(const float* pot, float* F, const MeshDims& d, cudaStream_t s) {
+  k_grad_meshes4<<<particle_grid_dims(d.cells() / 4, d.batch, 256, 16), 256, 0, s>>>(pot, F, make_pgrid(d));
+  note_launch();
+  return cudaGetLastError();
+}
+
+cudaError_t lpt2_source_meshes(const float* F, float* out, const MeshDims& d, cudaStream_t s) {
+  k_lpt2_source4<<<particle_grid_dims(d.cells() / 4, d.batch, 256, 16), 256, 0, s>>>(F, out, make_pgrid(d));
+  note_launch();
+  return cudaGetLastError();
+}
+
+cudaError_t lpt_apply(const float* pot1, const float* pot2, float c1x, float c2x, float c1p, float c2p, float* dx,
+                      float* p, const MeshDims& d, cudaStream_t s) {
+  const dim3 grid = particle_grid_dims(d.cells() / 4, d.batch, 256, 16);
+  if (pot2)
+    k_lpt_apply4<true><<<grid, 256, 0, s>>>(pot1, pot2, c1x, c2x, c1p, c2p, dx, p, make_pgrid(d));
+  else
+    k_lpt_apply4<false><<<grid, 256, 0, s>>>(pot1, nullptr, c1x, 0.f, c1p, 0.f, dx, p, make_pgrid(d));
   note_launch();
   return cudaGetLastError();
 }

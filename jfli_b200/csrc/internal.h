@@ -75,6 +75,13 @@ cudaError_t grid_gradient(const float* pot, float* out, float scale, int accumul
 cudaError_t lpt2_source(const float* grad, float* out, const MeshDims& d, cudaStream_t s);
 cudaError_t lpt_combine(const float* f1, const float* f2, float c1x, float c2x, float c1p, float c2p, float* dx,
                         float* p, const MeshDims& d, cudaStream_t s);
+// The same for four z cells per thread, where lpt_quads allows it: F1 as three meshes [3][cells]
+// in the space of dx, the source from them, dx and p from the two potentials (pot2 null: order 1).
+bool lpt_quads(const MeshDims& d, const float* pot, const float* src, const float* dx, const float* p);
+cudaError_t grad_meshes(const float* pot, float* F, const MeshDims& d, cudaStream_t s);
+cudaError_t lpt2_source_meshes(const float* F, float* out, const MeshDims& d, cudaStream_t s);
+cudaError_t lpt_apply(const float* pot1, const float* pot2, float c1x, float c2x, float c1p, float c2p, float* dx,
+                      float* p, const MeshDims& d, cudaStream_t s);
 cudaError_t axpy_particles(float* y, const float* x, float a, const MeshDims& d, cudaStream_t s);
 // q: six scratch meshes; out (+)= dL/dphi1 for sbar = dL/d delta2.
 cudaError_t lpt2_source_adjoint(const float* pot, const float* sbar, float* q, float* out, int accumulate,
