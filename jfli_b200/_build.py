@@ -10,6 +10,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -39,16 +40,21 @@ def _headers():
 def build(verbose: bool = False, force: bool = False) -> Path:
     BUILD.mkdir(exist_ok=True)
     hdr_mtime = max((h.stat().st_mtime for h in _headers()), default=0.0)
-    objs = []
+    objs, cmds = [], []
     for src in _sources():
         obj = BUILD / (src.stem + ".o")
         objs.append(obj)
         if not force and obj.exists() and obj.stat().st_mtime >= max(src.stat().st_mtime, hdr_mtime):
             continue
-        cmd = [NVCC, *FLAGS, "-c", str(src), "-o", str(obj)]
+        cmds.append([NVCC, *FLAGS, "-c", str(src), "-o", str(obj)])
+
+    def compile_one(cmd):
         if verbose:
             print(" ".join(cmd), flush=True)
         subprocess.run(cmd, check=True)
+
+    with ThreadPoolExecutor(os.cpu_count() or 1) as pool:  # the FFT files take minutes one after the other
+        list(pool.map(compile_one, cmds))
     if force or not LIB.exists() or LIB.stat().st_mtime < max(o.stat().st_mtime for o in objs):
         cmd = [NVCC, "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-o", str(LIB), *map(str, objs),
                "-lcudart"]

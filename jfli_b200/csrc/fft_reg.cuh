@@ -112,6 +112,10 @@ struct RegDFT<6, SIGN, TS> {
   static __device__ __forceinline__ void run(float2* v, const float2* tw) { rdft_ab<2, 3, SIGN, TS>(v, tw); }
 };
 template <int SIGN, int TS>
+struct RegDFT<9, SIGN, TS> {
+  static __device__ __forceinline__ void run(float2* v, const float2* tw) { rdft_ab<3, 3, SIGN, TS>(v, tw); }
+};
+template <int SIGN, int TS>
 struct RegDFT<12, SIGN, TS> {
   static __device__ __forceinline__ void run(float2* v, const float2* tw) { rdft_ab<4, 3, SIGN, TS>(v, tw); }
 };
@@ -122,6 +126,14 @@ struct RegDFT<16, SIGN, TS> {
 template <int SIGN, int TS>
 struct RegDFT<24, SIGN, TS> {
   static __device__ __forceinline__ void run(float2* v, const float2* tw) { rdft_ab<8, 3, SIGN, TS>(v, tw); }
+};
+template <int SIGN, int TS>
+struct RegDFT<18, SIGN, TS> {
+  static __device__ __forceinline__ void run(float2* v, const float2* tw) { rdft_ab<2, 9, SIGN, TS>(v, tw); }
+};
+template <int SIGN, int TS>
+struct RegDFT<27, SIGN, TS> {
+  static __device__ __forceinline__ void run(float2* v, const float2* tw) { rdft_ab<3, 9, SIGN, TS>(v, tw); }
 };
 template <int SIGN, int TS>
 struct RegDFT<32, SIGN, TS> {
@@ -152,6 +164,23 @@ JFLI_SPLIT(384, 24, 16)
 JFLI_SPLIT(512, 32, 16)
 JFLI_SPLIT(768, 32, 24)
 JFLI_SPLIT(1024, 32, 32)
+JFLI_SPLIT(18, 6, 3)
+JFLI_SPLIT(27, 9, 3)
+JFLI_SPLIT(36, 6, 6)
+JFLI_SPLIT(54, 9, 6)
+JFLI_SPLIT(72, 9, 8)
+JFLI_SPLIT(81, 9, 9)
+JFLI_SPLIT(108, 12, 9)
+JFLI_SPLIT(144, 12, 12)
+JFLI_SPLIT(162, 18, 9)
+JFLI_SPLIT(216, 18, 12)
+JFLI_SPLIT(243, 27, 9)
+JFLI_SPLIT(288, 18, 16)
+JFLI_SPLIT(324, 18, 18)
+JFLI_SPLIT(432, 24, 18)
+JFLI_SPLIT(486, 27, 18)
+JFLI_SPLIT(576, 24, 24)
+JFLI_SPLIT(648, 27, 24)
 #undef JFLI_SPLIT
 
 // Columns per CTA of a strided column pass of length N.

@@ -23,16 +23,13 @@
 #include "common.cuh"
 #include "fft_reg.cuh"
 #include "internal.h"
+#include "smem_async.cuh"
 
 namespace jfli {
 
 // Set (bit 0) by a kernel whose wait on an mbarrier ran out of its bound; read and cleared
-// by jfli_device_status. (This header is included by fft.cu alone, which owns the word.)
+// by jfli_device_status. (This header is included by fft_x.cu alone, which owns the word.)
 __device__ unsigned g_jfli_status = 0;
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) {
-  return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
