@@ -146,7 +146,9 @@ int jfli_force_adjoint(void* stream, const float* disp, const float* u, float sc
 /* forces[p] = scale * CIC readout of -grad_FD(pot) at the particle positions. */
 int jfli_readout_gradient(void* stream, const float* pos, int absolute, const float* pot, float scale, float* forces,
                           int nx, int ny, int nz, int batch, char* err, size_t errlen);
-/* forces = scale * (paint -> Poisson -> -grad_FD -> readout); jax-fli's _forces uses scale = 1.5 Omega_m. */
+/* forces = scale * (paint -> Poisson -> -grad_FD -> readout); jax-fli's _forces uses scale = 1.5 Omega_m.
+ * The workspace holds a density mesh, a spectrum and a force mesh; one of
+ * jfli_pm_step_workspace_bytes (no force mesh) is taken too, with a slower readout. */
 size_t jfli_pm_forces_workspace_bytes(int nx, int ny, int nz, int batch);
 int jfli_pm_forces(void* stream, const float* pos, int absolute, float scale, float* forces, void* workspace,
                    size_t workspace_bytes, int nx, int ny, int nz, int batch, char* err, size_t errlen);

@@ -247,9 +247,11 @@ int jfli_pgd_potential(void* stream, const float* rho, float rho_mean, float kl,
       "jfli_pgd_potential");
 }
 
+// density / potential mesh, spectrum, force mesh; without the last (a caller short of memory) the
+// forces are read out of the potential by the 56-point stencil
 size_t jfli_pm_forces_workspace_bytes(int nx, int ny, int nz, int batch) {
   const MeshDims d{nx, ny, nz, batch};
-  return mesh_bytes(d) + spec_bytes(d);
+  return mesh_bytes(d) + spec_bytes(d) + align256(sizeof(float) * 4 * (size_t)d.cells() * batch);
 }
 
 int jfli_pm_forces(void* stream, const float* pos, int absolute, float scale, float* forces, void* workspace,
@@ -261,16 +263,24 @@ int jfli_pm_forces(void* stream, const float* pos, int absolute, float scale, fl
   CHECK_PTR(forces);
   CHECK_PTR(workspace);
   const MeshDims d{nx, ny, nz, batch};
-  if (workspace_bytes < jfli_pm_forces_workspace_bytes(nx, ny, nz, batch))
-    return fail(err, errlen, JFLI_EINVAL, "workspace too small: %zu < %zu bytes", workspace_bytes,
-                jfli_pm_forces_workspace_bytes(nx, ny, nz, batch));
+  const size_t least = mesh_bytes(d) + spec_bytes(d);
+  if (workspace_bytes < least)
+    return fail(err, errlen, JFLI_EINVAL, "workspace too small: %zu < %zu bytes", workspace_bytes, least);
   cudaStream_t s = (cudaStream_t)stream;
   float* rho = (float*)workspace;  // the potential overwrites the density in place
   float2* spec = (float2*)((char*)workspace + mesh_bytes(d));
+  float* force = (float*)((char*)workspace + least);
+  const bool meshes = workspace_bytes >= jfli_pm_forces_workspace_bytes(nx, ny, nz, batch) &&
+                      ((uintptr_t)workspace) % 16 == 0;
   cudaError_t e = cudaMemsetAsync(rho, 0, (size_t)d.cells() * batch * sizeof(float), s);
   if (e == cudaSuccess) e = jfli::cic_paint(pos, absolute, nullptr, 1.0f, rho, d, s);
   if (e == cudaSuccess) e = jfli::poisson_potential(rho, spec, rho, d, 1.0f, 1.0f, s);
-  if (e == cudaSuccess) e = jfli::cic_readout_gradient(pos, absolute, rho, forces, scale, d, s);
+  if (meshes) {
+    if (e == cudaSuccess) e = jfli::force_mesh(rho, force, scale, d, s);
+    if (e == cudaSuccess) e = jfli::cic_readout_force(pos, absolute, force, forces, d, s);
+  } else if (e == cudaSuccess) {
+    e = jfli::cic_readout_gradient(pos, absolute, rho, forces, scale, d, s);
+  }
   return cuda_status(e, err, errlen, "jfli_pm_forces");
 }
 

@@ -161,6 +161,15 @@ struct XCarry {
 // weights to lane L+1, which adds them to its own lower-z deposits. Lanes with `on` false
 // deposit nothing and take part in no merge. Cell offsets are unique per cell, so equal
 // offsets mean equal cells.
+//
+// A lane that merges with neither neighbour has two adjacent cells of its own per y row: with VEC
+// (rows of a multiple of 4 cells, mesh 16-byte aligned) they go out as one 16-byte vector
+// atomic with zeros beside them, unless they lie in two aligned groups of four. On particles
+// that left their neighbours the paint is bound by the atomics' path: 216 x 144 x 324 in
+// absolute positions 269 -> 239 us, the particle pass of 256^3 347 -> 344 us over 40 steps.
+// (For every lane, merged or not: 259 and 385 us, as the merged rows' 4-byte atomics coalesce;
+// with 8-byte atomics at even cells: 239 and 364 us.)
+template <bool VEC>
 __device__ __forceinline__ void deposit_plane_merged(float* rho, bool on, int xo, int yo0, int yo1, int z0, int z1,
                                                      float w00, float w01, float w10, float w11) {
   const int lane = threadIdx.x & 31;
@@ -173,11 +182,21 @@ __device__ __forceinline__ void deposit_plane_merged(float* rho, bool on, int xo
   const float r0 = __shfl_up_sync(0xffffffffu, w01, 1);
   const float r1 = __shfl_up_sync(0xffffffffu, w11, 1);
   if (on) {
-    atomicAdd(rho + (xo + yo0 + z0), take ? w00 + r0 : w00);
-    atomicAdd(rho + (xo + yo1 + z0), take ? w10 + r1 : w10);
-    if (!give) {
-      atomicAdd(rho + (xo + yo0 + z1), w01);
-      atomicAdd(rho + (xo + yo1 + z1), w11);
+    if (VEC && !give && !take && (z0 & 3) != 3) {
+      const int q = z0 & 3;
+      const float4 a = make_float4(q == 0 ? w00 : 0.f, q == 0 ? w01 : (q == 1 ? w00 : 0.f),
+                                   q == 1 ? w01 : (q == 2 ? w00 : 0.f), q == 2 ? w01 : 0.f);
+      const float4 b = make_float4(q == 0 ? w10 : 0.f, q == 0 ? w11 : (q == 1 ? w10 : 0.f),
+                                   q == 1 ? w11 : (q == 2 ? w10 : 0.f), q == 2 ? w11 : 0.f);
+      atomicAdd(reinterpret_cast<float4*>(rho + (xo + yo0 + z0 - q)), a);
+      atomicAdd(reinterpret_cast<float4*>(rho + (xo + yo1 + z0 - q)), b);
+    } else {
+      atomicAdd(rho + (xo + yo0 + z0), take ? w00 + r0 : w00);
+      atomicAdd(rho + (xo + yo1 + z0), take ? w10 + r1 : w10);
+      if (!give) {
+        atomicAdd(rho + (xo + yo0 + z1), w01);
+        atomicAdd(rho + (xo + yo1 + z1), w11);
+      }
     }
   }
 }
@@ -195,9 +214,11 @@ __device__ __forceinline__ void carry_flush(float* rho, XCarry& c) {
 // plane is deposited now, with the carried upper-x plane of the lane's previous particle
 // added when the cells are the same (otherwise the carry is deposited on its own first),
 // and the upper-x plane becomes the new carry. The sums reaching each cell are those of
-// deposit(); only the FP32 addition order differs.
+// deposit(); only the FP32 addition order differs. Lanes with `on` false have no particle (in
+// any plane of the walk) and take part in the shuffles only.
+template <bool VEC>
 __device__ __forceinline__ void deposit_carried(float* rho, const PGrid& g, const Cic1& cx, const Cic1& cy,
-                                                const Cic1& cz, float w, XCarry& c) {
+                                                const Cic1& cz, float w, XCarry& c, bool on = true) {
   const float wx0 = cx.w0 * w, wx1 = cx.w1 * w;
   const int xo0 = cx.i0 * g.yz, yo0 = cy.i0 * g.nz, yo1 = cy.i1 * g.nz;
   float a00 = (wx0 * cy.w0) * cz.w0, a01 = (wx0 * cy.w0) * cz.w1;
@@ -212,7 +233,7 @@ __device__ __forceinline__ void deposit_carried(float* rho, const PGrid& g, cons
       carry_flush(rho, c);
     }
   }
-  deposit_plane_merged(rho, true, xo0, yo0, yo1, cz.i0, cz.i1, a00, a01, a10, a11);
+  deposit_plane_merged<VEC>(rho, on, xo0, yo0, yo1, cz.i0, cz.i1, a00, a01, a10, a11);
   c.xo = cx.i1 * g.yz;
   c.yo0 = yo0;
   c.yo1 = yo1;
@@ -222,7 +243,142 @@ __device__ __forceinline__ void deposit_carried(float* rho, const PGrid& g, cons
   c.w01 = (wx1 * cy.w0) * cz.w1;
   c.w10 = (wx1 * cy.w1) * cz.w0;
   c.w11 = (wx1 * cy.w1) * cz.w1;
-  c.valid = true;
+  c.valid = on;
+}
+
+// The walk of the paint and force readout: a warp takes a z row's segment of kw <= 32
+// consecutive particles and walks it along x for `depth` planes; the CTA's eight warps take
+// eight neighbouring rows in y. Neighbours that share CIC corners are then handled close in
+// time on one SM, and the paint can use the z and x merges of the brick walk, on any mesh.
+struct SegWalk {
+  int kw, nkb, njb, nxc, depth;
+};
+
+// Segments are of equal length; used where they fill at least three quarters of their lanes
+// (rows of 24 particles or more), the grid-stride kernels elsewhere.
+static bool seg_walk(const MeshDims& d, SegWalk* w) {
+  w->nkb = (d.nz + 31) / 32;
+  w->kw = (d.nz + w->nkb - 1) / w->nkb;
+  w->njb = (d.ny + 7) / 8;
+  w->depth = 16;
+  while (w->depth > 1 && (long long)w->nkb * w->njb * d.batch * ((d.nx + w->depth - 1) / w->depth) < 4ll * sm_count())
+    w->depth >>= 1;
+  w->nxc = (d.nx + w->depth - 1) / w->depth;
+  return 4 * d.nz >= 3 * 32 * w->nkb;
+}
+
+static dim3 seg_grid(const MeshDims& d, const SegWalk& w) {
+  const long long items = (long long)w.nkb * w.njb * w.nxc, cap = 16ll * sm_count();
+  return dim3((unsigned)(items < cap ? items : cap), d.batch);
+}
+
+// body(p, i, j, k, on) for every plane of every segment of this warp; flush() after each segment
+template <class Body, class Flush>
+__device__ __forceinline__ void walk_segments(const PGrid& g, const SegWalk& w, Body body, Flush flush) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned items = (unsigned)w.nkb * (unsigned)w.njb * (unsigned)w.nxc;
+  for (unsigned it = blockIdx.x; it < items; it += gridDim.x) {
+    const int kb = (int)(it % (unsigned)w.nkb);
+    const unsigned rest = it / (unsigned)w.nkb;
+    const int j = (int)(rest % (unsigned)w.njb) * 8 + warp, i0 = (int)(rest / (unsigned)w.njb) * w.depth;
+    if (j >= g.ny) continue;
+    const int k = kb * w.kw + lane;
+    const bool on = lane < w.kw && k < g.nz;
+    const int i1 = min(g.nx, i0 + w.depth);
+    for (int i = i0; i < i1; ++i)
+      body(((unsigned)i * (unsigned)g.ny + (unsigned)j) * (unsigned)g.nz + (unsigned)k, i, j, k, on);
+    flush();
+  }
+}
+
+__device__ __forceinline__ void cic_at(const float* __restrict__ pos, int absolute, const PGrid& g, unsigned p, int i,
+                                       int j, int k, Cic1& cx, Cic1& cy, Cic1& cz) {
+  const float px = __ldcs(pos + 3ull * p), py = __ldcs(pos + 3ull * p + 1), pz = __ldcs(pos + 3ull * p + 2);
+  if (absolute) {
+    cx = cic_abs(px, g.nx);
+    cy = cic_abs(py, g.ny);
+    cz = cic_abs(pz, g.nz);
+  } else {
+    cx = cic_rel(i, px, g.nx);
+    cy = cic_rel(j, py, g.ny);
+    cz = cic_rel(k, pz, g.nz);
+  }
+}
+
+// CIC paint. Bound by the atomics' path (L2 at 75% with the grid-stride kernel). 216 x 144 x 324
+// particles in absolute positions: 279 us grid-stride, 269 with the x merge, 239 with the
+// vector atomics of deposit_plane_merged.
+template <bool VEC>
+__global__ void __launch_bounds__(256) k_paint_walk(const float* __restrict__ pos, int absolute,
+                                                    const float* __restrict__ weights, float weight,
+                                                    float* __restrict__ mesh, PGrid g, SegWalk walk) {
+  const long long b = blockIdx.y;
+  pos += b * g.np * 3;
+  mesh += b * g.np;
+  if (weights) weights += b * g.np;
+  XCarry carry;
+  carry.valid = false;
+  carry.xo = carry.yo0 = carry.yo1 = carry.z0 = carry.z1 = 0;
+  carry.w00 = carry.w01 = carry.w10 = carry.w11 = 0.f;
+  walk_segments(
+      g, walk,
+      [&](unsigned p, int i, int j, int k, bool on) {
+        Cic1 cx = {0, 0, 0.f, 0.f}, cy = cx, cz = cx;
+        float w = 0.f;
+        if (on) {
+          cic_at(pos, absolute, g, p, i, j, k, cx, cy, cz);
+          w = weights ? weights[p] * weight : weight;
+        }
+        deposit_carried<VEC>(mesh, g, cx, cy, cz, w, carry, on);
+      },
+      [&] {
+        deposit_plane_merged<VEC>(mesh, carry.valid, carry.xo, carry.yo0, carry.yo1, carry.z0, carry.z1, carry.w00,
+                             carry.w01, carry.w10, carry.w11);
+        carry.valid = false;
+      });
+}
+
+// forces[p] = CIC readout of the float4 force mesh (jfli_pm_forces): 8 loads of 16 bytes per
+// particle against the 56 scalar loads of k_readout_gradient's stencil. 216 x 144 x 324: the
+// stencil 509 us; force mesh 44 + this kernel 143.
+__global__ void __launch_bounds__(256) k_readout_force_walk(const float* __restrict__ pos, int absolute,
+                                                            const float* __restrict__ force, float* __restrict__ out,
+                                                            PGrid g, SegWalk walk) {
+  const long long b = blockIdx.y;
+  pos += b * g.np * 3;
+  force += b * g.np * 4;
+  out += b * g.np * 3;
+  walk_segments(
+      g, walk,
+      [&](unsigned p, int i, int j, int k, bool on) {
+        if (!on) return;
+        Cic1 cx, cy, cz;
+        cic_at(pos, absolute, g, p, i, j, k, cx, cy, cz);
+        float fx, fy, fz;
+        gather_force_mesh(force, g, cx, cy, cz, fx, fy, fz);
+        __stcs(out + 3ull * p + 0, fx);
+        __stcs(out + 3ull * p + 1, fy);
+        __stcs(out + 3ull * p + 2, fz);
+      },
+      [] {});
+}
+
+__global__ void __launch_bounds__(256) k_readout_force(const float* __restrict__ pos, int absolute,
+                                                       const float* __restrict__ force, float* __restrict__ out,
+                                                       PGrid g) {
+  const long long b = blockIdx.y;
+  pos += b * g.np * 3;
+  force += b * g.np * 4;
+  out += b * g.np * 3;
+  for (unsigned p = blockIdx.x * blockDim.x + threadIdx.x; p < g.np; p += gridDim.x * blockDim.x) {
+    Cic1 cx, cy, cz;
+    cic_setup(pos + 3ull * p, p, absolute, g, cx, cy, cz);
+    float fx, fy, fz;
+    gather_force_mesh(force, g, cx, cy, cz, fx, fy, fz);
+    out[3ull * p + 0] = fx;
+    out[3ull * p + 1] = fy;
+    out[3ull * p + 2] = fz;
+  }
 }
 
 // Kick (with the CIC readout of the force mesh at the current position), drift (with the
@@ -333,7 +489,7 @@ __device__ __forceinline__ void kdp_brick_row(float* __restrict__ disp, float* _
   }
   if (flags & kStepPaint) {
     const Cic1 cx = cic_rel(i, x0, g.nx), cy = cic_rel(j, x1, g.ny), cz = cic_rel(k, x2, g.nz);
-    deposit_carried(rho, g, cx, cy, cz, weight, carry);
+    deposit_carried<true>(rho, g, cx, cy, cz, weight, carry);
   }
 }
 
@@ -365,7 +521,8 @@ __global__ void __launch_bounds__(256, 4) k_kick_drift_paint(float* __restrict__
   if (rho) rho += b * g.np;
   __shared__ float4 rowbuf[kBrickY][2][24];  // per warp: positions, velocities of one z row
   if (blockDim.x == kBrickY * kBrickZ && g.nz % kBrickZ == 0 && g.ny % kBrickY == 0 &&
-      ((reinterpret_cast<uintptr_t>(disp) | reinterpret_cast<uintptr_t>(vel)) & 15) == 0) {
+      ((reinterpret_cast<uintptr_t>(disp) | reinterpret_cast<uintptr_t>(vel) | reinterpret_cast<uintptr_t>(rho)) & 15) ==
+          0) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int tz = g.nz / kBrickZ, ty = g.ny / kBrickY, txc = (g.nx + xdepth - 1) / xdepth;
     const long long items = (long long)tz * ty * txc;
@@ -389,7 +546,7 @@ __global__ void __launch_bounds__(256, 4) k_kick_drift_paint(float* __restrict__
         kdp_brick_row(disp, vel, force, kick, drift, flags, weight, rho, g, p0, i, j, k, lane, rowbuf[w][0],
                       rowbuf[w][1], carry, xa, va, i + 1 < i1, p0 + row_stride);
       // every lane of the warp ran the same planes: the carries go out together, z-merged
-      deposit_plane_merged(rho, carry.valid, carry.xo, carry.yo0, carry.yo1, carry.z0, carry.z1, carry.w00,
+      deposit_plane_merged<true>(rho, carry.valid, carry.xo, carry.yo0, carry.yo1, carry.z0, carry.z1, carry.w00,
                            carry.w01, carry.w10, carry.w11);
     }
     return;
@@ -873,7 +1030,16 @@ __global__ void k_axpy(float* __restrict__ y, const float* __restrict__ x, float
 // ----------------------------------------------------------------------------------
 cudaError_t cic_paint(const float* pos, int absolute, const float* weights, float weight, float* mesh,
                       const MeshDims& d, cudaStream_t s) {
-  k_paint<<<particle_grid_dims(d.cells(), d.batch, 256, 16), 256, 0, s>>>(pos, absolute, weights, weight, mesh, make_pgrid(d));
+  SegWalk w;
+  if (seg_walk(d, &w)) {
+    if (d.nz % 4 == 0 && (uintptr_t)mesh % 16 == 0)
+      k_paint_walk<true><<<seg_grid(d, w), 256, 0, s>>>(pos, absolute, weights, weight, mesh, make_pgrid(d), w);
+    else
+      k_paint_walk<false><<<seg_grid(d, w), 256, 0, s>>>(pos, absolute, weights, weight, mesh, make_pgrid(d), w);
+  } else {
+    k_paint<<<particle_grid_dims(d.cells(), d.batch, 256, 16), 256, 0, s>>>(pos, absolute, weights, weight, mesh,
+                                                                            make_pgrid(d));
+  }
   note_launch();
   return cudaGetLastError();
 }
@@ -889,6 +1055,18 @@ cudaError_t cic_readout_gradient(const float* pos, int absolute, const float* po
                                  const MeshDims& d, cudaStream_t s) {
   k_readout_gradient<<<particle_grid_dims(d.cells(), d.batch, 256, 16), 256, 0, s>>>(pos, absolute, pot, out, scale,
                                                                                      make_pgrid(d));
+  note_launch();
+  return cudaGetLastError();
+}
+
+cudaError_t cic_readout_force(const float* pos, int absolute, const float* force, float* out, const MeshDims& d,
+                              cudaStream_t s) {
+  SegWalk w;
+  if (seg_walk(d, &w))
+    k_readout_force_walk<<<seg_grid(d, w), 256, 0, s>>>(pos, absolute, force, out, make_pgrid(d), w);
+  else
+    k_readout_force<<<particle_grid_dims(d.cells(), d.batch, 256, 16), 256, 0, s>>>(pos, absolute, force, out,
+                                                                                    make_pgrid(d));
   note_launch();
   return cudaGetLastError();
 }

@@ -63,6 +63,9 @@ cudaError_t cic_readout(const float* pos, int absolute, const float* mesh, float
                         cudaStream_t s);
 cudaError_t cic_readout_gradient(const float* pos, int absolute, const float* pot, float* out, float scale,
                                  const MeshDims& d, cudaStream_t s);
+// forces of a float4 force mesh (the force_mesh layout) at the particles
+cudaError_t cic_readout_force(const float* pos, int absolute, const float* force, float* out, const MeshDims& d,
+                              cudaStream_t s);
 cudaError_t kick_drift_paint(float* disp, float* vel, const float* force, float kick, float drift, int flags,
                              float weight, float* rho, const MeshDims& d, cudaStream_t s);
 cudaError_t force_mesh(const float* pot, float* force, float scale, const MeshDims& d, cudaStream_t s);

@@ -167,7 +167,10 @@ def pm_forces(pos: torch.Tensor, *, absolute: bool = False, scale: float = 1.0) 
     (nx, ny, nz), batch, lead = _mesh_dims(pos, True)
     out = torch.empty_like(pos)
     nb = query("jfli_pm_forces_workspace_bytes", nx, ny, nz, batch)
-    ws = workspace(nb, "forces", pos.device)
+    try:
+        ws = workspace(nb, "forces", pos.device)
+    except torch.cuda.OutOfMemoryError:  # without room for the force mesh: the density and the spectrum alone
+        ws = workspace(query("jfli_pm_step_workspace_bytes", nx, ny, nz, batch), "forces", pos.device)
     call("jfli_pm_forces", stream_ptr(), ptr(pos), int(absolute), float(scale), ptr(out), ptr(ws), ws.numel(), nx,
          ny, nz, batch)
     return out
