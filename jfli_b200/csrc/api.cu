@@ -466,12 +466,12 @@ int jfli_lpt(void* stream, const float* ic, int order, float c1x, float c2x, flo
   float* src = (float*)(w + spec_bytes(d) + mesh_bytes(d));
   float* f2 = (float*)(w + spec_bytes(d) + 2 * mesh_bytes(d));
   // first order: phi1 = laplace^-1 ic, F1 = -D phi1 at the grid points (written to dx)
-  cudaError_t e = jfli::poisson_potential(ic, spec, pot, d, 0.0f, 1.0f, s);
+  cudaError_t e = jfli::poisson_potential(ic, spec, pot, d, 0.0f, 1.0f, s, nullptr, false);
   if (jfli::lpt_quads(d, pot, src, dx, p)) {
     if (e == cudaSuccess && order == 2) {
       e = jfli::grad_meshes(pot, dx, d, s);
       if (e == cudaSuccess) e = jfli::lpt2_source_meshes(dx, src, d, s);
-      if (e == cudaSuccess) e = jfli::poisson_potential(src, spec, src, d, 0.0f, 1.0f, s);  // phi2 in place
+      if (e == cudaSuccess) e = jfli::poisson_potential(src, spec, src, d, 0.0f, 1.0f, s, nullptr, false);  // phi2 in place
     }
     if (e == cudaSuccess) e = jfli::lpt_apply(pot, order == 2 ? src : nullptr, c1x, c2x, c1p, c2p, dx, p, d, s);
     return cuda_status(e, err, errlen, "jfli_lpt");
@@ -479,7 +479,7 @@ int jfli_lpt(void* stream, const float* ic, int order, float c1x, float c2x, flo
   if (e == cudaSuccess) e = jfli::grid_gradient(pot, dx, 1.0f, 0, d, s);
   if (e == cudaSuccess && order == 2) {
     e = jfli::lpt2_source(dx, src, d, s);
-    if (e == cudaSuccess) e = jfli::poisson_potential(src, spec, pot, d, 0.0f, 1.0f, s);
+    if (e == cudaSuccess) e = jfli::poisson_potential(src, spec, pot, d, 0.0f, 1.0f, s, nullptr, false);
     if (e == cudaSuccess) e = jfli::grid_gradient(pot, f2, 1.0f, 0, d, s);
   }
   if (e == cudaSuccess) e = jfli::lpt_combine(dx, order == 2 ? f2 : nullptr, c1x, c2x, c1p, c2p, dx, p, d, s);
@@ -513,11 +513,11 @@ int jfli_lpt_lightcone(void* stream, const float* ic, int order, const double* t
   float* src = (float*)(w + spec_bytes(d) + mesh_bytes(d));
   float* f2 = (float*)(w + spec_bytes(d) + 2 * mesh_bytes(d));
   float* f1 = (float*)(w + jfli_lpt_workspace_bytes(nx, ny, nz, batch));
-  cudaError_t e = jfli::poisson_potential(ic, spec, pot, d, 0.0f, 1.0f, s);
+  cudaError_t e = jfli::poisson_potential(ic, spec, pot, d, 0.0f, 1.0f, s, nullptr, false);
   if (e == cudaSuccess) e = jfli::grid_gradient(pot, f1, 1.0f, 0, d, s);
   if (e == cudaSuccess && order == 2) {
     e = jfli::lpt2_source(f1, src, d, s);
-    if (e == cudaSuccess) e = jfli::poisson_potential(src, spec, pot, d, 0.0f, 1.0f, s);
+    if (e == cudaSuccess) e = jfli::poisson_potential(src, spec, pot, d, 0.0f, 1.0f, s, nullptr, false);
     if (e == cudaSuccess) e = jfli::grid_gradient(pot, f2, 1.0f, 0, d, s);
   }
   jfli::LptLightcone lc;

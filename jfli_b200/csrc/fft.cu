@@ -123,29 +123,29 @@ cudaError_t rfft3d_inverse(float2* spec, float* out, const MeshDims& d, float sc
   return launch_irfft_z(spec, out, d, scale, s);
 }
 
-// real mesh -> (forward 3D FFT, k-space op, inverse 3D FFT) -> real mesh.
+// real mesh -> (forward 3D FFT, k-space op, inverse 3D FFT) -> real mesh. `mixed`: see reg_fft_length
 template <class Op>
 static cudaError_t filter_chain(const float* in, float2* spec, float* out, const MeshDims& d, float sub, const Op& op,
-                                cudaStream_t s, float* clear = nullptr) {
-  cudaError_t e = launch_rfft_z(in, spec, d, sub, s, clear);
+                                cudaStream_t s, float* clear = nullptr, bool mixed = true) {
+  cudaError_t e = launch_rfft_z(in, spec, d, sub, s, clear, mixed);
   if (e != cudaSuccess) return e;
-  e = launch_cols(-1, spec, y_geom(d), d.spec_elems(), d.batch, s);
+  e = launch_cols(-1, spec, y_geom(d), d.spec_elems(), d.batch, s, mixed);
   if (e != cudaSuccess) return e;
-  e = launch_x_op(spec, d, op, s);
+  e = launch_x_op(spec, d, op, s, mixed);
   if (e != cudaSuccess) return e;
-  e = launch_cols(1, spec, y_geom(d), d.spec_elems(), d.batch, s);
+  e = launch_cols(1, spec, y_geom(d), d.spec_elems(), d.batch, s, mixed);
   if (e != cudaSuccess) return e;
-  return launch_irfft_z(spec, out, d, 1.0f, s);
+  return launch_irfft_z(spec, out, d, 1.0f, s, mixed);
 }
 
 cudaError_t poisson_potential(const float* rho, float2* spec, float* pot, const MeshDims& d, float rho_mean,
-                              float scale, cudaStream_t s, float* clear) {
+                              float scale, cudaStream_t s, float* clear, bool mixed) {
   PoissonOp op;
   op.nx = d.nx;
   op.ny = d.ny;
   op.nz = d.nz;
   op.norm = scale / ((float)d.nx * (float)d.ny * (float)d.nz);
-  return filter_chain(rho, spec, pot, d, rho_mean, op, s, clear);
+  return filter_chain(rho, spec, pot, d, rho_mean, op, s, clear, mixed);
 }
 
 cudaError_t pgd_potential(const float* rho, float2* spec, float* pot, const MeshDims& d, float rho_mean, float kl,
@@ -184,7 +184,7 @@ cudaError_t ic_filter(const float* noise, float2* spec, float* out, const MeshDi
   op.factor = (float)(((double)d.nx * d.ny * d.nz) / ((double)box[0] * box[1] * box[2]));
   op.norm = 1.0f / ((float)d.nx * (float)d.ny * (float)d.nz);
   op.zero_mode_one = zero_mode_one;
-  return filter_chain(noise, spec, out, d, 0.0f, op, s);
+  return filter_chain(noise, spec, out, d, 0.0f, op, s, nullptr, false);
 }
 
 cudaError_t power_adjoint(const float* mesh, float2* spec, float* out, const MeshDims& d, const float* kedges,

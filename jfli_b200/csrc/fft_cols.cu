@@ -113,8 +113,8 @@ static cudaError_t cols_generic_sign(float2* data, const ColGeom& g, long long b
 }
 
 template <int SIGN>
-static cudaError_t cols_sign(float2* data, const ColGeom& g, long long bstride, int batch, cudaStream_t s) {
-  switch (g.n) {
+static cudaError_t cols_sign(float2* data, const ColGeom& g, long long bstride, int batch, cudaStream_t s, bool mixed) {
+  switch (reg_fft_length(g.n, mixed)) {
 #define JFLI_CASE(N_) \
   case N_:            \
     return cols_reg<N_, SIGN>(data, g, bstride, batch, s);
@@ -127,8 +127,9 @@ static cudaError_t cols_sign(float2* data, const ColGeom& g, long long bstride, 
   return cols_generic_sign<SIGN>(data, g, bstride, batch, s);
 }
 
-cudaError_t launch_cols(int sign, float2* data, const ColGeom& g, long long bstride, int batch, cudaStream_t s) {
-  return sign < 0 ? cols_sign<-1>(data, g, bstride, batch, s) : cols_sign<1>(data, g, bstride, batch, s);
+cudaError_t launch_cols(int sign, float2* data, const ColGeom& g, long long bstride, int batch, cudaStream_t s,
+                        bool mixed) {
+  return sign < 0 ? cols_sign<-1>(data, g, bstride, batch, s, mixed) : cols_sign<1>(data, g, bstride, batch, s, mixed);
 }
 
 cudaError_t cols_generic(int sign, float2* data, const ColGeom& g, long long bstride, int batch, cudaStream_t s) {

@@ -118,7 +118,7 @@ static cudaError_t x_op_tma(float2* data, const MeshDims& d, const Op& op, bool*
 }
 
 template <class Op>
-static cudaError_t x_op(float2* data, const MeshDims& d, const Op& op, cudaStream_t s) {
+static cudaError_t x_op(float2* data, const MeshDims& d, const Op& op, cudaStream_t s, bool mixed) {
   const ColGeom g = x_geom(d);
   if constexpr (Op::kInverse) {
     if (x_pass_mode() == 1) {
@@ -146,10 +146,12 @@ static cudaError_t x_op(float2* data, const MeshDims& d, const Op& op, cudaStrea
     default:
       break;
   }
-  if constexpr (std::is_same_v<Op, PoissonOp> || std::is_same_v<Op, IcOp>) {
-    bool done = false;
-    const cudaError_t e = launch_x_op_mixed(data, d, op, &done, s);
-    if (done || e != cudaSuccess) return e;
+  if constexpr (std::is_same_v<Op, PoissonOp>) {
+    if (mixed) {
+      bool done = false;
+      const cudaError_t e = launch_x_op_mixed(data, d, op, &done, s);
+      if (done || e != cudaSuccess) return e;
+    }
   }
   FftPlan pl;
   make_fft_plan(g.n, &pl);
@@ -161,9 +163,17 @@ static cudaError_t x_op(float2* data, const MeshDims& d, const Op& op, cudaStrea
   return cudaGetLastError();
 }
 
-cudaError_t launch_x_op(float2* data, const MeshDims& d, const PoissonOp& op, cudaStream_t s) { return x_op(data, d, op, s); }
-cudaError_t launch_x_op(float2* data, const MeshDims& d, const PgdOp& op, cudaStream_t s) { return x_op(data, d, op, s); }
-cudaError_t launch_x_op(float2* data, const MeshDims& d, const IcOp& op, cudaStream_t s) { return x_op(data, d, op, s); }
-cudaError_t launch_x_op(float2* data, const MeshDims& d, const PkAdjOp& op, cudaStream_t s) { return x_op(data, d, op, s); }
+cudaError_t launch_x_op(float2* data, const MeshDims& d, const PoissonOp& op, cudaStream_t s, bool mixed) {
+  return x_op(data, d, op, s, mixed);
+}
+cudaError_t launch_x_op(float2* data, const MeshDims& d, const PgdOp& op, cudaStream_t s, bool mixed) {
+  return x_op(data, d, op, s, mixed);
+}
+cudaError_t launch_x_op(float2* data, const MeshDims& d, const IcOp& op, cudaStream_t s, bool mixed) {
+  return x_op(data, d, op, s, mixed);
+}
+cudaError_t launch_x_op(float2* data, const MeshDims& d, const PkAdjOp& op, cudaStream_t s, bool mixed) {
+  return x_op(data, d, op, s, mixed);
+}
 
 }  // namespace jfli

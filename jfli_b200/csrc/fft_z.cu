@@ -317,8 +317,8 @@ cudaError_t rfft_z_generic(const float* in, float2* out, const MeshDims& d, floa
 }
 
 cudaError_t launch_rfft_z(const float* in, float2* out, const MeshDims& d, float sub, cudaStream_t s,
-                          float* clear) {
-  switch (d.nz / 2) {
+                          float* clear, bool mixed) {
+  switch (reg_fft_length(d.nz / 2, mixed)) {
 #define JFLI_CASE(N_) \
   case N_:            \
     return rfft_z_reg<N_>(in, out, d, sub, s, clear);
@@ -333,8 +333,9 @@ cudaError_t launch_rfft_z(const float* in, float2* out, const MeshDims& d, float
   return e;
 }
 
-cudaError_t launch_irfft_z(const float2* in, float* out, const MeshDims& d, float scale, cudaStream_t s) {
-  switch (d.nz / 2) {
+cudaError_t launch_irfft_z(const float2* in, float* out, const MeshDims& d, float scale, cudaStream_t s,
+                           bool mixed) {
+  switch (reg_fft_length(d.nz / 2, mixed)) {
 #define JFLI_CASE(N_) \
   case N_:            \
     return irfft_z_reg<N_>(in, out, d, scale, s);

@@ -25,9 +25,10 @@ cudaError_t rfft3d_forward(const float* in, float2* spec, const MeshDims& d, flo
 cudaError_t rfft3d_inverse(float2* spec, float* out, const MeshDims& d, float scale, cudaStream_t s);
 cudaError_t rfft2d_forward(const float* in, float2* spec, const MeshDims& d, cudaStream_t s);  // d.nx == 1
 // clear: the density mesh (rho itself), set to 0 by the r2c pass once read, so the next
-// paint needs no memset; nullptr leaves rho as it is.
+// paint needs no memset; nullptr leaves rho as it is. mixed: register passes on the mixed
+// lengths too (false where particles are laid out: reg_fft_length has the reason).
 cudaError_t poisson_potential(const float* rho, float2* spec, float* pot, const MeshDims& d, float rho_mean,
-                              float scale, cudaStream_t s, float* clear = nullptr);
+                              float scale, cudaStream_t s, float* clear = nullptr, bool mixed = true);
 cudaError_t pgd_potential(const float* rho, float2* spec, float* pot, const MeshDims& d, float rho_mean, float kl,
                           float ks, float scale, cudaStream_t s);
 // pot_k = delta_k (-1/k^2) (c0 + c1 PGD filter) * scale: (0, 1) is pgd_potential, (kick, boost)
