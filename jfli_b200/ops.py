@@ -13,7 +13,6 @@ from __future__ import annotations
 
 import collections
 import ctypes
-import functools
 import math
 
 import numpy as np
@@ -428,27 +427,16 @@ def healpix_paint_shells_adjoint(pos: torch.Tensor, maps_bar: torch.Tensor, nsid
     return pos_bar
 
 
-@functools.lru_cache(maxsize=64)
-def _drift_tables_host(cosmo, n_dense: int) -> tuple:
-    """FP32 host copies of the FP64 tables the light-cone drift interpolates, as the growth and
-    distance tables they come from kept per cosmology: (chi ascending, a at chi), (growth a,
-    D1), (dense a, dGfa)."""
+def drift_tables(cosmo, n_dense: int = 4096):
+    """Device FP32 copies of the FP64 host tables the light-cone drift interpolates:
+    (chi ascending, a at chi), (growth a, D1), (dense a, dGfa)."""
     from . import cosmology as cj
 
     dt = cj.distance_table(cosmo)
     gt = cj.growth_table(cosmo)
     da = np.logspace(-3.0, 0.0, n_dense)
     tabs = (dt.chi[::-1], dt.a[::-1], gt.a, gt.g, da, cj.dGfa(cosmo, da))
-    return tuple(np.ascontiguousarray(t, dtype=np.float32) for t in tabs)
-
-
-def drift_tables(cosmo, n_dense: int = 4096):
-    """Device FP32 copies of the FP64 host tables the light-cone drift interpolates:
-    (chi ascending, a at chi), (growth a, D1), (dense a, dGfa). One pinned copy that the host
-    does not wait for."""
-    host = _drift_tables_host(cosmo, n_dense)
-    flat = torch.from_numpy(np.concatenate(host)).pin_memory().to("cuda", non_blocking=True)
-    return torch.split(flat, [t.size for t in host])
+    return tuple(torch.as_tensor(np.ascontiguousarray(t, dtype=np.float32), device="cuda") for t in tabs)
 
 
 def replica_positions(pos: torch.Tensor, box_size, observer_mpc, rotation, shift, *, absolute: bool = False,
@@ -580,8 +568,8 @@ def _tiled_prep(pos, rotations, shifts, scheme, vel, t, cosmo, tables, dbound):
     tabs = drift_tables(cosmo) if tables is None else tables
     t_arg = float(t)
     gp_t = float(cj.Gp(cosmo, t_arg))
-    if dbound is None:  # from the host's copies where there are: reading the device's would wait for the stream
-        dbound = drift_bound(_drift_tables_host(cosmo, 4096) if tables is None else tabs, t_arg, gp_t)
+    if dbound is None:
+        dbound = drift_bound(tabs, t_arg, gp_t)
     return sch, rot, sh, tabs, t_arg, gp_t, (dbound if math.isfinite(dbound) else 1e30)
 
 
