@@ -311,10 +311,16 @@ def exported_symbols() -> list[str]:
     return list(_SIGNATURES)
 
 
+_errors = threading.local()  # one message buffer per thread: the call that fills it also reads it
+
+
 def call(name: str, *args):
     """Call an entry point that ends with (err, errlen); raise JfliError on failure."""
-    lib = load()
-    buf = ctypes.create_string_buffer(512)
+    lib = _lib if _device_ok else load()
+    buf = getattr(_errors, "buf", None)
+    if buf is None:
+        buf = _errors.buf = ctypes.create_string_buffer(512)
+    buf[0] = b"\0"
     rc = getattr(lib, name)(*args, buf, 512)
     if rc != 0:
         raise JfliError(name, rc, buf.value.decode(errors="replace"))
@@ -323,12 +329,15 @@ def call(name: str, *args):
 
 def query(name: str, *args):
     """Call a pure query entry point (no error buffer)."""
-    return getattr(load(check_device=False), name)(*args)
+    lib = _lib if _lib is not None else load(check_device=False)
+    return getattr(lib, name)(*args)
 
 
 def stream_ptr(stream: torch.cuda.Stream | None = None) -> int:
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    # the handle itself: a Stream object around it costs 5 us, as much as a kernel launch
+    if stream is None:
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    return stream.cuda_stream
 
 
 def ptr(t: torch.Tensor | None) -> int | None:

@@ -119,7 +119,8 @@ def interp(x, xp, fp):
     x = np.asarray(x, dtype=np.float64)
     xp = np.asarray(xp, dtype=np.float64)
     fp = np.asarray(fp, dtype=np.float64)
-    i = np.clip(np.searchsorted(xp, x) - 1, 0, len(xp) - 2)
+    # minimum of maximum rather than np.clip, whose checks cost more than the whole lookup of a scalar
+    i = np.minimum(np.maximum(np.searchsorted(xp, x) - 1, 0), len(xp) - 2)
     slope = (fp[i + 1] - fp[i]) / (xp[i + 1] - xp[i])
     return fp[i] + (x - xp[i]) * slope
 
@@ -180,7 +181,7 @@ def growth_table(c: Cosmology, log10_amin: float = -3.0, steps: int = 128) -> Gr
 
 def growth_factor(c: Cosmology, a):
     t = growth_table(c)
-    return np.clip(interp(a, t.a, t.g), 0.0, 1.0)
+    return np.minimum(np.maximum(interp(a, t.a, t.g), 0.0), 1.0)
 
 
 def growth_rate(c: Cosmology, a):
@@ -253,7 +254,7 @@ def distance_table(c: Cosmology, log10_amin: float = -3.0, steps: int = 256) -> 
 
 def radial_comoving_distance(c: Cosmology, a):
     t = distance_table(c)
-    return np.clip(interp(a, t.a, t.chi), 0.0, 1e6)
+    return np.minimum(np.maximum(interp(a, t.a, t.chi), 0.0), 1e6)
 
 
 def a_of_chi(c: Cosmology, chi):

@@ -13,6 +13,7 @@ from __future__ import annotations
 
 import collections
 import ctypes
+import functools
 import math
 
 import numpy as np
@@ -27,9 +28,9 @@ _workspaces: dict[tuple, torch.Tensor] = {}
 def workspace(nbytes: int, key: str = "default", device=None) -> torch.Tensor:
     """A cached uint8 device buffer of at least `nbytes`, one per key, device and current
     stream, so that work enqueued on different streams never shares scratch space."""
-    dev = torch.device("cuda") if device is None else torch.device(device)
+    dev = torch.device("cuda" if device is None else device)
     idx = dev.index if dev.index is not None else torch.cuda.current_device()
-    k = (key, idx, torch.cuda.current_stream(idx).cuda_stream)
+    k = (key, idx, torch._C._cuda_getCurrentRawStream(idx))
     buf = _workspaces.get(k)
     if buf is None or buf.numel() < nbytes:
         buf = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=dev)
@@ -41,14 +42,16 @@ _TABLES: "collections.OrderedDict[tuple, torch.Tensor]" = collections.OrderedDic
 
 
 def device_table(values, device="cuda", dtype=np.float32) -> torch.Tensor:
-    """A small host table (bin edges, P(k) samples) on the device, cached by content and
-    read-only for callers. A copy from pageable host memory makes the host wait until the
+    """A small host table (bin edges, P(k) samples) on the device, cached by content (and by
+    the stream it went up on, so that no other stream reads it too early) and read-only for
+    callers. A copy from pageable host memory makes the host wait until the
     stream has drained, which stalls a caller that enqueues the next request while the GPU
     works on this one: a table met before is reused, a new one goes up through pinned
     memory without blocking."""
     a = np.ascontiguousarray(np.asarray(values, dtype=dtype))
     dev = torch.device(device)
-    key = (a.tobytes(), a.shape, a.dtype.str, str(dev))
+    stream = stream_ptr() if dev.type == "cuda" else 0
+    key = (a.tobytes(), a.shape, a.dtype.str, str(dev), stream)
     t = _TABLES.get(key)
     if t is None:
         t = torch.from_numpy(a.copy())
@@ -71,8 +74,7 @@ def _mesh_dims(t: torch.Tensor, particle: bool):
     if len(core) != 3:
         raise ValueError(f"bad {'particle' if particle else 'mesh'} tensor shape {shape}")
     lead = shape[:-4] if particle else shape[:-3]
-    batch = int(np.prod(lead)) if lead else 1
-    return tuple(int(v) for v in core), batch, lead
+    return tuple(int(v) for v in core), math.prod(lead), lead
 
 
 def _check(t: torch.Tensor, name: str, dtype=torch.float32):
@@ -427,16 +429,27 @@ def healpix_paint_shells_adjoint(pos: torch.Tensor, maps_bar: torch.Tensor, nsid
     return pos_bar
 
 
-def drift_tables(cosmo, n_dense: int = 4096):
-    """Device FP32 copies of the FP64 host tables the light-cone drift interpolates:
-    (chi ascending, a at chi), (growth a, D1), (dense a, dGfa)."""
+@functools.lru_cache(maxsize=64)
+def _drift_tables_host(cosmo, n_dense: int) -> tuple:
+    """FP32 host copies of the FP64 tables the light-cone drift interpolates, as the growth and
+    distance tables they come from kept per cosmology: (chi ascending, a at chi), (growth a,
+    D1), (dense a, dGfa)."""
     from . import cosmology as cj
 
     dt = cj.distance_table(cosmo)
     gt = cj.growth_table(cosmo)
     da = np.logspace(-3.0, 0.0, n_dense)
     tabs = (dt.chi[::-1], dt.a[::-1], gt.a, gt.g, da, cj.dGfa(cosmo, da))
-    return tuple(torch.as_tensor(np.ascontiguousarray(t, dtype=np.float32), device="cuda") for t in tabs)
+    return tuple(np.ascontiguousarray(t, dtype=np.float32) for t in tabs)
+
+
+def drift_tables(cosmo, n_dense: int = 4096):
+    """Device FP32 copies of the FP64 host tables the light-cone drift interpolates:
+    (chi ascending, a at chi), (growth a, D1), (dense a, dGfa). One pinned copy that the host
+    does not wait for."""
+    host = _drift_tables_host(cosmo, n_dense)
+    flat = torch.from_numpy(np.concatenate(host)).pin_memory().to("cuda", non_blocking=True)
+    return torch.split(flat, [t.size for t in host])
 
 
 def replica_positions(pos: torch.Tensor, box_size, observer_mpc, rotation, shift, *, absolute: bool = False,
@@ -568,8 +581,8 @@ def _tiled_prep(pos, rotations, shifts, scheme, vel, t, cosmo, tables, dbound):
     tabs = drift_tables(cosmo) if tables is None else tables
     t_arg = float(t)
     gp_t = float(cj.Gp(cosmo, t_arg))
-    if dbound is None:
-        dbound = drift_bound(tabs, t_arg, gp_t)
+    if dbound is None:  # from the host's copies where there are: reading the device's would wait for the stream
+        dbound = drift_bound(_drift_tables_host(cosmo, 4096) if tables is None else tabs, t_arg, gp_t)
     return sch, rot, sh, tabs, t_arg, gp_t, (dbound if math.isfinite(dbound) else 1e30)
 
 

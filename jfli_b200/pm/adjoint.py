@@ -398,7 +398,7 @@ class PowerSpectrum(torch.autograd.Function):
     @staticmethod
     def forward(ctx, mesh, kedges: np.ndarray, box):
         mesh = mesh.contiguous()
-        ke = _dev(kedges)
+        ke = ops.device_table(kedges, mesh.device)  # a pageable copy would wait for the steps before it
         sums = ops.power_sums(mesh, ke, box)
         cnt = sums[1]
         vol = float(np.prod(np.asarray(box, np.float64) / np.asarray(mesh.shape[-3:], np.float64)))
@@ -436,7 +436,7 @@ class PowerPoles(torch.autograd.Function):
         vol = float(np.prod(np.asarray(box, np.float64) / np.asarray(mesh.shape[-3:], np.float64)))
         norm = torch.where(cnt > 0, cnt, torch.ones_like(cnt))
         pk = (re / norm[None, :])[:, 1:-1] * vol
-        ctx.save_for_backward(mesh, _dev(kedges), cnt)
+        ctx.save_for_backward(mesh, ops.device_table(kedges, mesh.device), cnt)
         ctx.vol, ctx.box, ctx.poles, ctx.los = vol, box, tuple(int(p) for p in poles), los
         return pk[0] if nell == 1 else pk
 

@@ -241,10 +241,16 @@ def run_differentiable(solver, dx: ParticleField, p: ParticleField, cosmo, ts, t
             paint_boosts = np.concatenate([[0.0], np.atleast_1d(b)])
             boosts = paint_boosts[:-1]
     else:
-        cs = [solver.step_coefficients(cosmo, a, b, dt0, t0) for a, b in steps]
-        kicks, drifts = np.array([c.kick for c in cs]), np.array([c.drift for c in cs])
+        if type(solver).step_coefficients is ReversibleDoubleKickDrift.step_coefficients:
+            # all steps in one evaluation of the growth tables, as in run_fused: step by step it took
+            # 4 of the 8.5 ms of a 128^3 gradient through 20 steps, with the GPU idle
+            kicks, drifts = ReversibleDoubleKickDrift.schedule_arrays(cosmo, [a for a, _ in steps],
+                                                                      [b for _, b in steps], dt0, t0)
+        else:
+            cs = [solver.step_coefficients(cosmo, a, b, dt0, t0) for a, b in steps]
+            kicks, drifts = np.array([c.kick for c in cs]), np.array([c.drift for c in cs])
         if sharpen is not None:
-            boosts = np.array([sharpen.boost(c.drift) for c in cs], np.float64)
+            boosts = np.array([sharpen.boost(d) for d in drifts], np.float64)
     tables = ForwardTables(ktab=None, ptab=None, lpt=None, kicks=np.asarray(kicks, np.float64),
                            drifts=np.asarray(drifts, np.float64),
                            sharpen=None if sharpen is None else (boosts, float(sharpen.kl), float(sharpen.ks)))

@@ -56,7 +56,7 @@ class AbstractInterp:
         reference's time variables and of jnp.isin on its FP32 ts (pm/interp.py:148): the
         time loop clips each step to the FP32 value of the next snapshot time, so the FP64
         shell times (from the distance table) only match after the same rounding."""
-        return self.ts is not None and bool(np.isin(np.float32(t), np.asarray(self.ts, np.float32)))
+        return self.ts is not None and bool((np.asarray(self.ts, np.float32) == np.float32(t)).any())
 
     def advance(self, state: InterpTilerState, t) -> InterpTilerState:
         return dataclasses.replace(state, shell_idx=state.shell_idx + 1) if self._is_snapshot(t) else state
