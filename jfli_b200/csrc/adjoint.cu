@@ -291,6 +291,8 @@ cudaError_t paint_vec4(const float* disp, const float* u, float* ubar, const Mes
 __global__ void k_div_fd(const float* __restrict__ u, float alpha, const float* __restrict__ w, float beta,
                          long long cell_stride, long long comp_stride, int accumulate, float* __restrict__ out,
                          PGrid g) {
+  grid_release();
+  grid_wait();
   const long long b = blockIdx.y;
   u += b * g.np * 3;
   if (w) w += b * g.np * 3;
@@ -414,6 +416,8 @@ size_t adjoint_partials_count(const MeshDims& d) { return (size_t)2 * adj_grid(d
 // slice, then a shared-memory tree in a fixed order (deterministic).
 __global__ void __launch_bounds__(256) k_sum_partials(const double* __restrict__ partials, int nctas,
                                                       double* __restrict__ out) {
+  grid_release();
+  grid_wait();
   __shared__ double sk[256], sd[256];
   const double* p = partials + 2ll * nctas * blockIdx.x;
   double a = 0.0, c = 0.0;
@@ -438,7 +442,8 @@ __global__ void __launch_bounds__(256) k_sum_partials(const double* __restrict__
 }
 
 cudaError_t sum_adjoint_partials(const double* partials, const MeshDims& d, double* out, cudaStream_t s) {
-  k_sum_partials<<<d.batch, 256, 0, s>>>(partials, (int)adj_grid(d).x, out);
+  launch_next(overlap_starts(d.cells() * d.batch), k_sum_partials, d.batch, 256, 0, s, partials, (int)adj_grid(d).x,
+              out);
   note_launch();
   return cudaGetLastError();
 }
@@ -467,8 +472,8 @@ cudaError_t divergence_fd(const float* u, float alpha, const float* w, float bet
   // aos 0: three meshes; 1: particle grids (3 floats per cell); 2: float4 meshes
   const long long cell_stride = aos == 2 ? 4 : (aos ? 3 : 1);
   const long long comp_stride = aos ? 1 : d.cells();
-  k_div_fd<<<particle_grid_dims(d.cells(), d.batch, 256, 16), 256, 0, s>>>(u, alpha, w, beta, cell_stride, comp_stride,
-                                                                          accumulate, out, make_pgrid(d));
+  launch_next(overlap_starts(d.cells() * d.batch), k_div_fd, particle_grid_dims(d.cells(), d.batch, 256, 16), 256, 0, s,
+              u, alpha, w, beta, cell_stride, comp_stride, accumulate, out, make_pgrid(d));
   note_launch();
   return cudaGetLastError();
 }

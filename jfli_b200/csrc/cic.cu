@@ -598,6 +598,8 @@ constexpr int kForceMeshThreads = 256;
 
 __global__ void __launch_bounds__(kForceMeshThreads) k_force_mesh4(const float* __restrict__ pot,
                                                                    float* __restrict__ F, float scale, PGrid g) {
+  grid_release();
+  grid_wait();
   const long long b = blockIdx.y;
   pot += b * g.np;
   F += b * g.np * 4;
@@ -1008,6 +1010,8 @@ __global__ void k_lpt_combine(const float* __restrict__ f1, const float* __restr
 
 // Zero n floats (16-byte stores where the pointer allows; the tail element by element).
 __global__ void k_zero(float* __restrict__ y, long long n) {
+  grid_release();
+  grid_wait();
   const long long n4 = ((reinterpret_cast<uintptr_t>(y) & 15) == 0) ? n / 4 : 0;
   float4* y4 = reinterpret_cast<float4*>(y);
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -1017,7 +1021,7 @@ __global__ void k_zero(float* __restrict__ y, long long n) {
 }
 
 cudaError_t zero_floats(float* y, long long n, cudaStream_t s) {
-  k_zero<<<particle_grid_dims((n + 3) / 4, 1, 256, 16), 256, 0, s>>>(y, n);
+  launch_next(overlap_starts(n), k_zero, particle_grid_dims((n + 3) / 4, 1, 256, 16), 256, 0, s, y, n);
   note_launch();
   return cudaGetLastError();
 }
@@ -1118,8 +1122,9 @@ cudaError_t kick_drift_paint_slots(float* disp, float* vel, const float* force, 
 cudaError_t force_mesh(const float* pot, float* force, float scale, const MeshDims& d, cudaStream_t s) {
   const bool vec4 = d.nz % 4 == 0 && d.nz >= 8 && ((uintptr_t)pot % 16) == 0 && ((uintptr_t)force % 16) == 0;
   if (vec4)
-    k_force_mesh4<<<particle_grid_dims(d.cells() / 4, d.batch, kForceMeshThreads, 16), kForceMeshThreads, 0, s>>>(
-        pot, force, scale, make_pgrid(d));
+    launch_next(overlap_starts(d.cells() * d.batch), k_force_mesh4,
+                particle_grid_dims(d.cells() / 4, d.batch, kForceMeshThreads, 16), kForceMeshThreads, 0, s, pot, force,
+                scale, make_pgrid(d));
   else
     k_force_mesh<<<particle_grid_dims(d.cells(), d.batch, 256, 16), 256, 0, s>>>(pot, force, scale, make_pgrid(d));
   note_launch();

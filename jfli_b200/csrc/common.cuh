@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "launch.cuh"
+
 namespace jfli {
 
 constexpr int kFftThreads = 256;     // threads per FFT CTA

@@ -54,6 +54,8 @@ __global__ void __launch_bounds__(ColCfg<N>::T) k_cols_reg(float2* __restrict__ 
   float2* ybuf = sm + N;
   data += (long long)blockIdx.y * bstride;
   const int tid = threadIdx.x;
+  grid_release();
+  grid_wait();
   for (int m = tid; m < N; m += T) tw[m] = twg[m];
   __syncthreads();
   const int c0 = blockIdx.x * W;
@@ -95,7 +97,8 @@ static cudaError_t cols_reg(float2* data, const ColGeom& g, long long bstride, i
   if (!tw) return cudaErrorMemoryAllocation;
   const size_t smem = ((size_t)N + (size_t)N * W) * sizeof(float2);
   cudaFuncSetAttribute(k_cols_reg<N, SIGN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_cols_reg<N, SIGN><<<dim3((g.ncols + W - 1) / W, batch), T, smem, s>>>(data, g, tw, bstride);
+  launch_next(overlap_starts(2 * bstride * batch), k_cols_reg<N, SIGN>, dim3((g.ncols + W - 1) / W, batch), T, smem, s,
+              data, g, tw, bstride);
   note_launch();
   return cudaGetLastError();
 }

@@ -108,8 +108,10 @@ __global__ void __launch_bounds__(ColCfg<N>::T) k_x_op_tma(const __grid_constant
   const int batch = blockIdx.y;
   const int tid = threadIdx.x;
   const int c0 = blockIdx.x * W;
+  grid_release();
+  if (tid == 0) mbar_init(&bar, 1);
+  grid_wait();
   if (tid == 0) {
-    mbar_init(&bar, 1);
     mbar_expect_tx(&bar, (unsigned)TmaCfg<N>::tile_bytes);
 #pragma unroll
     for (int b = 0; b < TmaCfg<N>::BOXES; ++b)

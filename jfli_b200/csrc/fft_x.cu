@@ -111,7 +111,8 @@ static cudaError_t x_op_tma(float2* data, const MeshDims& d, const Op& op, bool*
   const size_t smem = TmaCfg<N>::tile_bytes * 2 + sizeof(float2) * (size_t)N + Op::smem_bytes(op);
   cudaError_t e = cudaFuncSetAttribute(k_x_op_tma<N, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k_x_op_tma<N, Op><<<dim3((g.ncols + W - 1) / W, d.batch), T, smem, s>>>(map, g, tw, op);
+  launch_next(overlap_starts(d.cells() * d.batch), k_x_op_tma<N, Op>, dim3((g.ncols + W - 1) / W, d.batch), T, smem, s,
+              map, g, tw, op);
   note_launch();
   *done = true;
   return cudaGetLastError();

@@ -17,6 +17,8 @@ __global__ void __launch_bounds__(ColCfg<N>::T) k_x_op_reg(float2* __restrict__ 
   const int batch = blockIdx.y;
   data += (long long)batch * bstride;
   const int tid = threadIdx.x;
+  grid_release();
+  grid_wait();
   for (int m = tid; m < N; m += T) tw[m] = twg[m];
   op.prologue(opsm, batch);  // ends with __syncthreads()
   const int c0 = blockIdx.x * W;
@@ -92,7 +94,8 @@ static cudaError_t x_op_reg(float2* data, const ColGeom& g, const Op& op, long l
   if (!tw) return cudaErrorMemoryAllocation;
   const size_t smem = ((size_t)N + (size_t)N * W) * sizeof(float2) + Op::smem_bytes(op);
   cudaFuncSetAttribute(k_x_op_reg<N, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_x_op_reg<N, Op><<<dim3((g.ncols + W - 1) / W, batch), T, smem, s>>>(data, g, tw, op, bstride);
+  launch_next(overlap_starts(2 * bstride * batch), k_x_op_reg<N, Op>, dim3((g.ncols + W - 1) / W, batch), T, smem, s,
+              data, g, tw, op, bstride);
   note_launch();
   return cudaGetLastError();
 }

@@ -140,6 +140,8 @@ __global__ void __launch_bounds__(RowCfg<N>::T) k_rfft_z_reg(const float* in, fl
   out += (long long)blockIdx.y * out_b;
   if (clear) clear += (long long)blockIdx.y * in_b;
   const int tid = threadIdx.x;
+  grid_release();
+  grid_wait();
   for (int m = tid; m < N; m += T) tw[m] = twg[m];
   for (int m = tid; m <= N; m += T) tw2[m] = twg2[m];
   __syncthreads();
@@ -218,6 +220,8 @@ __global__ void __launch_bounds__(RowCfg<N>::T) k_irfft_z_reg(const float2* __re
   const int row0 = blockIdx.x * R;
   const int have = min(R, nrows - row0) * (N + 1);  // rows past the last are not read
   const float2* src = in + (long long)row0 * (N + 1);
+  grid_release();
+  grid_wait();
   if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
     for (int w = tid; w < have / 2; w += T) copy_async<16>(xbuf + 2 * w, src + 2 * w);
     if ((have & 1) && tid == 0) copy_async<8>(xbuf + have - 1, src + have - 1);
@@ -279,8 +283,8 @@ static cudaError_t rfft_z_reg(const float* in, float2* out, const MeshDims& d, f
   const int nrows = d.nx * d.ny;
   const size_t smem = ((size_t)N + N + 1 + (size_t)R * P * (Q + 1)) * sizeof(float2);
   cudaFuncSetAttribute(k_rfft_z_reg<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_rfft_z_reg<N><<<dim3((nrows + R - 1) / R, d.batch), T, smem, s>>>(in, out, nrows, sub, tw, tw2, d.cells(),
-                                                                       d.spec_elems(), clear);
+  launch_next(overlap_starts(d.cells() * d.batch), k_rfft_z_reg<N>, dim3((nrows + R - 1) / R, d.batch), T, smem, s, in,
+              out, nrows, sub, tw, tw2, d.cells(), d.spec_elems(), clear);
   note_launch();
   return cudaGetLastError();
 }
@@ -295,8 +299,8 @@ static cudaError_t irfft_z_reg(const float2* in, float* out, const MeshDims& d, 
   const size_t rows_buf = (size_t)R * P * (Q + 1) > (size_t)R * (N + 1) ? (size_t)R * P * (Q + 1) : (size_t)R * (N + 1);
   const size_t smem = ((size_t)N + N + 1 + rows_buf) * sizeof(float2);
   cudaFuncSetAttribute(k_irfft_z_reg<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_irfft_z_reg<N><<<dim3((nrows + R - 1) / R, d.batch), T, smem, s>>>(in, out, nrows, scale, tw, tw2,
-                                                                        d.spec_elems(), d.cells());
+  launch_next(overlap_starts(d.cells() * d.batch), k_irfft_z_reg<N>, dim3((nrows + R - 1) / R, d.batch), T, smem, s, in,
+              out, nrows, scale, tw, tw2, d.spec_elems(), d.cells());
   note_launch();
   return cudaGetLastError();
 }
