@@ -412,6 +412,13 @@ int jfli_sht_map2alm(void* stream, const double* F, const double* z, int nrings,
                      double* alm, char* err, size_t errlen);
 int jfli_sht_alm2map(void* stream, const double* alm, const double* z, int nrings, int lmax, double* G, char* err,
                      size_t errlen);
+/* Both stages for nmaps RING maps at once (map after map, as F, G and alm): alm of the maps with
+ * the quadrature weight 4 pi / npix and z of the 4 nside - 1 rings, and the maps of alm. F and G
+ * are scratch, nmaps (4 nside - 1)(lmax + 1) complex values. */
+int jfli_sht_maps2alm(void* stream, const double* maps, const double* z, int nside, int lmax, int nmaps, double* F,
+                      double* alm, char* err, size_t errlen);
+int jfli_sht_alm2maps(void* stream, const double* alm, const double* z, int nside, int lmax, int nmaps, double* G,
+                      double* maps, char* err, size_t errlen);
 /* Variant of the x pass of the Poisson, PGD and initial-condition filter chains (the
  * forward x FFT, k-space operator and inverse x FFT in one read and write of the half
  * spectrum): 0 (default) loads each pencil tile from global memory into registers; 1

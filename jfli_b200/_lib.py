@@ -136,6 +136,8 @@ _SIGNATURES = {
     "jfli_sht_ring_analysis": (c_int, [c_void_p, c_void_p, c_int, c_int, c_void_p, *_ERR]),
     "jfli_sht_ring_synthesis": (c_int, [c_void_p, c_void_p, c_int, c_int, c_void_p, *_ERR]),
     "jfli_sht_alm2map": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, *_ERR]),
+    "jfli_sht_maps2alm": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, *_ERR]),
+    "jfli_sht_alm2maps": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, *_ERR]),
     "jfli_sht_alm2cl": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, *_ERR]),
     "jfli_set_fft_x_pass": (c_int, [c_int, *_ERR]),
     "jfli_zero": (c_int, [c_void_p, c_void_p, ctypes.c_longlong, *_ERR]),

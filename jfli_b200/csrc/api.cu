@@ -1108,6 +1108,37 @@ int jfli_sht_alm2map(void* stream, const double* alm, const double* z, int nring
                      "jfli_sht_alm2map");
 }
 
+int jfli_sht_maps2alm(void* stream, const double* maps, const double* z, int nside, int lmax, int nmaps, double* F,
+                      double* alm, char* err, size_t errlen) {
+  CHECK_PTR(maps);
+  CHECK_PTR(z);
+  CHECK_PTR(F);
+  CHECK_PTR(alm);
+  if (nside < 1 || nside > 4096) return fail(err, errlen, JFLI_EINVAL, "nside %d outside [1, 4096]", nside);
+  if (lmax < 0 || lmax > 8191) return fail(err, errlen, JFLI_EINVAL, "lmax %d outside [0, 8191]", lmax);
+  if (nmaps < 1 || nmaps > 65535) return fail(err, errlen, JFLI_EINVAL, "nmaps %d outside [1, 65535]", nmaps);
+  cudaStream_t s = (cudaStream_t)stream;
+  const double weight = 4.0 * 3.14159265358979323846 / (12.0 * nside * nside);
+  cudaError_t e = jfli::sht_ring_analysis(maps, nside, lmax, F, s, nmaps);
+  if (e == cudaSuccess) e = jfli::sht_analysis(F, z, 4 * nside - 1, lmax, weight, alm, s, nmaps);
+  return cuda_status(e, err, errlen, "jfli_sht_maps2alm");
+}
+
+int jfli_sht_alm2maps(void* stream, const double* alm, const double* z, int nside, int lmax, int nmaps, double* G,
+                      double* maps, char* err, size_t errlen) {
+  CHECK_PTR(alm);
+  CHECK_PTR(z);
+  CHECK_PTR(G);
+  CHECK_PTR(maps);
+  if (nside < 1 || nside > 4096) return fail(err, errlen, JFLI_EINVAL, "nside %d outside [1, 4096]", nside);
+  if (lmax < 0 || lmax > 8191) return fail(err, errlen, JFLI_EINVAL, "lmax %d outside [0, 8191]", lmax);
+  if (nmaps < 1 || nmaps > 65535) return fail(err, errlen, JFLI_EINVAL, "nmaps %d outside [1, 65535]", nmaps);
+  cudaStream_t s = (cudaStream_t)stream;
+  cudaError_t e = jfli::sht_synthesis(alm, z, 4 * nside - 1, lmax, G, s, nmaps);
+  if (e == cudaSuccess) e = jfli::sht_ring_synthesis(G, nside, lmax, maps, s, nmaps);
+  return cuda_status(e, err, errlen, "jfli_sht_alm2maps");
+}
+
 int jfli_zero(void* stream, float* data, long long n, char* err, size_t errlen) {
   CHECK_PTR(data);
   if (n < 0) return fail(err, errlen, JFLI_EINVAL, "n must be >= 0");

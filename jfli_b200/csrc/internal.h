@@ -136,11 +136,13 @@ cudaError_t born_flat(const float* maps, int nplanes, int n0, int n1, const floa
                       const float* s1, float* out, double* partials, float* mean, cudaStream_t s);
 
 // ---- sht.cu ----
+// nmaps transforms per launch, maps, F, G and alm one after the other
 cudaError_t sht_analysis(const double* F, const double* z, int nrings, int lmax, double weight, double* alm,
-                         cudaStream_t s);
-cudaError_t sht_synthesis(const double* alm, const double* z, int nrings, int lmax, double* G, cudaStream_t s);
-cudaError_t sht_ring_analysis(const double* map, int nside, int lmax, double* F, cudaStream_t s);
-cudaError_t sht_ring_synthesis(const double* G, int nside, int lmax, double* map, cudaStream_t s);
+                         cudaStream_t s, int nmaps = 1);
+cudaError_t sht_synthesis(const double* alm, const double* z, int nrings, int lmax, double* G, cudaStream_t s,
+                          int nmaps = 1);
+cudaError_t sht_ring_analysis(const double* map, int nside, int lmax, double* F, cudaStream_t s, int nmaps = 1);
+cudaError_t sht_ring_synthesis(const double* G, int nside, int lmax, double* map, cudaStream_t s, int nmaps = 1);
 cudaError_t sht_alm2cl(const double* alm1, const double* alm2, int lmax, double* cl, cudaStream_t s);
 cudaError_t zero_floats(float* y, long long n, cudaStream_t s);
 // x pass of the Poisson / PGD / IC filter chains: 0 register pass, 1 TMA-staged pass

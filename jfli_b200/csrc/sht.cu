@@ -194,6 +194,8 @@ __global__ void __launch_bounds__(kLegendreThreads, kLegendreCtas<RP>) k_sht_ana
   __shared__ double2 part[kLegendreWarps][kLegendreWarps * kLTile];
   extern __shared__ double2 rows[];  // per warp [16 l][33]
   const int m = blockIdx.x;
+  F += (long long)blockIdx.z * nrings * (lmax + 1);
+  alm += blockIdx.z * alm_offset(lmax + 1, lmax);
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double2* row = rows + (size_t)warp * kRowTile * 33;
   const RingPairs rp{nrings, (nrings + 1) / 2};
@@ -324,6 +326,8 @@ __global__ void __launch_bounds__(kLegendreThreads, kLegendreCtas<RP>) k_sht_syn
   __shared__ double2 a_tile[kLegendreWarps * kLTile];  // alpha_l a_lm
   __shared__ double scratch[kLegendreWarps];
   const int m = blockIdx.x;
+  alm += blockIdx.z * alm_offset(lmax + 1, lmax);
+  G += (long long)blockIdx.z * nrings * (lmax + 1);
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const RingPairs rp{nrings, (nrings + 1) / 2};
   const int first = blockIdx.y * (blockDim.x * RP);
@@ -413,16 +417,18 @@ __global__ void __launch_bounds__(kLegendreThreads, kLegendreCtas<RP>) k_sht_syn
 
 // Pairs per thread and threads of a CTA. Eight pairs per thread (eight independent chains, the
 // least reduction and table work per pair) for large maps; two for small ones, whose 3 nside
-// CTAs do not fill the SMs for long and end on the serial chain of their first m (four maps of
-// nside 256: 2 pairs 3.6 ms, 4 pairs 4.0, 8 pairs 4.5).
+// CTAs do not fill the SMs for long and end on the serial chain of their first m, unless
+// several maps go together. a_lm with three refinements, 2 against 8 pairs: nside 512 5.1 and
+// 4.4 ms, nside 256 0.94 and 1.07 (two maps together 1.72 and 1.60, four 3.26 and 3.08), four of
+// nside 128 0.69 and 0.85.
 struct LegendreShape {
   int rp, threads, blocks;
 };
 
-static LegendreShape legendre_shape(int nrings) {
+static LegendreShape legendre_shape(int nrings, int nmaps) {
   const int pairs = (nrings + 1) / 2;
   LegendreShape s;
-  s.rp = pairs >= 1024 ? 8 : 2;
+  s.rp = pairs >= 1024 || (pairs >= 512 && nmaps >= 2) ? 8 : 2;
   int warps = (pairs + 32 * s.rp - 1) / (32 * s.rp);
   s.blocks = (warps + kLegendreWarps - 1) / kLegendreWarps;
   warps = (warps + s.blocks - 1) / s.blocks;
@@ -479,6 +485,8 @@ __global__ void __launch_bounds__(kRingThreads) k_ring_analysis(const double* __
                                                                 double2* __restrict__ F) {
   extern __shared__ double ring[];
   const int r = blockIdx.y;
+  map += blockIdx.z * 12LL * nside * nside;
+  F += (long long)blockIdx.z * gridDim.y * (lmax + 1);
   const RingPhi g = ring_phi(r, nside);
   for (int j = threadIdx.x; j < g.n; j += blockDim.x) ring[j] = map[g.start + j];
   __syncthreads();
@@ -511,6 +519,8 @@ __global__ void __launch_bounds__(kRingThreads) k_ring_synthesis(const double2* 
                                                                  double* __restrict__ map) {
   extern __shared__ double2 coef[];
   const int r = blockIdx.y;
+  map += blockIdx.z * 12LL * nside * nside;
+  G += (long long)blockIdx.z * gridDim.y * (lmax + 1);
   const RingPhi g = ring_phi(r, nside);
   for (int m = threadIdx.x; m <= lmax; m += blockDim.x) coef[m] = G[(long long)r * (lmax + 1) + m];
   __syncthreads();
@@ -734,6 +744,8 @@ __global__ void __launch_bounds__(kRingFftThreads) k_ring_fft_analysis(const dou
                                                                        int lmax, double2* __restrict__ F) {
   extern __shared__ double2 sm2[];
   const int r = blockIdx.x;
+  map += blockIdx.z * 12LL * nside * nside;
+  F += (long long)blockIdx.z * gridDim.x * (lmax + 1);
   const RingPhi g = ring_phi(r, nside);
   const int n = g.n, h = n / 2;
   const RingFft f = ring_fft_setup(n / 4, sm2);
@@ -759,6 +771,8 @@ __global__ void __launch_bounds__(kRingFftThreads) k_ring_fft_synthesis(const do
                                                                         int lmax, double* __restrict__ map) {
   extern __shared__ double2 sm2[];
   const int r = blockIdx.x;
+  map += blockIdx.z * 12LL * nside * nside;
+  G += (long long)blockIdx.z * gridDim.x * (lmax + 1);
   const RingPhi g = ring_phi(r, nside);
   const int n = g.n, h = n / 2;
   const RingFft f = ring_fft_setup(n / 4, sm2);
@@ -812,7 +826,7 @@ __global__ void __launch_bounds__(kRingFftThreads) k_ring_fft_synthesis(const do
   }
 }
 
-cudaError_t sht_ring_analysis(const double* map, int nside, int lmax, double* F, cudaStream_t s) {
+cudaError_t sht_ring_analysis(const double* map, int nside, int lmax, double* F, cudaStream_t s, int nmaps) {
   const int nrings = 4 * nside - 1;
   double2* out = reinterpret_cast<double2*>(F);
   cudaError_t e;
@@ -820,19 +834,19 @@ cudaError_t sht_ring_analysis(const double* map, int nside, int lmax, double* F,
     const size_t smem = ring_fft_smem(nside);
     e = cudaFuncSetAttribute(k_ring_fft_analysis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_ring_fft_analysis<<<nrings, kRingFftThreads, smem, s>>>(map, nside, lmax, out);
+    k_ring_fft_analysis<<<dim3(nrings, 1, nmaps), kRingFftThreads, smem, s>>>(map, nside, lmax, out);
   } else {
     const size_t smem = sizeof(double) * 4 * (size_t)nside;
     e = cudaFuncSetAttribute(k_ring_analysis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_ring_analysis<<<dim3((lmax + kRingThreads) / kRingThreads, nrings), kRingThreads, smem, s>>>(map, nside, lmax,
-                                                                                                   out);
+    k_ring_analysis<<<dim3((lmax + kRingThreads) / kRingThreads, nrings, nmaps), kRingThreads, smem, s>>>(map, nside,
+                                                                                                          lmax, out);
   }
   note_launch();
   return cudaGetLastError();
 }
 
-cudaError_t sht_ring_synthesis(const double* G, int nside, int lmax, double* map, cudaStream_t s) {
+cudaError_t sht_ring_synthesis(const double* G, int nside, int lmax, double* map, cudaStream_t s, int nmaps) {
   const int nrings = 4 * nside - 1;
   const double2* in = reinterpret_cast<const double2*>(G);
   cudaError_t e;
@@ -840,12 +854,12 @@ cudaError_t sht_ring_synthesis(const double* G, int nside, int lmax, double* map
     const size_t smem = ring_fft_smem(nside);
     e = cudaFuncSetAttribute(k_ring_fft_synthesis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_ring_fft_synthesis<<<nrings, kRingFftThreads, smem, s>>>(in, nside, lmax, map);
+    k_ring_fft_synthesis<<<dim3(nrings, 1, nmaps), kRingFftThreads, smem, s>>>(in, nside, lmax, map);
   } else {
     const size_t smem = sizeof(double2) * (size_t)(lmax + 1);
     e = cudaFuncSetAttribute(k_ring_synthesis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_ring_synthesis<<<dim3((4 * nside + kRingThreads - 1) / kRingThreads, nrings), kRingThreads, smem, s>>>(
+    k_ring_synthesis<<<dim3((4 * nside + kRingThreads - 1) / kRingThreads, nrings, nmaps), kRingThreads, smem, s>>>(
         in, nside, lmax, map);
   }
   note_launch();
@@ -854,30 +868,31 @@ cudaError_t sht_ring_synthesis(const double* G, int nside, int lmax, double* map
 
 template <int RP>
 static cudaError_t analysis_launch(const LegendreShape& sh, const double* F, const double* z, int nrings, int lmax,
-                                   double weight, double* alm, cudaStream_t s) {
+                                   double weight, double* alm, int nmaps, cudaStream_t s) {
   const size_t smem = sizeof(double2) * (size_t)(sh.threads / 32) * kRowTile * 33;
   cudaError_t e = cudaFuncSetAttribute(k_sht_analysis<RP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k_sht_analysis<RP><<<dim3(lmax + 1, sh.blocks), sh.threads, smem, s>>>(
+  k_sht_analysis<RP><<<dim3(lmax + 1, sh.blocks, nmaps), sh.threads, smem, s>>>(
       reinterpret_cast<const double2*>(F), z, nrings, lmax, weight, reinterpret_cast<double2*>(alm));
   note_launch();
   return cudaGetLastError();
 }
 
 cudaError_t sht_analysis(const double* F, const double* z, int nrings, int lmax, double weight, double* alm,
-                         cudaStream_t s) {
-  const LegendreShape sh = legendre_shape(nrings);
+                         cudaStream_t s, int nmaps) {
+  const LegendreShape sh = legendre_shape(nrings, nmaps);
   if (sh.blocks > 1) {  // the blocks of one m add to alm
-    const cudaError_t e = cudaMemsetAsync(alm, 0, sizeof(double2) * (size_t)alm_offset(lmax + 1, lmax), s);
+    const cudaError_t e = cudaMemsetAsync(alm, 0, sizeof(double2) * (size_t)alm_offset(lmax + 1, lmax) * nmaps, s);
     if (e != cudaSuccess) return e;
   }
-  if (sh.rp == 8) return analysis_launch<8>(sh, F, z, nrings, lmax, weight, alm, s);
-  return analysis_launch<2>(sh, F, z, nrings, lmax, weight, alm, s);
+  if (sh.rp == 8) return analysis_launch<8>(sh, F, z, nrings, lmax, weight, alm, nmaps, s);
+  return analysis_launch<2>(sh, F, z, nrings, lmax, weight, alm, nmaps, s);
 }
 
-cudaError_t sht_synthesis(const double* alm, const double* z, int nrings, int lmax, double* G, cudaStream_t s) {
-  const LegendreShape sh = legendre_shape(nrings);
-  const dim3 grid(lmax + 1, sh.blocks);
+cudaError_t sht_synthesis(const double* alm, const double* z, int nrings, int lmax, double* G, cudaStream_t s,
+                          int nmaps) {
+  const LegendreShape sh = legendre_shape(nrings, nmaps);
+  const dim3 grid(lmax + 1, sh.blocks, nmaps);
   const double2* a = reinterpret_cast<const double2*>(alm);
   double2* out = reinterpret_cast<double2*>(G);
   if (sh.rp == 8)

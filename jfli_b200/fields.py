@@ -533,7 +533,7 @@ class SphericalDensity(AbstractField):
         """C_ell of each map, auto or cross with mesh2 (reference fields/lightcone.py:632-674):
         healpy's anafast algorithm in this library's GPU engine (ring transforms and
         Legendre stages in FP64)."""
-        from .power import angular_cl_spherical
+        from .power import angular_cl_spherical, angular_cls_spherical
 
         d1 = self.array
         d2 = mesh2.array if mesh2 is not None else None
@@ -541,13 +541,7 @@ class SphericalDensity(AbstractField):
             raise ValueError("SphericalDensity.angular_cl expects array shape (npix) or (B,npix)")
         if d2 is not None and d2.shape != d1.shape:
             raise ValueError("mesh2 must match shape for cross Cl")
-        rows1 = [d1] if d1.ndim == 1 else list(d1)
-        rows2 = [None] * len(rows1) if d2 is None else ([d2] if d2.ndim == 1 else list(d2))
-        ell, spectra = None, []
-        for a, b in zip(rows1, rows2):
-            ell, cl = angular_cl_spherical(a, b, lmax=lmax, method=method)
-            spectra.append(cl)
-        arr = torch.stack(spectra) if d1.ndim == 2 else spectra[0]
+        ell, arr = (angular_cl_spherical if d1.ndim == 1 else angular_cls_spherical)(d1, d2, lmax=lmax, method=method)
         return PowerSpectrum(wavenumber=ell, array=arr, name="cl", scale_factors=self.scale_factors)
 
     def ud_sample(self, new_nside: int) -> "SphericalDensity":

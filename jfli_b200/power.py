@@ -223,6 +223,19 @@ def angular_cl_spherical(map_sphere, map_sphere2=None, *, lmax: int | None = Non
     return torch.arange(lmax + 1, dtype=torch.float64, device=cl.device), cl
 
 
+def angular_cls_spherical(maps, maps2=None, *, lmax: int | None = None, method: str = "jax"):
+    """angular_cl_spherical of each row of (B, npix) maps, whose transforms run together."""
+    from . import sht
+
+    if method not in ("jax", "healpy"):
+        raise ValueError(f"unknown method {method!r}")
+    lmax = 3 * sht._nside_of(int(maps.shape[-1])) - 1 if lmax is None else int(lmax)
+    a1 = sht.maps2alm(maps, lmax)
+    a2 = [None] * len(a1) if maps2 is None else sht.maps2alm(maps2, lmax)
+    cls = torch.stack([sht.alm2cl(a, lmax, b) for a, b in zip(a1, a2)])
+    return torch.arange(lmax + 1, dtype=torch.float64, device=cls.device), cls
+
+
 def cross_angular_cl_spherical(maps, *, lmax: int | None = None, method: str = "healpy"):
     """All cross C_l of B maps in healpy's order (reference power/compute.py:101-109)."""
     from . import sht

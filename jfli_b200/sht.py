@@ -59,8 +59,8 @@ def packed_offsets(lmax: int) -> np.ndarray:
 
 
 class _GpuSht:
-    """Device tables of one (nside, lmax) and the four device stages: ring transforms along
-    phi and the Legendre stages. Maps and a_lm stay on the device."""
+    """Device tables of one (nside, lmax) and the device stages, ring transforms along phi and
+    Legendre, of one map or of several at once. Maps and a_lm stay on the device."""
 
     def __init__(self, nside: int, lmax: int, device=None):
         self.nside, self.lmax = nside, lmax
@@ -69,27 +69,37 @@ class _GpuSht:
         self.nrings = z.size
         self.z = torch.as_tensor(z, dtype=torch.float64, device=self.device)
         self.nalm = (lmax + 1) * (lmax + 2) // 2
-        self.F = torch.empty(self.nrings, lmax + 1, dtype=torch.complex128, device=self.device)
+
+    def _scratch(self, lead) -> torch.Tensor:
+        return torch.empty(*lead, self.nrings, self.lmax + 1, dtype=torch.complex128, device=self.device)
 
     def map2alm_once(self, m: torch.Tensor) -> torch.Tensor:
-        """Packed a_lm (device, complex128) of a device FP64 map."""
+        """Packed a_lm (..., nalm) (device, complex128) of device FP64 maps (..., npix)."""
         from ._lib import call, stream_ptr
 
-        call("jfli_sht_ring_analysis", stream_ptr(), m.data_ptr(), self.nside, self.lmax, self.F.data_ptr())
-        alm = torch.empty(self.nalm, dtype=torch.complex128, device=self.device)
-        call("jfli_sht_map2alm", stream_ptr(), self.F.data_ptr(), self.z.data_ptr(), self.nrings, self.lmax,
-             4.0 * math.pi / m.numel(), alm.data_ptr())
+        lead = m.shape[:-1]
+        F = self._scratch(lead)
+        alm = torch.empty(*lead, self.nalm, dtype=torch.complex128, device=self.device)
+        call("jfli_sht_maps2alm", stream_ptr(), m.data_ptr(), self.z.data_ptr(), self.nside, self.lmax,
+             math.prod(lead), F.data_ptr(), alm.data_ptr())
         return alm
 
     def alm2map(self, alm: torch.Tensor) -> torch.Tensor:
-        """Device FP64 map of packed device a_lm."""
+        """Device FP64 maps (..., npix) of packed device a_lm (..., nalm)."""
         from ._lib import call, stream_ptr
 
-        call("jfli_sht_alm2map", stream_ptr(), alm.data_ptr(), self.z.data_ptr(), self.nrings, self.lmax,
-             self.F.data_ptr())
-        out = torch.empty(12 * self.nside * self.nside, dtype=torch.float64, device=self.device)
-        call("jfli_sht_ring_synthesis", stream_ptr(), self.F.data_ptr(), self.nside, self.lmax, out.data_ptr())
+        lead = alm.shape[:-1]
+        G = self._scratch(lead)
+        out = torch.empty(*lead, 12 * self.nside * self.nside, dtype=torch.float64, device=self.device)
+        call("jfli_sht_alm2maps", stream_ptr(), alm.data_ptr(), self.z.data_ptr(), self.nside, self.lmax,
+             math.prod(lead), G.data_ptr(), out.data_ptr())
         return out
+
+    def map2alm(self, m: torch.Tensor, iter: int) -> torch.Tensor:
+        alm = self.map2alm_once(m)
+        for _ in range(iter):
+            alm = alm + self.map2alm_once(m - self.alm2map(alm))
+        return alm
 
 
 _ENGINES: dict = {}
@@ -127,11 +137,27 @@ def map2alm(m, lmax: int | None = None, iter: int = 3) -> torch.Tensor:
     md = _device_map(m).reshape(-1)
     nside = _nside_of(md.numel())
     lmax = 3 * nside - 1 if lmax is None else int(lmax)
-    eng = _engine(nside, lmax, md.device)
-    alm = eng.map2alm_once(md)
-    for _ in range(iter):
-        alm = alm + eng.map2alm_once(md - eng.alm2map(alm))
-    return alm
+    return _engine(nside, lmax, md.device).map2alm(md, iter)
+
+
+# Scratch of the maps that go through the stages together. The CTAs of a small map end on the
+# serial chain of their first m: four maps took 0.88 ms one after the other and take 0.28
+# together at nside 64, 1.23 and 0.69 at nside 128, 3.76 and 3.08 at nside 256 (13 MB of ring
+# coefficients each). One of nside 1024 (201 MB) fills the GPU alone.
+_BATCH_BYTES = 1 << 28
+
+
+def maps2alm(maps, lmax: int | None = None, iter: int = 3):
+    """map2alm of each of B maps (B, npix), as many at a time as _BATCH_BYTES allow: a list of B
+    packed a_lm."""
+    nside = _nside_of(int(maps.shape[-1]))
+    lmax = 3 * nside - 1 if lmax is None else int(lmax)
+    step = max(1, _BATCH_BYTES // (16 * (4 * nside - 1) * (lmax + 1)))
+    alms = []
+    for first in range(0, len(maps), step):
+        md = _device_map(maps[first:first + step])
+        alms += list(_engine(nside, lmax, md.device).map2alm(md, iter))
+    return alms
 
 
 def alm2cl(alm1: torch.Tensor, lmax: int, alm2: torch.Tensor | None = None) -> torch.Tensor:
@@ -159,6 +185,6 @@ def cross_cls(maps, lmax: int | None = None, iter: int = 3) -> torch.Tensor:
     md = _device_map(maps)
     md = md.reshape(-1, md.shape[-1])
     lmax = 3 * _nside_of(md.shape[1]) - 1 if lmax is None else int(lmax)
-    alms = [map2alm(row, lmax, iter) for row in md]
+    alms = maps2alm(md, lmax, iter)
     b = len(alms)
     return torch.stack([alm2cl(alms[i], lmax, alms[i + d]) for d in range(b) for i in range(b - d)])
