@@ -294,7 +294,7 @@ __global__ void k_div_fd(const float* __restrict__ u, float alpha, const float* 
   grid_release();
   grid_wait();
   const long long b = blockIdx.y;
-  u += b * g.np * 3;
+  u += b * g.np * (cell_stride == 4 ? 4 : 3);
   if (w) w += b * g.np * 3;
   out += b * g.np;
   const float s = 1.0f / 12.0f;
