@@ -85,6 +85,89 @@ __device__ __forceinline__ void deposit_vec4_lane_merged(float4* mesh, const PGr
     }
 }
 
+// The upper-x corners of a lane's previous particle in the column walk, held back in registers:
+// when the lane's next particle, one Lagrangian plane further in x, has its lower-x corners in
+// the same four cells, both go out in one atomic per cell.
+struct VecCarry {
+  int xo, yo0, yo1, z0, z1;  // cell offsets of the 2 (y) x 2 (z) corners: x ny nz, y nz, z
+  float w[4];                // weights [y][z]
+  float u[3];
+  bool valid;
+};
+
+// Deposit, for every lane of a full warp, the vectors v of the 2 (y) x 2 (z) corners of one x
+// plane, with the z merge of deposit_vec4_lane_merged. Lanes with `on` false deposit nothing.
+__device__ __forceinline__ void deposit_vec4_plane(float4* mesh, bool on, int xo, int yo0, int yo1, int z0, int z1,
+                                                   const float v[4][3]) {
+  const int lane = threadIdx.x & 31;
+  const int lo = on ? xo + yo0 + z0 : -1;
+  const int hi = on ? xo + yo0 + z1 : -2;
+  const int next_lo = __shfl_down_sync(0xffffffffu, lo, 1);
+  const int prev_hi = __shfl_up_sync(0xffffffffu, hi, 1);
+  const bool give = on && lane < 31 && next_lo == hi;
+  const bool take = on && lane > 0 && prev_hi == lo;
+#pragma unroll
+  for (int b = 0; b < 2; ++b) {
+    float low[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const float recv = __shfl_up_sync(0xffffffffu, v[2 * b + 1][a], 1);
+      low[a] = take ? v[2 * b][a] + recv : v[2 * b][a];
+    }
+    const int row = xo + (b ? yo1 : yo0);
+    if (on) {
+      atomicAdd(mesh + (row + z0), make_float4(low[0], low[1], low[2], 0.f));
+      if (!give)
+        atomicAdd(mesh + (row + z1), make_float4(v[2 * b + 1][0], v[2 * b + 1][1], v[2 * b + 1][2], 0.f));
+    }
+  }
+}
+
+__device__ __forceinline__ void vec_carry_deposit(float4* mesh, VecCarry& c) {
+  float v[4][3];
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+#pragma unroll
+    for (int a = 0; a < 3; ++a) v[q][a] = c.w[q] * c.u[a];
+  deposit_vec4_plane(mesh, c.valid, c.xo, c.yo0, c.yo1, c.z0, c.z1, v);
+  c.valid = false;
+}
+
+// CIC deposit of u in the column walk (full warps, lanes on consecutive z particles of one row,
+// successive calls of a lane on successive x planes): the lower-x plane now, with the carry
+// when its cells are the same (otherwise the carry goes out alone), the upper-x plane later.
+__device__ __forceinline__ void deposit_vec4_carried(float4* mesh, const PGrid& g, const Cic1& cx, const Cic1& cy,
+                                                     const Cic1& cz, const float u[3], VecCarry& c) {
+  const int xo0 = cx.i0 * g.yz, yo0 = cy.i0 * g.nz, yo1 = cy.i1 * g.nz;
+  const float wyz[4] = {cy.w0 * cz.w0, cy.w0 * cz.w1, cy.w1 * cz.w0, cy.w1 * cz.w1};
+  const bool same = c.valid && c.xo == xo0 && c.yo0 == yo0 && c.z0 == cz.i0;
+  if (c.valid && !same) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      atomicAdd(mesh + (c.xo + (q & 2 ? c.yo1 : c.yo0) + (q & 1 ? c.z1 : c.z0)),
+                make_float4(c.w[q] * c.u[0], c.w[q] * c.u[1], c.w[q] * c.u[2], 0.f));
+  }
+  float v[4][3];
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      v[q][a] = cx.w0 * wyz[q] * u[a];
+      if (same) v[q][a] += c.w[q] * c.u[a];
+    }
+  deposit_vec4_plane(mesh, true, xo0, yo0, yo1, cz.i0, cz.i1, v);
+  c.xo = cx.i1 * g.yz;
+  c.yo0 = yo0;
+  c.yo1 = yo1;
+  c.z0 = cz.i0;
+  c.z1 = cz.i1;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) c.w[q] = cx.w1 * wyz[q];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) c.u[a] = u[a];
+  c.valid = true;
+}
+
 // Reverse kick + first half of the VJP of one reversible step, at the un-drifted
 // positions x (relative displacements). Per particle:
 //   F = R_x[force];  <lambda_x, v'> -> partial[1];  u = lambda_v + drift * lambda_x;
@@ -97,7 +180,7 @@ template <bool kVec4>
 __device__ __forceinline__ void unkick_core(float x[3], float v[3], const float lx[3], float lv[3], bool undrift,
                                             const float* __restrict__ force, float kick, float drift,
                                             float* __restrict__ ubar, const PGrid& g, int i, int j, int k, double& sk,
-                                            double& sd) {
+                                            double& sd, VecCarry* carry = nullptr) {
   if (undrift) {
 #pragma unroll
     for (int a = 0; a < 3; ++a) x[a] += v[a] * -drift;
@@ -114,7 +197,9 @@ __device__ __forceinline__ void unkick_core(float x[3], float v[3], const float 
     v[a] = v[a] - f[a] * kick;
     lv[a] = u[a];
   }
-  if (kVec4) {
+  if (kVec4 && carry) {
+    deposit_vec4_carried(reinterpret_cast<float4*>(ubar), g, cx, cy, cz, u, *carry);
+  } else if (kVec4) {
     deposit_vec4_lane_merged(reinterpret_cast<float4*>(ubar), g, cx, cy, cz, u);
   } else {
 #pragma unroll
@@ -158,16 +243,24 @@ __device__ __forceinline__ void unkick_row(float* __restrict__ disp, bool undrif
                                            const float* __restrict__ lam_x, float* __restrict__ lam_v,
                                            const float* __restrict__ force, float kick, float drift,
                                            float* __restrict__ ubar, const PGrid& g, unsigned p0, int i, int j, int k,
-                                           int lane, float4 (*buf)[24], double& sk, double& sd) {
+                                           int lane, float4 (*buf)[24], double& sk, double& sd, float4 row[4],
+                                           bool more, VecCarry& carry) {
   float4* d4 = reinterpret_cast<float4*>(disp + 3ull * p0);
   float4* v4 = reinterpret_cast<float4*>(vel + 3ull * p0);
   const float4* x4 = reinterpret_cast<const float4*>(lam_x + 3ull * p0);
   float4* l4 = reinterpret_cast<float4*>(lam_v + 3ull * p0);
   if (lane < 24) {
-    buf[0][lane] = __ldcs(d4 + lane);
-    buf[1][lane] = __ldcs(v4 + lane);
-    buf[2][lane] = __ldcs(x4 + lane);
-    buf[3][lane] = __ldcs(l4 + lane);
+    buf[0][lane] = row[0];
+    buf[1][lane] = row[1];
+    buf[2][lane] = row[2];
+    buf[3][lane] = row[3];
+    if (more) {  // the row of the next plane, on its way while this one is worked on
+      const unsigned q = 3u * (unsigned)g.yz / 4u + (unsigned)lane;
+      row[0] = __ldcs(d4 + q);
+      row[1] = __ldcs(v4 + q);
+      row[2] = __ldcs(x4 + q);
+      row[3] = __ldcs(l4 + q);
+    }
   }
   __syncwarp();
   float x[3], v[3], lx[3], lv[3];
@@ -183,7 +276,7 @@ __device__ __forceinline__ void unkick_row(float* __restrict__ disp, bool undrif
     lv[a] = f3[3 * lane + a];
   }
   __syncwarp();
-  unkick_core<kVec4>(x, v, lx, lv, undrift, force, kick, drift, ubar, g, i, j, k, sk, sd);
+  unkick_core<kVec4>(x, v, lx, lv, undrift, force, kick, drift, ubar, g, i, j, k, sk, sd, &carry);
   float* w0 = reinterpret_cast<float*>(buf[0]);
   float* w1 = reinterpret_cast<float*>(buf[1]);
   float* w3 = reinterpret_cast<float*>(buf[3]);
@@ -203,17 +296,61 @@ __device__ __forceinline__ void unkick_row(float* __restrict__ disp, bool undrif
 }
 
 constexpr int kAdjBrickY = 8, kAdjBrickZ = 32;
+constexpr int kUnkickCtas = 2;  // resident per SM (128 registers)
+
+// How walk_columns cuts the columns. Up to 2^22 cells the meshes that are gathered from and painted
+// are in L2, and equal ranges of planes, one per resident CTA, leave no last round (0). Larger
+// meshes are taken in slabs of 8 planes, so that columns that share lines meet in L2. Un-kick,
+// ranges against slabs: 64^3 12.3 and 19.5 us, 128^3 67 and 73, 192^3 290 and 249, 256^3 717 and
+// 611, 384^3 2450 and 2146. (The forward pass gains nothing from ranges: 64^3 10.0 us against
+// 9.7 with bricks, 128^3 46.6 and 46.6.)
+inline int walk_depth(const MeshDims& d) { return d.cells() * d.batch <= (1ll << 22) ? 0 : 8; }
+
+// The columns of 8 (y) x 32 (z) cells of a mesh (ny a multiple of 8, nz of 32), in pieces for each
+// CTA: run(first y, first z, first x, last x + 1). depth 0: the planes of all columns, one column
+// after the other, cut into one range per CTA, equal to a plane; otherwise pieces of `depth`
+// planes, all columns of a slab before the next slab (walk_depth).
+template <class Run>
+__device__ __forceinline__ void walk_columns(const PGrid& g, int depth, Run run) {
+  const unsigned nx = (unsigned)g.nx, tz = (unsigned)g.nz / kAdjBrickZ, columns = tz * ((unsigned)g.ny / kAdjBrickY);
+  unsigned t = blockIdx.x, last = depth ? columns * ((nx + depth - 1) / depth) : 0;
+  if (!depth) {
+    const unsigned long long planes = (unsigned long long)columns * nx;
+    t = (unsigned)(planes * blockIdx.x / gridDim.x);
+    last = (unsigned)(planes * (blockIdx.x + 1) / gridDim.x);
+  }
+  while (t < last) {
+    unsigned col, i0, i1;
+    if (depth) {
+      col = t % columns;
+      i0 = t / columns * depth;
+      i1 = min(nx, i0 + depth);
+      t += gridDim.x;
+    } else {
+      col = t / nx;
+      i0 = t - col * nx;
+      i1 = min(nx, i0 + (last - t));
+      t += i1 - i0;
+    }
+    run((int)(col / tz) * kAdjBrickY, (int)(col % tz) * kAdjBrickZ, (int)i0, (int)i1);
+  }
+}
+
 
 // Work order of the float4 form: when nz is a multiple of 32 and ny of 8, a CTA of 8 warps
-// takes an 8 (y) x 32 (z) brick of Lagrangian cells and walks it along x in chunks of
-// xdepth planes (brick_xdepth), each warp on one z row (the z merge of the deposit needs consecutive z in a
-// warp), so that the rows and planes whose particles share CIC corners gather and deposit
-// on one SM close in time (as the forward particle pass). Otherwise a grid-stride walk.
+// walks 8 (y) x 32 (z) columns of Lagrangian cells along x, each warp on one z row (the z merge
+// of the deposit needs consecutive z in a warp), so that the rows and planes whose particles
+// share CIC corners gather and deposit on one SM close in time (as the forward particle
+// pass). Otherwise a grid-stride walk.
+//
+// Bound by L1 (gathers and atomics of 16 bytes a lane). 128^3: 88 us with pieces of 8 planes over
+// 1184 CTAs (2.3 rounds of the resident ones), 78 with equal ranges, 76.7 with the next row's
+// loads ahead of this one (128 registers, two CTAs per SM), 67 with the x merge of VecCarry.
 template <bool kVec4>
-__global__ void __launch_bounds__(kAdjThreads, 3) k_adj_unkick_paint(
+__global__ void __launch_bounds__(kAdjThreads, kUnkickCtas) k_adj_unkick_paint(
     float* __restrict__ disp, int undrift, float* __restrict__ vel, const float* __restrict__ lam_x,
     float* __restrict__ lam_v, const float* __restrict__ force, float kick, float drift, float* __restrict__ ubar,
-    double* __restrict__ partials, PGrid g, int xdepth) {
+    double* __restrict__ partials, PGrid g, int depth) {
   const long long b = blockIdx.y;
   disp += b * g.np * 3;
   vel += b * g.np * 3;
@@ -227,24 +364,30 @@ __global__ void __launch_bounds__(kAdjThreads, 3) k_adj_unkick_paint(
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const bool staged = ((reinterpret_cast<uintptr_t>(disp) | reinterpret_cast<uintptr_t>(vel) |
                           reinterpret_cast<uintptr_t>(lam_x) | reinterpret_cast<uintptr_t>(lam_v)) & 15) == 0;
-    const int tz = g.nz / kAdjBrickZ, ty = g.ny / kAdjBrickY, txc = (g.nx + xdepth - 1) / xdepth;
-    const long long items = (long long)tz * ty * txc;
-    for (long long it = blockIdx.x; it < items; it += gridDim.x) {
-      const int iz = (int)(it % tz);
-      const long long rest = it / tz;
-      const int iy = (int)(rest % ty), xc = (int)(rest / ty);
-      const int j = iy * kAdjBrickY + w, k = iz * kAdjBrickZ + lane;
-      const int i1 = min(g.nx, (xc + 1) * xdepth);
-      for (int i = xc * xdepth; i < i1; ++i) {
+    walk_columns(g, depth, [&](int jc, int kc, int i0, int i1) {
+      const int j = jc + w, k = kc + lane;
+      VecCarry carry;
+      carry.valid = false;
+      float4 row[4];
+      if (staged && lane < 24) {
+        const unsigned p0 = ((unsigned)i0 * (unsigned)g.ny + (unsigned)j) * (unsigned)g.nz + (unsigned)(k - lane);
+        row[0] = __ldcs(reinterpret_cast<const float4*>(disp + 3ull * p0) + lane);
+        row[1] = __ldcs(reinterpret_cast<const float4*>(vel + 3ull * p0) + lane);
+        row[2] = __ldcs(reinterpret_cast<const float4*>(lam_x + 3ull * p0) + lane);
+        row[3] = __ldcs(reinterpret_cast<const float4*>(lam_v + 3ull * p0) + lane);
+      }
+      for (int i = i0; i < i1; ++i) {
         const unsigned p = ((unsigned)i * (unsigned)g.ny + (unsigned)j) * (unsigned)g.nz + (unsigned)k;
         if (staged)
           unkick_row<kVec4>(disp, undrift != 0, vel, lam_x, lam_v, force, kick, drift, ubar, g, p - (unsigned)lane,
-                            i, j, k, lane, rowbuf[kVec4 ? w : 0], sk, sd);
+                            i, j, k, lane, rowbuf[kVec4 ? w : 0], sk, sd, row, i + 1 < i1,
+                            carry);
         else
           unkick_particle<kVec4>(disp, undrift != 0, vel, lam_x, lam_v, force, kick, drift, ubar, g, p, i, j, k, sk,
                                  sd);
       }
-    }
+      if (staged) vec_carry_deposit(reinterpret_cast<float4*>(ubar), carry);
+    });
   } else {
     for (unsigned p = blockIdx.x * blockDim.x + threadIdx.x; p < g.np; p += gridDim.x * blockDim.x) {
       int i, j, k;
@@ -321,6 +464,65 @@ __global__ void k_div_fd(const float* __restrict__ u, float alpha, const float* 
     }
     out[p] = accumulate ? out[p] + acc : acc;
   }
+}
+
+// The same of a float4 mesh (x, y, z, 0) with ny a multiple of 8 and nz of 32: CTAs of 8 x 32 threads
+// walk columns along x. A thread loads its cell's 16 bytes once, three planes ahead, and keeps
+// the x components of five planes in registers; the y and z components of a plane go through
+// shared memory with two cells more on either side. The stencil form above loads 12 words, each
+// 16 bytes from the next lane's, and is bound by L1. Stencil and this form: 64^3 4.4 and 5.3 us
+// (few planes per CTA, each a round trip to L2), 96^3 10.0 and 8.4, 128^3 20.4 and 14.7, 192^3 62
+// and 47, 256^3 164 and 100.
+constexpr int kDivCtas = 5;  // resident per SM
+
+__global__ void __launch_bounds__(kAdjThreads, kDivCtas) k_div_march(const float4* __restrict__ u, float alpha,
+                                                                     int accumulate, float* __restrict__ out, PGrid g,
+                                                                     int depth) {
+  grid_release();
+  grid_wait();
+  __shared__ float ys[2][kAdjBrickY + 4][kAdjBrickZ];
+  __shared__ float zs[2][kAdjBrickY][kAdjBrickZ + 4];
+  const long long b = blockIdx.y;
+  u += b * g.np;
+  out += b * g.np;
+  const float s = 1.0f / 12.0f;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  // threads 0..127 fetch the y halo (rows -2, -1, 8, 9), 128..159 the z halo (cells -2, -1, 32, 33)
+  const bool hy = w < 4, hz = w == 4;
+  const int hrow = w < 2 ? w : w + kAdjBrickY;  // row of ys
+  const int zrow = lane >> 2, zcol = (lane & 3) < 2 ? (lane & 3) : (lane & 3) + kAdjBrickZ;
+  walk_columns(g, depth, [&](int jc, int kc, int i0, int i1) {
+    const int j = jc + w, k = kc + lane;
+    const float4* cell = u + (j * g.nz + k);
+    const float* halo = nullptr;
+    if (hy) halo = &u[wrap1(jc + hrow - 2, g.ny) * g.nz + k].y;
+    if (hz) halo = &u[(jc + zrow) * g.nz + wrap1(kc + zcol - 2, g.nz)].z;
+    auto plane = [&](int i) { return (long long)wrap1(i, g.nx) * g.yz; };
+    float xm2 = alpha * cell[plane(i0 - 2)].x, xm1 = alpha * cell[plane(i0 - 1)].x;
+    float4 c0 = cell[plane(i0)], c1 = cell[plane(i0 + 1)], c2 = cell[plane(i0 + 2)];
+    float h = halo ? halo[4 * plane(i0)] : 0.f;
+    int buf = 0;
+    for (int i = i0; i < i1; ++i, buf ^= 1) {
+      const float4 next = i + 1 < i1 ? cell[plane(i + 3)] : c2;
+      ys[buf][w + 2][lane] = alpha * c0.y;
+      zs[buf][w][lane + 2] = alpha * c0.z;
+      if (hy) ys[buf][hrow][lane] = alpha * h;
+      if (hz) zs[buf][zrow][zcol] = alpha * h;
+      if (halo && i + 1 < i1) h = halo[4 * plane(i + 1)];
+      __syncthreads();  // the other buffer is written only after this plane's barrier
+      float acc = (8.0f * (alpha * c1.x - xm1) - (alpha * c2.x - xm2)) * s;
+      acc += (8.0f * (ys[buf][w + 3][lane] - ys[buf][w + 1][lane]) - (ys[buf][w + 4][lane] - ys[buf][w][lane])) * s;
+      acc += (8.0f * (zs[buf][w][lane + 3] - zs[buf][w][lane + 1]) - (zs[buf][w][lane + 4] - zs[buf][w][lane])) * s;
+      float* dst = out + (plane(i) + j * g.nz + k);
+      *dst = accumulate ? *dst + acc : acc;
+      xm2 = xm1;
+      xm1 = alpha * c0.x;
+      c0 = c1;
+      c1 = c2;
+      c2 = next;
+    }
+    __syncthreads();  // before the next piece writes a buffer that may still be read
+  });
 }
 
 // lam_x += scale * grad_x R_x[h], h(corner) = rho_bar(corner) + sum_a u_a force_a(corner)
@@ -410,6 +612,15 @@ __global__ void __launch_bounds__(256) k_adj_position(const float* __restrict__ 
 // ----------------------------------------------------------------------------------
 static dim3 adj_grid(const MeshDims& d) { return particle_grid_dims(d.cells(), d.batch, kAdjThreads, kAdjCtasPerSm); }
 
+// The grid of the float4 un-kick, whose partials sum_adjoint_partials adds up: its resident CTAs.
+// No larger than adj_grid, the grid of the other form, all of whose partials the caller sums.
+static dim3 unkick_grid(const MeshDims& d) {
+  const long long resident = max(1ll, (long long)kUnkickCtas * sm_count() / d.batch);
+  dim3 grid = adj_grid(d);
+  if (resident < grid.x) grid.x = (unsigned)resident;
+  return grid;
+}
+
 size_t adjoint_partials_count(const MeshDims& d) { return (size_t)2 * adj_grid(d).x * d.batch; }
 
 // out[b][2] = sums of the per-CTA partials of batch entry b: each thread adds a strided
@@ -442,8 +653,8 @@ __global__ void __launch_bounds__(256) k_sum_partials(const double* __restrict__
 }
 
 cudaError_t sum_adjoint_partials(const double* partials, const MeshDims& d, double* out, cudaStream_t s) {
-  launch_next(overlap_starts(d.cells() * d.batch), k_sum_partials, d.batch, 256, 0, s, partials, (int)adj_grid(d).x,
-              out);
+  launch_next(overlap_starts(d.cells() * d.batch), k_sum_partials, d.batch, 256, 0, s, partials,
+              (int)unkick_grid(d).x, out);
   note_launch();
   return cudaGetLastError();
 }
@@ -457,12 +668,11 @@ cudaError_t adjoint_unkick_paint(const float* disp, float* vel, const float* lam
   cudaError_t e = cudaMemsetAsync(ubar, 0, sizeof(float) * (vec4 ? 4 : 3) * (size_t)d.cells() * d.batch, s);
   if (e != cudaSuccess) return e;
   if (vec4)
-    k_adj_unkick_paint<true><<<adj_grid(d), kAdjThreads, 0, s>>>(dp, undrift, vel, lam_x, lam_v, force, kick, drift, ubar,
-                                                                 partials, make_pgrid(d),
-                                                                 brick_xdepth(d.nx, d.ny, d.nz, d.batch, 4ll * sm_count()));
+    k_adj_unkick_paint<true><<<unkick_grid(d), kAdjThreads, 0, s>>>(dp, undrift, vel, lam_x, lam_v, force, kick, drift,
+                                                                    ubar, partials, make_pgrid(d), walk_depth(d));
   else
     k_adj_unkick_paint<false><<<adj_grid(d), kAdjThreads, 0, s>>>(dp, undrift, vel, lam_x, lam_v, force, kick, drift, ubar,
-                                                                  partials, make_pgrid(d), 16);
+                                                                  partials, make_pgrid(d), 0);
   note_launch();
   return cudaGetLastError();
 }
@@ -472,6 +682,16 @@ cudaError_t divergence_fd(const float* u, float alpha, const float* w, float bet
   // aos 0: three meshes; 1: particle grids (3 floats per cell); 2: float4 meshes
   const long long cell_stride = aos == 2 ? 4 : (aos ? 3 : 1);
   const long long comp_stride = aos ? 1 : d.cells();
+  if (aos == 2 && w == nullptr && d.ny % kAdjBrickY == 0 && d.nz % kAdjBrickZ == 0 &&
+      d.cells() * d.batch >= (1ll << 19)) {
+    const long long planes = d.cells() / (kAdjBrickY * kAdjBrickZ);
+    const long long resident = max(1ll, (long long)kDivCtas * sm_count() / d.batch);
+    launch_next(overlap_starts(d.cells() * d.batch), k_div_march, dim3((unsigned)min(planes, resident), d.batch),
+                kAdjThreads, 0, s, reinterpret_cast<const float4*>(u), alpha, accumulate, out, make_pgrid(d),
+                walk_depth(d));
+    note_launch();
+    return cudaGetLastError();
+  }
   launch_next(overlap_starts(d.cells() * d.batch), k_div_fd, particle_grid_dims(d.cells(), d.batch, 256, 16), 256, 0, s,
               u, alpha, w, beta, cell_stride, comp_stride, accumulate, out, make_pgrid(d));
   note_launch();
