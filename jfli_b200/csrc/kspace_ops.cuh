@@ -126,26 +126,75 @@ struct IcOp {
   // of the table, interp(dptab) * factor / (2 sqrt(P)) (0 where P <= 0 and at the
   // k = 0 guard), used for gradients with respect to the cosmology behind P(k).
   const float* dptab = nullptr;
-  static size_t smem_bytes(const IcOp& op) { return sizeof(float) * (op.nx + 3 * op.ntab); }
+  // Shared memory: kx [nx], the tables k, P [ntab], the segments' slopes or in tangent mode dP
+  // [ntab], the buckets' starts, and the buckets' shift and base.
+  //
+  // A search from the ends of the table per mode (seven dependent reads for 128 points) and the
+  // division of its slope took longer than the transform. The slopes are made once per CTA, and
+  // k's bits above `shift` (eighths of an octave or coarser, so that the table's span fits) give
+  // a bucket whose first and last index are tabulated: a logarithmic table has about one point
+  // to a bucket. The index, and so the result, is the same. 384^3: 380 -> 287 us (Poisson 171).
+  static constexpr int kBuckets = 256;
+  static size_t smem_bytes(const IcOp& op) {
+    return sizeof(float) * (op.nx + 3 * op.ntab) + sizeof(unsigned short) * (kBuckets + 2) + 2 * sizeof(int);
+  }
   __device__ void prologue(float* sm, int) const {
     for (int i = threadIdx.x; i < nx; i += blockDim.x) {
       sm[i] = k_rad_per_cell(i, nx) / lx * (float)nx;
     }
+    float* xp = sm + nx;
+    float* fp = xp + ntab;
     for (int i = threadIdx.x; i < ntab; i += blockDim.x) {
-      sm[nx + i] = ktab[i];
-      sm[nx + ntab + i] = ptab[i];
-      if (dptab) sm[nx + 2 * ntab + i] = dptab[i];
+      xp[i] = ktab[i];
+      fp[i] = ptab[i];
+      if (dptab) fp[ntab + i] = dptab[i];
     }
     __syncthreads();
+    if (!dptab)
+      for (int i = threadIdx.x; i + 1 < ntab; i += blockDim.x)
+        fp[ntab + i] = (fp[i + 1] - fp[i]) / (xp[i + 1] - xp[i]);
+    unsigned short* start = reinterpret_cast<unsigned short*>(fp + 2 * ntab);
+    // bucket 1 starts from the second k of the table: the first may be 0
+    const int first = __float_as_int(fmaxf(xp[1], 0.f)), span = __float_as_int(fmaxf(xp[ntab - 1], 0.f)) - first;
+    int shift = 20;
+    while ((span >> shift) > kBuckets - 4) ++shift;
+    const int base = first >> shift;
+    if (threadIdx.x == 0) {
+      int* at = reinterpret_cast<int*>(start + kBuckets + 2);
+      at[0] = shift;
+      at[1] = base - 1;
+    }
+    for (int b = threadIdx.x; b <= kBuckets; b += blockDim.x)
+      start[b] = (unsigned short)(b == 0          ? 0
+                                  : b == kBuckets ? ntab
+                                                  : search(__int_as_float((base + b - 1) << shift), xp, 0, ntab));
+    __syncthreads();
+  }
+  // first index in [lo, hi) with xp[i] >= x, or hi
+  static __device__ __forceinline__ int search(float x, const float* xp, int lo, int hi) {
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (xp[mid] < x)
+        lo = mid + 1;
+      else
+        hi = mid;
+    }
+    return lo;
   }
   __device__ float2 apply(float2 v, int kx, int ky, int kz, float* sm, int) const {
     const float ax = sm[kx];
     const float ay = k_rad_per_cell(ky, ny) / ly * (float)ny;
     const float az = k_rad_per_cell(kz, nz) / lz * (float)nz;
     const float kmag = sqrtf(ax * ax + ay * ay + az * az);
-    float pk = interp_table(kmag, sm + nx, sm + nx + ntab, ntab) * factor;
+    const float *xp = sm + nx, *fp = xp + ntab;
+    const unsigned short* start = reinterpret_cast<const unsigned short*>(fp + 2 * ntab);
+    const int* at = reinterpret_cast<const int*>(start + kBuckets + 2);
+    const int b = min(max((__float_as_int(kmag) >> at[0]) - at[1], 0), kBuckets - 1);
+    const int i = min(max(search(kmag, xp, start[b], start[b + 1]) - 1, 0), ntab - 2);
+    const float slope = dptab ? (fp[i + 1] - fp[i]) / (xp[i + 1] - xp[i]) : fp[ntab + i];
+    float pk = (fp[i] + (kmag - xp[i]) * slope) * factor;
     if (dptab) {
-      const float dpk = interp_table(kmag, sm + nx, sm + nx + 2 * ntab, ntab) * factor;
+      const float dpk = interp_table(kmag, xp, fp + ntab, ntab) * factor;
       float m = pk > 0.f ? dpk / (2.0f * sqrtf(pk)) : 0.f;
       if (zero_mode_one && kmag == 0.f) m = 0.f;
       return cscale(v, m * norm);
