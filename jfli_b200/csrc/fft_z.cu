@@ -122,6 +122,34 @@ __global__ void __launch_bounds__(kFftThreads) k_irfft_z(const float2* __restric
   }
 }
 
+// Shared-memory layout of the register row passes, without bank conflicts. A half warp's 16
+// eight-byte accesses are served at once when their indices differ mod 16.
+//   * exchange buffer: stage 1 has t across the lanes, so its t stride YS is odd; stage 2 has kb
+//     and then the row across the lanes, so the row stride is Q mod 16 (kb + Q r = tid).
+//   * transformed rows (r2c): the row stride ZS is Q mod 16 for the same reason.
+//   * stage-1 twiddles w^(t kb) are laid out by (kb, t) from Q = 12 on: read from the plain table
+//     the stride kb costs up to 8 passes (384^3 c2r 93.9 -> 90.7 us; with Q = 8 the fill costs
+//     as much as it saves, 256^3 c2r 26.6 and 27.5).
+// And the r2c output takes the pair (k, N - k) per thread, whose two inputs are the same. r2c
+// with all of it: 256^3 35.2 -> 31.7 us, 384^3 120 -> 106, 512^3 230 -> 205; c2r 384^3 98 -> 91.
+template <int N>
+struct RowSmem {
+  static constexpr int P = Split<N>::P, Q = Split<N>::Q, R = RowCfg<N>::R;
+  static constexpr int mod16(int least) { return least + ((Q - least) % 16 + 16) % 16; }
+  static constexpr int YS = Q | 1;
+  static constexpr int S = mod16(P * YS);
+  static constexpr int ZS = mod16(N + 1);
+  static constexpr bool kStaged = Q >= 12;
+  static constexpr int TWS = kStaged ? (Q - 1) * P : 0;  // w^(t kb), kb = 1 .. Q - 1
+  static constexpr int r2c = N + N + 1 + TWS + R * (S > ZS ? S : ZS);
+  static constexpr int XB = R * (N + 1 > S ? N + 1 : S);
+  static constexpr int c2r = XB + N + N + 1 + TWS;
+};
+
+template <int P>
+__device__ __forceinline__ float2 stage_twiddle(const float2* __restrict__ twg, int m) {
+  return twg[(m % P) * (m / P + 1)];
+}
 // r2c along z, nh = nz/2 = N complex per row, R rows per CTA.
 // With `clear` (the input mesh itself) each input value is overwritten with 0 by the thread
 // that read it, so a density mesh comes out cleared for the next paint.
@@ -131,11 +159,12 @@ __global__ void __launch_bounds__(RowCfg<N>::T) k_rfft_z_reg(const float* in, fl
                                                              const float2* __restrict__ twg2, long long in_b,
                                                              long long out_b, float* clear) {
   constexpr int P = Split<N>::P, Q = Split<N>::Q, R = RowCfg<N>::R, T = RowCfg<N>::T;
-  constexpr int S = P * (Q + 1);
+  constexpr int S = RowSmem<N>::S, YS = RowSmem<N>::YS, ZS = RowSmem<N>::ZS;
   extern __shared__ float2 sm[];
   float2* tw = sm;
-  float2* tw2 = tw + N;        // N+1 entries: exp(-2 pi i k / (2N))
-  float2* ybuf = tw2 + N + 1;  // R*S; reused for the Z rows (stride N+1 <= S)
+  float2* tw2 = tw + N;       // N+1 entries: exp(-2 pi i k / (2N))
+  float2* tws = tw2 + N + 1;  // stage-1 twiddles
+  float2* ybuf = tws + RowSmem<N>::TWS;  // rows of stride S; reused for the Z rows (stride ZS)
   in += (long long)blockIdx.y * in_b;
   out += (long long)blockIdx.y * out_b;
   if (clear) clear += (long long)blockIdx.y * in_b;
@@ -144,6 +173,7 @@ __global__ void __launch_bounds__(RowCfg<N>::T) k_rfft_z_reg(const float* in, fl
   grid_wait();
   for (int m = tid; m < N; m += T) tw[m] = twg[m];
   for (int m = tid; m <= N; m += T) tw2[m] = twg2[m];
+  for (int m = tid; m < RowSmem<N>::TWS; m += T) tws[m] = stage_twiddle<P>(twg, m);
   __syncthreads();
   const int row0 = blockIdx.x * R;
   const float2* in2 = reinterpret_cast<const float2*>(in);
@@ -170,50 +200,56 @@ __global__ void __launch_bounds__(RowCfg<N>::T) k_rfft_z_reg(const float* in, fl
     RegDFT<Q, -1, P>::run(u, tw);
 #pragma unroll
     for (int kb = 0; kb < Q; ++kb)
-      ybuf[r * S + t * (Q + 1) + kb] = (kb == 0) ? u[0] : cmul(u[kb], twid<-1>(tw, t * kb));
+      ybuf[r * S + t * YS + kb] = (kb == 0) ? u[0] : cmul(u[kb], RowSmem<N>::kStaged ? tws[(kb - 1) * P + t] : tw[t * kb]);
   }
   __syncthreads();
   const int kb = tid % Q, r = tid / Q;
   float2 u[P];
 #pragma unroll
-  for (int t = 0; t < P; ++t) u[t] = ybuf[r * S + t * (Q + 1) + kb];
+  for (int t = 0; t < P; ++t) u[t] = ybuf[r * S + t * YS + kb];
   RegDFT<P, -1, Q>::run(u, tw);
   __syncthreads();
 #pragma unroll
-  for (int ka = 0; ka < P; ++ka) ybuf[r * (N + 1) + kb + Q * ka] = u[ka];
+  for (int ka = 0; ka < P; ++ka) ybuf[r * ZS + kb + Q * ka] = u[ka];
   __syncthreads();
-  for (int w = tid; w < R * (N + 1); w += T) {
-    const int rr = w / (N + 1);
-    const int k = w - rr * (N + 1);
-    const int row = row0 + rr;
-    if (row >= nrows) continue;
-    const float2 zk = ybuf[rr * (N + 1) + (k == N ? 0 : k)];
-    const float2 zm = ybuf[rr * (N + 1) + (k == 0 ? 0 : N - k)];
+  const auto untangle = [](float2 zk, float2 zm, float2 w) {
     const float2 e = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
     const float2 d = make_float2(zk.x - zm.x, zk.y + zm.y);
     const float2 o = make_float2(0.5f * d.y, -0.5f * d.x);
-    out[(long long)row * (N + 1) + k] = cadd(e, cmul(tw2[k], o));
+    return cadd(e, cmul(w, o));
+  };
+  constexpr int H = N / 2 + 1;
+  for (int w = tid; w < R * H; w += T) {
+    const int rr = w / H;
+    const int k = w - rr * H;
+    const int row = row0 + rr;
+    if (row >= nrows) continue;
+    const float2 zk = ybuf[rr * ZS + k];
+    const float2 zm = ybuf[rr * ZS + (k == 0 ? 0 : N - k)];
+    float2* dst = out + (long long)row * (N + 1);
+    dst[k] = untangle(zk, zm, tw2[k]);
+    if (2 * k != N) dst[N - k] = untangle(zm, zk, tw2[N - k]);
   }
 }
 
 // c2r along z (unnormalised times `scale`). A CTA's input rows are one contiguous block; its
 // threads bring it into shared memory with asynchronous 16-byte copies, so the whole block is
 // in flight at once (a loop of loads, each waited for before its store, left the pass at 2.0
-// TB/s: 384^3 222 -> 98 us, 256^3 41.5 -> 26.6 us, 64^3 6.0 -> 3.7 us).
+// TB/s: 384^3 222 -> 98 us (91 with RowSmem), 256^3 41.5 -> 26.6 us, 64^3 6.0 -> 3.7 us).
 template <int N>
 __global__ void __launch_bounds__(RowCfg<N>::T) k_irfft_z_reg(const float2* __restrict__ in, float* __restrict__ out,
                                                               int nrows, float scale, const float2* __restrict__ twg,
                                                               const float2* __restrict__ twg2, long long in_b,
                                                               long long out_b) {
   constexpr int P = Split<N>::P, Q = Split<N>::Q, R = RowCfg<N>::R, T = RowCfg<N>::T;
-  constexpr int S = P * (Q + 1);
+  constexpr int S = RowSmem<N>::S, YS = RowSmem<N>::YS;
   constexpr int IT = (R * P + T - 1) / T;  // stage-1 items per thread
   extern __shared__ __align__(16) float2 sm[];
-  constexpr int XB = (R * (N + 1) > R * S ? R * (N + 1) : R * S);
   float2* xbuf = sm;  // R*(N+1) input rows, then (aliased) the R*S exchange buffer
   float2* ybuf = xbuf;
-  float2* tw = sm + XB;
+  float2* tw = sm + RowSmem<N>::XB;
   float2* tw2 = tw + N;
+  float2* tws = tw2 + N + 1;  // stage-1 twiddles
   in += (long long)blockIdx.y * in_b;
   out += (long long)blockIdx.y * out_b;
   const int tid = threadIdx.x;
@@ -230,6 +266,7 @@ __global__ void __launch_bounds__(RowCfg<N>::T) k_irfft_z_reg(const float2* __re
   }
   for (int m = tid; m < N; m += T) tw[m] = twg[m];
   for (int m = tid; m <= N; m += T) tw2[m] = twg2[m];
+  for (int m = tid; m < RowSmem<N>::TWS; m += T) tws[m] = stage_twiddle<P>(twg, m);
   copy_async_wait();
   __syncthreads();
   float2 u1[IT][Q];
@@ -257,14 +294,14 @@ __global__ void __launch_bounds__(RowCfg<N>::T) k_irfft_z_reg(const float2* __re
     const int t = w % P, r = w / P;
 #pragma unroll
     for (int kb = 0; kb < Q; ++kb)
-      ybuf[r * S + t * (Q + 1) + kb] = (kb == 0) ? u1[it][0] : cmul(u1[it][kb], twid<1>(tw, t * kb));
+      ybuf[r * S + t * YS + kb] = (kb == 0) ? u1[it][0] : cmul(u1[it][kb], conjf2(RowSmem<N>::kStaged ? tws[(kb - 1) * P + t] : tw[t * kb]));
   }
   __syncthreads();
   const int kb = tid % Q, r = tid / Q;
   const int row = row0 + r;
   float2 u[P];
 #pragma unroll
-  for (int t = 0; t < P; ++t) u[t] = ybuf[r * S + t * (Q + 1) + kb];
+  for (int t = 0; t < P; ++t) u[t] = ybuf[r * S + t * YS + kb];
   RegDFT<P, 1, Q>::run(u, tw);
   if (row < nrows) {
     float2* dst = reinterpret_cast<float2*>(out) + (long long)row * N + kb;
@@ -276,12 +313,12 @@ __global__ void __launch_bounds__(RowCfg<N>::T) k_irfft_z_reg(const float2* __re
 template <int N>
 static cudaError_t rfft_z_reg(const float* in, float2* out, const MeshDims& d, float sub, cudaStream_t s,
                               float* clear) {
-  constexpr int R = RowCfg<N>::R, T = RowCfg<N>::T, P = Split<N>::P, Q = Split<N>::Q;
+  constexpr int R = RowCfg<N>::R, T = RowCfg<N>::T;
   const float2* tw = twiddle_table(N);
   const float2* tw2 = twiddle_table(2 * N);
   if (!tw || !tw2) return cudaErrorMemoryAllocation;
   const int nrows = d.nx * d.ny;
-  const size_t smem = ((size_t)N + N + 1 + (size_t)R * P * (Q + 1)) * sizeof(float2);
+  const size_t smem = (size_t)RowSmem<N>::r2c * sizeof(float2);
   cudaFuncSetAttribute(k_rfft_z_reg<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   launch_next(overlap_starts(d.cells() * d.batch), k_rfft_z_reg<N>, dim3((nrows + R - 1) / R, d.batch), T, smem, s, in,
               out, nrows, sub, tw, tw2, d.cells(), d.spec_elems(), clear);
@@ -291,13 +328,12 @@ static cudaError_t rfft_z_reg(const float* in, float2* out, const MeshDims& d, f
 
 template <int N>
 static cudaError_t irfft_z_reg(const float2* in, float* out, const MeshDims& d, float scale, cudaStream_t s) {
-  constexpr int R = RowCfg<N>::R, T = RowCfg<N>::T, P = Split<N>::P, Q = Split<N>::Q;
+  constexpr int R = RowCfg<N>::R, T = RowCfg<N>::T;
   const float2* tw = twiddle_table(N);
   const float2* tw2 = twiddle_table(2 * N);
   if (!tw || !tw2) return cudaErrorMemoryAllocation;
   const int nrows = d.nx * d.ny;
-  const size_t rows_buf = (size_t)R * P * (Q + 1) > (size_t)R * (N + 1) ? (size_t)R * P * (Q + 1) : (size_t)R * (N + 1);
-  const size_t smem = ((size_t)N + N + 1 + rows_buf) * sizeof(float2);
+  const size_t smem = (size_t)RowSmem<N>::c2r * sizeof(float2);
   cudaFuncSetAttribute(k_irfft_z_reg<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   launch_next(overlap_starts(d.cells() * d.batch), k_irfft_z_reg<N>, dim3((nrows + R - 1) / R, d.batch), T, smem, s, in,
               out, nrows, scale, tw, tw2, d.spec_elems(), d.cells());
