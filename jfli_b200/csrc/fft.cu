@@ -101,41 +101,31 @@ static PkArgs pk_args(const MeshDims& d, const float* kedges, int nedges, const 
 }
 
 cudaError_t rfft3d_forward(const float* in, float2* spec, const MeshDims& d, float sub, cudaStream_t s) {
-  cudaError_t e = launch_rfft_z(in, spec, d, sub, s);
-  if (e != cudaSuccess) return e;
-  e = launch_cols(-1, spec, y_geom(d), d.spec_elems(), d.batch, s);
+  const cudaError_t e = launch_forward_zy(in, spec, d, sub, s);
   if (e != cudaSuccess) return e;
   return launch_cols(-1, spec, x_geom(d), d.spec_elems(), d.batch, s);
 }
 
 // 2D r2c of (ny, nz) maps: the z and y passes of rfft3d_forward on a mesh with nx = 1
 cudaError_t rfft2d_forward(const float* in, float2* spec, const MeshDims& d, cudaStream_t s) {
-  cudaError_t e = launch_rfft_z(in, spec, d, 0.0f, s);
-  if (e != cudaSuccess) return e;
-  return launch_cols(-1, spec, y_geom(d), d.spec_elems(), d.batch, s);
+  return launch_forward_zy(in, spec, d, 0.0f, s);
 }
 
 cudaError_t rfft3d_inverse(float2* spec, float* out, const MeshDims& d, float scale, cudaStream_t s) {
-  cudaError_t e = launch_cols(1, spec, x_geom(d), d.spec_elems(), d.batch, s);
+  const cudaError_t e = launch_cols(1, spec, x_geom(d), d.spec_elems(), d.batch, s);
   if (e != cudaSuccess) return e;
-  e = launch_cols(1, spec, y_geom(d), d.spec_elems(), d.batch, s);
-  if (e != cudaSuccess) return e;
-  return launch_irfft_z(spec, out, d, scale, s);
+  return launch_inverse_yz(spec, out, d, scale, s);
 }
 
 // real mesh -> (forward 3D FFT, k-space op, inverse 3D FFT) -> real mesh. `mixed`: see reg_fft_length
 template <class Op>
 static cudaError_t filter_chain(const float* in, float2* spec, float* out, const MeshDims& d, float sub, const Op& op,
                                 cudaStream_t s, float* clear = nullptr, bool mixed = true) {
-  cudaError_t e = launch_rfft_z(in, spec, d, sub, s, clear, mixed);
-  if (e != cudaSuccess) return e;
-  e = launch_cols(-1, spec, y_geom(d), d.spec_elems(), d.batch, s, mixed);
+  cudaError_t e = launch_forward_zy(in, spec, d, sub, s, clear, mixed);
   if (e != cudaSuccess) return e;
   e = launch_x_op(spec, d, op, s, mixed);
   if (e != cudaSuccess) return e;
-  e = launch_cols(1, spec, y_geom(d), d.spec_elems(), d.batch, s, mixed);
-  if (e != cudaSuccess) return e;
-  return launch_irfft_z(spec, out, d, 1.0f, s, mixed);
+  return launch_inverse_yz(spec, out, d, 1.0f, s, mixed);
 }
 
 cudaError_t poisson_potential(const float* rho, float2* spec, float* pot, const MeshDims& d, float rho_mean,
@@ -228,9 +218,7 @@ cudaError_t power_poles_adjoint(const float* mesh, float2* spec, float* out, con
 
 cudaError_t power_partials(const float* mesh, float2* spec, double* partials, const MeshDims& d, const float* kedges,
                            int nedges, const float* box, float norm, cudaStream_t s) {
-  cudaError_t e = launch_rfft_z(mesh, spec, d, 0.0f, s);
-  if (e != cudaSuccess) return e;
-  e = launch_cols(-1, spec, y_geom(d), d.spec_elems(), d.batch, s);
+  const cudaError_t e = launch_forward_zy(mesh, spec, d, 0.0f, s);
   if (e != cudaSuccess) return e;
   return launch_x_pk(spec, d, pk_args(d, kedges, nedges, box, norm, partials), s);
 }

@@ -112,6 +112,11 @@ cudaError_t rfft_z_generic(const float* in, float2* out, const MeshDims& d, floa
 cudaError_t launch_cols(int sign, float2* data, const ColGeom& g, long long bstride, int batch, cudaStream_t s,
                         bool mixed = true);
 cudaError_t cols_generic(int sign, float2* data, const ColGeom& g, long long bstride, int batch, cudaStream_t s);
+// ---- fft_planes.cu: r2c along z and forward y, inverse y and c2r along z, in one kernel or two
+cudaError_t launch_forward_zy(const float* in, float2* spec, const MeshDims& d, float sub, cudaStream_t s,
+                              float* clear = nullptr, bool mixed = true);
+cudaError_t launch_inverse_yz(float2* spec, float* out, const MeshDims& d, float scale, cudaStream_t s,
+                              bool mixed = true);
 // ---- fft_x.cu, fft_x_mixed.cu
 cudaError_t launch_x_op(float2* data, const MeshDims& d, const PoissonOp& op, cudaStream_t s, bool mixed);
 cudaError_t launch_x_op(float2* data, const MeshDims& d, const PgdOp& op, cudaStream_t s, bool mixed);

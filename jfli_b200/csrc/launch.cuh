@@ -27,7 +27,8 @@ __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.la
 // there is nothing to win, and the CTAs that wait take shared memory and L1 from the ones at
 // work. Off -> on, forces: 48^3 48.0 -> 37.1 us, 64^3 51.4 -> 40.3, 96^3 74.8 -> 67.2, 128^3 130.6 ->
 // 128.4, 216^3 452 -> 437, 256^3 682 -> 687; 2LPT and 10 steps: 128^3 1.73 -> 1.62 ms, 216^3
-// 6.48 -> 6.27, 256^3 7.65 -> 7.67; 2LPT, 40 steps at 256^3 25.9 -> 26.3 ms. The particle passes
+// 6.48 -> 6.27, 256^3 7.65 -> 7.67; 2LPT, 40 steps at 256^3 25.9 -> 26.3 ms (measured with the z
+// and y passes apart at every size; 64^3 forces are 35.8 us with them together). The particle passes
 // are left out at every size (launched plainly, no grid_release): with the next pass's CTAs on
 // their SMs their gathers lose L1 (256^3 step 345 -> 470 us, 64^3 forces 40 -> 45).
 inline bool overlap_starts(long long cells) { return cells < (1ll << 24); }
