@@ -5,10 +5,11 @@ The reference computes angular power spectra with healpy.anafast
 published algorithm with the map, the a_lm and the spectrum on the device, in the
 library's FP64 kernels:
 
-* the ring transforms along phi (`jfli_sht_ring_analysis`, `jfli_sht_ring_synthesis`):
-  F_r(m) = e^{-i m phi_0} sum_j f_j e^{-2 pi i m j / n_r};
-* the O(lmax^2 x rings) Legendre stages (`jfli_sht_map2alm`, `jfli_sht_alm2map`) with
-  uniform quadrature weights 4 pi / npix and a_lm packed by m (a[m][l - m]);
+* the ring transforms along phi: F_r(m) = e^{-i m phi_0} sum_j f_j e^{-2 pi i m j / n_r};
+* the O(lmax^2 x rings) Legendre stages with uniform quadrature weights 4 pi / npix and a_lm
+  packed by m (a[m][l - m]); both stages of a batch of maps in one call (`jfli_sht_maps2alm`,
+  `jfli_sht_alm2maps`; the stages apart: `jfli_sht_ring_analysis`, `jfli_sht_map2alm`,
+  `jfli_sht_alm2map`, `jfli_sht_ring_synthesis`);
 * healpy's default iterative refinement (iter=3): a += map2alm(map - alm2map(a));
 * C_l = (Re a_l0 b_l0* + 2 sum_{m>0} Re a_lm b_lm*) / (2l + 1) (`jfli_sht_alm2cl`).
 lambda_lm are the orthonormal associated Legendre functions with the Condon-Shortley
