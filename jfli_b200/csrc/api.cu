@@ -1557,7 +1557,7 @@ int jfli_lpt_adjoint(void* stream, const float* ic, int order, float c1x, float 
     if (e == cudaSuccess) e = jfli::divergence_fd(lam_x, c2x, lam_v, c2p * c2x, 1, 0, sbar, d, s);
     if (e == cudaSuccess) e = jfli::poisson_potential(sbar, spec, sbar, d, 0.0f, 1.0f, s);
     // dL/dphi1 accumulated into acc, then the common P: dL/dic = P(div ubar_1 + dL/dphi1)
-    if (e == cudaSuccess) e = jfli::lpt2_source_adjoint(phi1, sbar, q, acc, 1, d, s);
+    if (e == cudaSuccess) e = jfli::lpt2_source_adjoint(phi1, sbar, (float*)spec, q, acc, 1, d, s);
   }
   if (e == cudaSuccess) e = jfli::poisson_potential(acc, spec, out, d, 0.0f, 1.0f, s);
   return cuda_status(e, err, errlen, "jfli_lpt_adjoint");

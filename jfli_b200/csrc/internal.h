@@ -87,8 +87,9 @@ cudaError_t lpt2_source_meshes(const float* F, float* out, const MeshDims& d, cu
 cudaError_t lpt_apply(const float* pot1, const float* pot2, float c1x, float c2x, float c1p, float c2p, float* dx,
                       float* p, const MeshDims& d, cudaStream_t s);
 cudaError_t axpy_particles(float* y, const float* x, float a, const MeshDims& d, cudaStream_t s);
-// q: six scratch meshes; out (+)= dL/dphi1 for sbar = dL/d delta2.
-cudaError_t lpt2_source_adjoint(const float* pot, const float* sbar, float* q, float* out, int accumulate,
+// q: six scratch meshes, scratch: one; out (+)= dL/dphi1 for sbar = dL/d delta2. pot and sbar are
+// overwritten.
+cudaError_t lpt2_source_adjoint(float* pot, float* sbar, float* scratch, float* q, float* out, int accumulate,
                                 const MeshDims& d, cudaStream_t s);
 
 // ---- lightcone.cu ----
