@@ -267,9 +267,26 @@ __device__ __forceinline__ double small_asin(double s) {
   return s + s * q * (1.0 / 6.0 + q * (3.0 / 40.0 + q * (15.0 / 336.0 + q * (105.0 / 3456.0))));
 }
 
-// The pixels and weights of interp_weights for the direction of v (s2 = vx^2 + vy^2, inv_r = 1
-// / |v|), in FP64 but without its inverse trigonometry and divisions, which were nearly all of
-// a deposit's ~700 FP64 instructions:
+// The direction that stands for v / |v| where |v| is 0 or infinite and the quotient is not a
+// number, which no table may be read at: that of interp_weights' clamped angles. A particle at
+// the observer, or infinitely far along z, counts as the south pole, one infinitely far along
+// x or y as on the equator.
+__device__ __forceinline__ void clamped_direction(double& vx, double& vy, double& vz, double& s2, double& r) {
+  const bool pole = r == 0.0 || isinf(vz);
+  vx = !pole && isinf(vx) ? copysign(1.0, vx) : 0.0;
+  vy = !pole && isinf(vy) ? copysign(1.0, vy) : 0.0;
+  vz = pole ? -1.0 : 0.0;
+  s2 = vx * vx + vy * vy;
+  r = s2 > 1.0 ? 1.4142135623730951 : 1.0;
+}
+
+// Whether rmin < r <= rmax lets r = 0 or r = infinity in. Only such shells are painted with `any`
+// set: the look at r takes 1% of the kernels' time elsewhere (a branch that merges v again).
+static bool shell_admits_any(double rmin, double rmax) { return !(rmin >= 0.0) || std::isinf(rmax); }
+
+// The pixels and weights of interp_weights for the direction of v (s2 = vx^2 + vy^2, r = |v|,
+// neither 0 nor infinite unless `any`), in FP64 but without its inverse trigonometry and
+// divisions, which were nearly all of a deposit's ~700 FP64 instructions:
 //   * theta - theta_1 (to the ring above) is asin(sin theta cos theta_1 - cos theta sin theta_1),
 //     a small angle, from tabulated cos and sin of the rings; the gap's reciprocal is tabulated;
 //   * phi is a tabulated longitude phi_k near it (found in FP32; any neighbour does) plus
@@ -277,8 +294,11 @@ __device__ __forceinline__ double small_asin(double s) {
 //     a ring of n pixels is n k / kPhiTable (exact) + n (phi - phi_k) / 2 pi.
 // Pixel numbers fit 32 bits (nside <= 8192). Shells of 256^3 particles at nside 256 (16
 // shells, 8.7M deposits): 1.44 -> 0.94 ms, and 0.27 with the lookup of ShellSet.
-__device__ __forceinline__ void bilinear_pixels(double vx, double vy, double vz, double s2, double inv_r, int nside,
+template <bool any>
+__device__ __forceinline__ void bilinear_pixels(double vx, double vy, double vz, double s2, double r, int nside,
                                                 const HealpixTables& tb, int pix[4], double w[4]) {
+  if (any && !(r > 0.0 && r < INFINITY)) clamped_direction(vx, vy, vz, s2, r);
+  const double inv_r = 1.0 / r;
   const double z = vz * inv_r;
   const int above = ring_above(z, nside);
   const double inv_s = s2 > 0.0 ? rsqrt(s2) : 0.0;
@@ -335,13 +355,14 @@ __device__ __forceinline__ void deposit_pixels(const int pix[4], const double wt
     if (pix[q] >= 0 && pix[q] < npix) atomicAdd(map + pix[q], (float)(wt[q] * (double)w));
 }
 
-// Deposit of weight w at direction (vx, vy, vz) (length rr > 0, FP64) on the RING map.
+// Deposit of weight w at direction (vx, vy, vz) (length rr, FP64; bilinear without `any`: neither 0
+// nor infinite) on the RING map.
 // scheme 0: nearest pixel; 1: bilinear weights of the 4 surrounding pixel centres; 2 (the
 // "rbf_neighbor" scheme): the same 4 pixels weighted by a Gaussian radial basis function of
 // the angle d between the direction and each pixel centre, exp(-d^2 / (2 sigma^2)),
 // normalised to sum 1 (sigma in radians; taken relative to the nearest centre, so the
 // weights never all underflow).
-template <int scheme>
+template <int scheme, bool any>
 __device__ __forceinline__ void deposit_direction(double vx, double vy, double vz, double rr, float w, int nside,
                                                   const HealpixTables& tb, float* __restrict__ map,
                                                   float sigma = 0.f) {
@@ -349,7 +370,7 @@ __device__ __forceinline__ void deposit_direction(double vx, double vy, double v
   if (scheme == 1) {
     int pix[4];
     double wt[4];
-    bilinear_pixels(vx, vy, vz, vx * vx + vy * vy, 1.0 / rr, nside, tb, pix, wt);
+    bilinear_pixels<any>(vx, vy, vz, vx * vx + vy * vy, rr, nside, tb, pix, wt);
     deposit_pixels(pix, wt, w, npix, map);
     return;
   }
@@ -464,7 +485,7 @@ __device__ __forceinline__ double shell_position(const float* __restrict__ disp,
   return v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
 }
 
-template <int scheme>
+template <int scheme, bool any>
 __global__ void __launch_bounds__(256, scheme == 1 ? 4 : 2) k_healpix_paint_shells(const float* __restrict__ disp, int absolute,
                                                               const float* __restrict__ weights, float weight, PGrid g,
                                                               double3 cell, double3 obs, ShellSet shells, int nside,
@@ -496,7 +517,7 @@ __global__ void __launch_bounds__(256, scheme == 1 ? 4 : 2) k_healpix_paint_shel
     if (first < 0) continue;
     int pix[4];
     double wt[4];
-    if (scheme == 1) bilinear_pixels(v[0], v[1], v[2], v[0] * v[0] + v[1] * v[1], 1.0 / rr, nside, tb, pix, wt);
+    if (scheme == 1) bilinear_pixels<any>(v[0], v[1], v[2], v[0] * v[0] + v[1] * v[1], rr, nside, tb, pix, wt);
     for (int sh = first; sh < shells.n; ++sh) {
       if (sh > first && !(rf >= shells.lo[sh] && rf <= shells.hi[sh] && rr > shells.rmin[sh] && rr <= shells.rmax[sh]))
         continue;
@@ -504,7 +525,7 @@ __global__ void __launch_bounds__(256, scheme == 1 ? 4 : 2) k_healpix_paint_shel
       if (scheme == 1)
         deposit_pixels(pix, wt, w * shells.scale[sh], (int)npix, map);
       else
-        deposit_direction<scheme>(v[0], v[1], v[2], rr, w * shells.scale[sh], nside, tb, map, sigma);
+        deposit_direction<scheme, any>(v[0], v[1], v[2], rr, w * shells.scale[sh], nside, tb, map, sigma);
       if (shells.disjoint) break;
     }
   }
@@ -627,7 +648,7 @@ struct TileCull {
   float4 t[kMaxTiles];  // 2 M^T s, |s|^2
 };
 
-template <int scheme>
+template <int scheme, bool any>
 __global__ void __launch_bounds__(kTiledThreads, 4)
     k_healpix_paint_tiled(const float* __restrict__ disp, int absolute, const float* __restrict__ vel,
                           const float* __restrict__ weights, float weight, PGrid g, float3 box, float3 obs, TileSet ts,
@@ -692,7 +713,7 @@ __global__ void __launch_bounds__(kTiledThreads, 4)
     }
     const double rr = sqrt(qd[0] * qd[0] + qd[1] * qd[1] + qd[2] * qd[2]);
     if (!(rr > (double)rmin && rr <= (double)rmax)) return;
-    deposit_direction<scheme>(qd[0], qd[1], qd[2], rr, weights ? weights[p] * weight : weight, nside, ht, map);
+    deposit_direction<scheme, any>(qd[0], qd[1], qd[2], rr, weights ? weights[p] * weight : weight, nside, ht, map);
   };
   unsigned count = 0;  // queued pairs, the same in every lane
   for (unsigned p0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); p0 < g.np; p0 += gridDim.x * blockDim.x) {
@@ -1051,17 +1072,22 @@ static cudaError_t launch_shells(const float* disp, int absolute, const float* w
   HealpixTables tb;
   if (!ring_tables(nside, &tb)) return cudaErrorMemoryAllocation;
   set.bound();
+  bool any = false;
+  for (int i = 0; i < set.n; ++i) any = any || shell_admits_any(set.rmin[i], set.rmax[i]);
   const dim3 grid = particle_grid_dims(d.cells(), d.batch, 256, 16);
   const PGrid g = make_pgrid(d);
   if (scheme == 0)
-    k_healpix_paint_shells<0><<<grid, 256, 0, s>>>(disp, absolute, weights, weight, g, cell, obs, set, nside, tb, maps,
-                                                   sigma);
+    k_healpix_paint_shells<0, false><<<grid, 256, 0, s>>>(disp, absolute, weights, weight, g, cell, obs, set, nside, tb,
+                                                          maps, sigma);
+  else if (scheme == 1 && any)
+    k_healpix_paint_shells<1, true><<<grid, 256, 0, s>>>(disp, absolute, weights, weight, g, cell, obs, set, nside, tb,
+                                                         maps, sigma);
   else if (scheme == 1)
-    k_healpix_paint_shells<1><<<grid, 256, 0, s>>>(disp, absolute, weights, weight, g, cell, obs, set, nside, tb, maps,
-                                                   sigma);
+    k_healpix_paint_shells<1, false><<<grid, 256, 0, s>>>(disp, absolute, weights, weight, g, cell, obs, set, nside, tb,
+                                                          maps, sigma);
   else
-    k_healpix_paint_shells<2><<<grid, 256, 0, s>>>(disp, absolute, weights, weight, g, cell, obs, set, nside, tb, maps,
-                                                   sigma);
+    k_healpix_paint_shells<2, false><<<grid, 256, 0, s>>>(disp, absolute, weights, weight, g, cell, obs, set, nside, tb,
+                                                          maps, sigma);
   note_launch();
   return cudaGetLastError();
 }
@@ -1169,11 +1195,17 @@ cudaError_t healpix_paint_tiled(const float* disp, int absolute, const float* ve
   }
   const float3 bx = make_float3(box[0], box[1], box[2]), ob = make_float3(observer[0], observer[1], observer[2]);
   if (scheme == 0)
-    k_healpix_paint_tiled<0><<<grid, 256, 0, s>>>(disp, absolute, vel, weights, weight, make_pgrid(d), bx, ob, ts, cull,
-                                                  telephoto, rmin, rmax, t, gp_t, dbound, tb, nside, tab, map);
+    k_healpix_paint_tiled<0, false><<<grid, 256, 0, s>>>(disp, absolute, vel, weights, weight, make_pgrid(d), bx, ob, ts,
+                                                         cull, telephoto, rmin, rmax, t, gp_t, dbound, tb, nside, tab,
+                                                         map);
+  else if (shell_admits_any(rmin, rmax))
+    k_healpix_paint_tiled<1, true><<<grid, 256, 0, s>>>(disp, absolute, vel, weights, weight, make_pgrid(d), bx, ob, ts,
+                                                        cull, telephoto, rmin, rmax, t, gp_t, dbound, tb, nside, tab,
+                                                        map);
   else
-    k_healpix_paint_tiled<1><<<grid, 256, 0, s>>>(disp, absolute, vel, weights, weight, make_pgrid(d), bx, ob, ts, cull,
-                                                  telephoto, rmin, rmax, t, gp_t, dbound, tb, nside, tab, map);
+    k_healpix_paint_tiled<1, false><<<grid, 256, 0, s>>>(disp, absolute, vel, weights, weight, make_pgrid(d), bx, ob, ts,
+                                                         cull, telephoto, rmin, rmax, t, gp_t, dbound, tb, nside, tab,
+                                                         map);
   note_launch();
   return cudaGetLastError();
 }
