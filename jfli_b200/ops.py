@@ -15,6 +15,7 @@ import collections
 import ctypes
 import functools
 import math
+import threading
 
 import numpy as np
 import torch
@@ -38,30 +39,70 @@ def workspace(nbytes: int, key: str = "default", device=None) -> torch.Tensor:
     return buf
 
 
-_TABLES: "collections.OrderedDict[tuple, torch.Tensor]" = collections.OrderedDict()
+class _Table:
+    """A table of device_table: the tensor, the stream it went up on with the event behind the
+    copy, the other streams that have waited for it, whether a CUDA graph reads it."""
+
+    __slots__ = ("tensor", "event", "streams", "captured")
+
+    def __init__(self, tensor, event, streams):
+        self.tensor, self.event, self.streams, self.captured = tensor, event, streams, False
+
+
+_TABLES: "collections.OrderedDict[tuple, _Table]" = collections.OrderedDict()
+_TABLES_MOST = 64  # beside those that graphs read
+_tables_captured = 0
+_tables_lock = threading.Lock()  # the serving engine's threads share the tables
 
 
 def device_table(values, device="cuda", dtype=np.float32) -> torch.Tensor:
-    """A small host table (bin edges, P(k) samples) on the device, cached by content (and by
-    the stream it went up on, so that no other stream reads it too early) and read-only for
-    callers. A copy from pageable host memory makes the host wait until the
+    """A small host table (bin edges, P(k) samples) on the device, cached by content and
+    read-only for callers. A copy from pageable host memory makes the host wait until the
     stream has drained, which stalls a caller that enqueues the next request while the GPU
     works on this one: a table met before is reused, a new one goes up through pinned
-    memory without blocking."""
+    memory without blocking. Another stream than the one it went up on waits for the copy
+    (on the device) before it reads the table first. Under stream capture a table met before
+    is used as it is and kept for good, so a call warmed up outside, on any stream, captures
+    no copy; a new one belongs to that capture alone."""
+    global _tables_captured
     a = np.ascontiguousarray(np.asarray(values, dtype=dtype))
     dev = torch.device(device)
-    stream = stream_ptr() if dev.type == "cuda" else 0
-    key = (a.tobytes(), a.shape, a.dtype.str, str(dev), stream)
-    t = _TABLES.get(key)
-    if t is None:
+    stream = capturing = None
+    if dev.type == "cuda":
+        here = torch.cuda.current_device()
+        dev = torch.device("cuda", here if dev.index is None else dev.index)
+        stream = torch._C._cuda_getCurrentRawStream(dev.index)
+        if dev.index == here:
+            capturing = torch.cuda.is_current_stream_capturing()
+        else:
+            with torch.cuda.device(dev):
+                capturing = torch.cuda.is_current_stream_capturing()
+    key = (a.tobytes(), a.shape, a.dtype.str, str(dev))
+    with _tables_lock:
+        e = _TABLES.get(key)
+        if e is not None:
+            _TABLES.move_to_end(key)
+            if capturing:
+                _tables_captured += not e.captured
+                e.captured = True
+            elif stream is not None and stream not in e.streams:
+                s = torch.cuda.current_stream(dev)
+                s.wait_event(e.event)
+                e.tensor.record_stream(s)
+                e.streams.add(stream)
+            return e.tensor
         t = torch.from_numpy(a.copy())
-        t = t.pin_memory().to(dev, non_blocking=True) if dev.type == "cuda" else t.to(dev)
-        _TABLES[key] = t
-        if len(_TABLES) > 64:
-            _TABLES.popitem(last=False)
-    else:
-        _TABLES.move_to_end(key)
-    return t
+        if stream is None:
+            e = _Table(t.to(dev), None, None)
+        else:
+            t = t.pin_memory().to(dev, non_blocking=True)
+            if capturing:
+                return t
+            e = _Table(t, torch.cuda.current_stream(dev).record_event(), {stream})
+        _TABLES[key] = e
+        if len(_TABLES) - _tables_captured > _TABLES_MOST:  # the oldest that no graph reads goes
+            del _TABLES[next(k for k, v in _TABLES.items() if not v.captured)]
+        return e.tensor
 
 
 def release_workspaces():
