@@ -486,8 +486,14 @@ def _drift_tables_host(cosmo, n_dense: int) -> tuple:
 
 def drift_tables(cosmo, n_dense: int = 4096):
     """Device FP32 copies of the FP64 host tables the light-cone drift interpolates:
-    (chi ascending, a at chi), (growth a, D1), (dense a, dGfa). One pinned copy that the host
-    does not wait for."""
+    (chi ascending, a at chi), (growth a, D1), (dense a, dGfa). They are on the device when
+    this returns: any stream may read them."""
+    host = _drift_tables_host(cosmo, n_dense)
+    return torch.split(torch.from_numpy(np.concatenate(host)).to("cuda"), [t.size for t in host])
+
+
+def _drift_tables_here(cosmo, n_dense: int = 4096):
+    """drift_tables for the current stream alone: one pinned copy that the host does not wait for."""
     host = _drift_tables_host(cosmo, n_dense)
     flat = torch.from_numpy(np.concatenate(host)).pin_memory().to("cuda", non_blocking=True)
     return torch.split(flat, [t.size for t in host])
@@ -510,7 +516,7 @@ def replica_positions(pos: torch.Tensor, box_size, observer_mpc, rotation, shift
         _check(vel, "vel")
         if t is None or cosmo is None:
             raise ValueError("the light-cone drift needs the time t and the cosmology")
-        tabs = drift_tables(cosmo) if tables is None else tables
+        tabs = _drift_tables_here(cosmo) if tables is None else tables
         t_arg = float(t)
         gp_t = float(cj.Gp(cosmo, t_arg))
     chi, a_chi, ga, g, da, dg = tabs
@@ -619,7 +625,7 @@ def _tiled_prep(pos, rotations, shifts, scheme, vel, t, cosmo, tables, dbound):
         raise ValueError("vel must have the shape of pos")
     if t is None or cosmo is None:
         raise ValueError("the light-cone drift needs the time t and the cosmology")
-    tabs = drift_tables(cosmo) if tables is None else tables
+    tabs = _drift_tables_here(cosmo) if tables is None else tables
     t_arg = float(t)
     gp_t = float(cj.Gp(cosmo, t_arg))
     if dbound is None:  # from the host's copies where there are: reading the device's would wait for the stream
@@ -692,7 +698,7 @@ def lightcone_drift_array(disp: torch.Tensor, vel: torch.Tensor, t: float, cosmo
     _check(disp, "disp")
     _check(vel, "vel")
     (nx, ny, nz), batch, _ = _mesh_dims(disp, True)
-    chi, a_chi, ga, g, da, dg = drift_tables(cosmo) if tables is None else tables
+    chi, a_chi, ga, g, da, dg = _drift_tables_here(cosmo) if tables is None else tables
     out = torch.empty_like(disp)
     lx, ly, lz = (float(v) for v in box_size)
     ox, oy, oz = (float(v) for v in observer_mpc)

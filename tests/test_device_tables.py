@@ -1,4 +1,4 @@
-"""Small tables on the device (ops.device_table): shared by threads, streams and
+"""Small tables on the device (ops.device_table, ops.drift_tables): shared by threads, streams and
 CUDA graphs."""
 
 from __future__ import annotations
@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 import torch
 
+import jfli_b200 as jf
 from jfli_b200 import ops
 
 
@@ -81,3 +82,15 @@ def test_a_table_first_met_in_a_capture_belongs_to_that_capture():
     np.testing.assert_array_equal(t.cpu().numpy(), values.astype(np.float32))
     g.replay()
     np.testing.assert_array_equal(out.cpu().numpy(), 2.0 * values.astype(np.float32))
+
+
+@pytest.mark.gpu
+def test_drift_tables_serve_any_stream():
+    want = ops._drift_tables_host(jf.Planck18(), 4096)
+    torch.cuda._sleep(20_000_000)
+    tables = ops.drift_tables(jf.Planck18())
+    with torch.cuda.stream(torch.cuda.Stream()):
+        got = [t.clone() for t in tables]
+        torch.cuda.current_stream().synchronize()
+    for g, w in zip(got, want):
+        np.testing.assert_array_equal(g.cpu().numpy(), w)
