@@ -113,6 +113,12 @@ def _dev(a) -> torch.Tensor:
     return torch.as_tensor(np.asarray(a, np.float32), device="cuda")
 
 
+def _edges(kedges, device) -> torch.Tensor:
+    """Bin edges on the device: a tensor as it is, a host table by way of ops.device_table (a
+    pageable copy would wait for the steps before it)."""
+    return _dev(kedges) if isinstance(kedges, torch.Tensor) else ops.device_table(kedges, device)
+
+
 def _dot(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     return torch.sum(a.double() * b.double())
 
@@ -398,7 +404,7 @@ class PowerSpectrum(torch.autograd.Function):
     @staticmethod
     def forward(ctx, mesh, kedges: np.ndarray, box):
         mesh = mesh.contiguous()
-        ke = ops.device_table(kedges, mesh.device)  # a pageable copy would wait for the steps before it
+        ke = _edges(kedges, mesh.device)
         sums = ops.power_sums(mesh, ke, box)
         cnt = sums[1]
         vol = float(np.prod(np.asarray(box, np.float64) / np.asarray(mesh.shape[-3:], np.float64)))
@@ -436,7 +442,7 @@ class PowerPoles(torch.autograd.Function):
         vol = float(np.prod(np.asarray(box, np.float64) / np.asarray(mesh.shape[-3:], np.float64)))
         norm = torch.where(cnt > 0, cnt, torch.ones_like(cnt))
         pk = (re / norm[None, :])[:, 1:-1] * vol
-        ctx.save_for_backward(mesh, ops.device_table(kedges, mesh.device), cnt)
+        ctx.save_for_backward(mesh, _edges(kedges, mesh.device), cnt)
         ctx.vol, ctx.box, ctx.poles, ctx.los = vol, box, tuple(int(p) for p in poles), los
         return pk[0] if nell == 1 else pk
 

@@ -94,3 +94,13 @@ def test_drift_tables_serve_any_stream():
         torch.cuda.current_stream().synchronize()
     for g, w in zip(got, want):
         np.testing.assert_array_equal(g.cpu().numpy(), w)
+
+
+@pytest.mark.gpu
+def test_bin_edges_may_be_a_device_tensor():
+    from jfli_b200.pm.adjoint import PowerSpectrum
+
+    m = torch.randn(16, 16, 16, device="cuda", requires_grad=True)
+    ke = np.linspace(0.05, 0.3, 6)
+    pk = PowerSpectrum.apply(m, torch.as_tensor(ke, device="cuda"), (300.0,) * 3)
+    torch.testing.assert_close(pk, PowerSpectrum.apply(m, ke, (300.0,) * 3))
