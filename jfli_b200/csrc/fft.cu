@@ -58,6 +58,23 @@ bool mesh_fft_supported(int nx, int ny, int nz) {
   return nz % 2 == 0 && nz >= 4 && fft_axis_supported(nx) && fft_axis_supported(ny) && fft_axis_supported(nz / 2);
 }
 
+void* device_table(const void* host, size_t bytes) {
+  // An allocation is refused while a stream is captured, by this thread or (global mode) another, but
+  // in relaxed mode: without it a length first met in a capture would fail.
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  void* d = nullptr;
+  cudaStream_t s = nullptr;
+  bool ok = cudaMalloc(&d, bytes) == cudaSuccess &&
+            cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess &&
+            cudaMemcpyAsync(d, host, bytes, cudaMemcpyHostToDevice, s) == cudaSuccess &&
+            cudaStreamSynchronize(s) == cudaSuccess;
+  if (s) cudaStreamDestroy(s);
+  if (!ok && d) cudaFree(d);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return ok ? d : nullptr;
+}
+
 // ---- twiddle tables w_n^m = exp(-2 pi i m / n), one per (device, n), built once on the host
 static std::mutex g_tw_mutex;
 static std::map<std::pair<int, int>, float2*> g_tw_tables;
@@ -74,12 +91,8 @@ const float2* twiddle_table(int n) {
     const double ang = 2.0 * M_PI * (double)m / (double)n;
     h[m] = make_float2((float)std::cos(ang), (float)-std::sin(ang));
   }
-  float2* d = nullptr;
-  if (cudaMalloc(&d, sizeof(float2) * n) != cudaSuccess) return nullptr;
-  if (cudaMemcpy(d, h.data(), sizeof(float2) * n, cudaMemcpyHostToDevice) != cudaSuccess) {
-    cudaFree(d);
-    return nullptr;
-  }
+  float2* d = static_cast<float2*>(device_table(h.data(), sizeof(float2) * n));
+  if (!d) return nullptr;
   g_tw_tables[key] = d;
   return d;
 }

@@ -1051,11 +1051,8 @@ static bool ring_tables(int nside, HealpixTables* out) {
       h[phi + 2 * k] = std::cos(2.0 * M_PI * k / kPhiTable);
       h[phi + 2 * k + 1] = std::sin(2.0 * M_PI * k / kPhiTable);
     }
-    if (cudaMalloc(&d, sizeof(double) * total) != cudaSuccess) return false;
-    if (cudaMemcpy(d, h.data(), sizeof(double) * total, cudaMemcpyHostToDevice) != cudaSuccess) {
-      cudaFree(d);
-      return false;
-    }
+    d = static_cast<double*>(device_table(h.data(), sizeof(double) * total));
+    if (!d) return false;
     g_ring_tables[key] = d;
   }
   out->theta = d;

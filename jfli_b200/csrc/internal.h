@@ -16,6 +16,10 @@ struct MeshDims {
   __host__ __device__ long long spec_elems() const { return (long long)nx * ny * (nz / 2 + 1); }
 };
 
+// A host table on the device, in memory of its own that is never freed; nullptr without memory. The
+// calling thread may be capturing a stream: the copy is on a stream of its own, and done on return.
+void* device_table(const void* host, size_t bytes);
+
 // ---- fft.cu ----
 bool fft_axis_supported(int n);
 bool mesh_fft_supported(int nx, int ny, int nz);
