@@ -164,32 +164,43 @@ struct XCarry {
 //
 // A lane that merges with neither neighbour has two adjacent cells of its own per y row: with VEC
 // (rows of a multiple of 4 cells, mesh 16-byte aligned) they go out as one 16-byte vector
-// atomic with zeros beside them, unless they lie in two aligned groups of four. On particles
-// that left their neighbours the paint is bound by the atomics' path: 216 x 144 x 324 in
-// absolute positions 269 -> 239 us, the particle pass of 256^3 347 -> 344 us over 40 steps.
-// (For every lane, merged or not: 259 and 385 us, as the merged rows' 4-byte atomics coalesce;
-// with 8-byte atomics at even cells: 239 and 364 us.)
+// atomic with zeros beside them (deposit_pair), unless they lie in two aligned groups of four. On
+// particles that left their neighbours the paint is bound by the atomics' path: the particle
+// pass of 256^3 347 -> 344 us over 40 steps (385 with vectors for every lane, merged or not, as the
+// merged rows' 4-byte atomics coalesce; 364 with 8-byte atomics at even cells); figures of the
+// paint at its kernels. A warp with lanes of both kinds issues both: with LEAST > 0 it does so
+// only from that many lanes of the one kind on.
 template <bool VEC>
+__device__ __forceinline__ void deposit_pair(float* row, int z0, int z1, float a, float b) {
+  const int q = z0 & 3;
+  if (VEC && q != 3) {
+    atomicAdd(reinterpret_cast<float4*>(row + (z0 - q)),
+              make_float4(q == 0 ? a : 0.f, q == 0 ? b : (q == 1 ? a : 0.f), q == 1 ? b : (q == 2 ? a : 0.f),
+                          q == 2 ? b : 0.f));
+  } else {
+    atomicAdd(row + z0, a);
+    atomicAdd(row + z1, b);
+  }
+}
+
+template <bool VEC, int LEAST = 0>
 __device__ __forceinline__ void deposit_plane_merged(float* rho, bool on, int xo, int yo0, int yo1, int z0, int z1,
                                                      float w00, float w01, float w10, float w11) {
   const int lane = threadIdx.x & 31;
-  const int lo = on ? xo + yo0 + z0 : -1;
-  const int hi = on ? xo + yo0 + z1 : -2;
-  const int next_lo = __shfl_down_sync(0xffffffffu, lo, 1);
-  const int prev_hi = __shfl_up_sync(0xffffffffu, hi, 1);
-  const bool give = on && lane < 31 && next_lo == hi;
-  const bool take = on && lane > 0 && prev_hi == lo;
+  const int lo0 = on ? xo + yo0 + z0 : -1;
+  const int hi0 = on ? xo + yo0 + z1 : -2;
+  const int next_lo = __shfl_down_sync(0xffffffffu, lo0, 1);
+  const int prev_hi = __shfl_up_sync(0xffffffffu, hi0, 1);
+  const bool give = on && lane < 31 && next_lo == hi0;
+  const bool take = on && lane > 0 && prev_hi == lo0;
   const float r0 = __shfl_up_sync(0xffffffffu, w01, 1);
   const float r1 = __shfl_up_sync(0xffffffffu, w11, 1);
+  bool pair = VEC && !give && !take && (z0 & 3) != 3;
+  if (LEAST > 0) pair = __popc(__ballot_sync(0xffffffffu, on && pair)) >= LEAST && pair;
   if (on) {
-    if (VEC && !give && !take && (z0 & 3) != 3) {
-      const int q = z0 & 3;
-      const float4 a = make_float4(q == 0 ? w00 : 0.f, q == 0 ? w01 : (q == 1 ? w00 : 0.f),
-                                   q == 1 ? w01 : (q == 2 ? w00 : 0.f), q == 2 ? w01 : 0.f);
-      const float4 b = make_float4(q == 0 ? w10 : 0.f, q == 0 ? w11 : (q == 1 ? w10 : 0.f),
-                                   q == 1 ? w11 : (q == 2 ? w10 : 0.f), q == 2 ? w11 : 0.f);
-      atomicAdd(reinterpret_cast<float4*>(rho + (xo + yo0 + z0 - q)), a);
-      atomicAdd(reinterpret_cast<float4*>(rho + (xo + yo1 + z0 - q)), b);
+    if (pair) {
+      deposit_pair<true>(rho + (xo + yo0), z0, z1, w00, w01);
+      deposit_pair<true>(rho + (xo + yo1), z0, z1, w10, w11);
     } else {
       atomicAdd(rho + (xo + yo0 + z0), take ? w00 + r0 : w00);
       atomicAdd(rho + (xo + yo1 + z0), take ? w10 + r1 : w10);
@@ -216,19 +227,34 @@ __device__ __forceinline__ void carry_flush(float* rho, XCarry& c) {
 // and the upper-x plane becomes the new carry. The sums reaching each cell are those of
 // deposit(); only the FP32 addition order differs. Lanes with `on` false have no particle (in
 // any plane of the walk) and take part in the shuffles only.
-template <bool VEC>
+//
+// A carry that goes out alone is deposited by carry_flush's 4-byte atomics; with WIDE, when at least
+// kWideLanes lanes of the warp have one, by deposit_pair. (From any number on: 256^3 particles that
+// keep their neighbours 151 us, from 24 on 134, never 130; particles that left them 418, 418 and
+// 517. The particle pass, at its register bound, goes without.)
+constexpr int kWideLanes = 24;
+
+template <bool VEC, bool WIDE = false>
 __device__ __forceinline__ void deposit_carried(float* rho, const PGrid& g, const Cic1& cx, const Cic1& cy,
                                                 const Cic1& cz, float w, XCarry& c, bool on = true) {
   const float wx0 = cx.w0 * w, wx1 = cx.w1 * w;
   const int xo0 = cx.i0 * g.yz, yo0 = cy.i0 * g.nz, yo1 = cy.i1 * g.nz;
   float a00 = (wx0 * cy.w0) * cz.w0, a01 = (wx0 * cy.w0) * cz.w1;
   float a10 = (wx0 * cy.w1) * cz.w0, a11 = (wx0 * cy.w1) * cz.w1;
+  bool wide = false;
+  if (WIDE) {
+    const bool alone = c.valid && !(c.xo == xo0 && c.yo0 == yo0 && c.z0 == cz.i0);
+    wide = __popc(__ballot_sync(0xffffffffu, alone)) >= kWideLanes;
+  }
   if (c.valid) {
     if (c.xo == xo0 && c.yo0 == yo0 && c.z0 == cz.i0) {
       a00 += c.w00;
       a01 += c.w01;
       a10 += c.w10;
       a11 += c.w11;
+    } else if (WIDE && wide) {
+      deposit_pair<VEC>(rho + (c.xo + c.yo0), c.z0, c.z1, c.w00, c.w01);
+      deposit_pair<VEC>(rho + (c.xo + c.yo1), c.z0, c.z1, c.w10, c.w11);
     } else {
       carry_flush(rho, c);
     }
@@ -246,22 +272,24 @@ __device__ __forceinline__ void deposit_carried(float* rho, const PGrid& g, cons
   c.valid = on;
 }
 
-// The walk of the paint and force readout: a warp takes a z row's segment of kw <= 32
-// consecutive particles and walks it along x for `depth` planes; the CTA's eight warps take
-// eight neighbouring rows in y. Neighbours that share CIC corners are then handled close in
-// time on one SM, and the paint can use the z and x merges of the brick walk, on any mesh.
+// The walk of the force readout and of the paint of large meshes: a warp takes a z row's segment of
+// kw <= 32 consecutive particles and walks it along x for `depth` planes; the CTA's eight warps
+// take eight neighbouring rows in y. Neighbours that share CIC corners are then handled close in
+// time on one SM, and the paint can use the z and x merges of the brick walk.
 struct SegWalk {
   int kw, nkb, njb, nxc, depth;
 };
 
 // Segments are of equal length; used where they fill at least three quarters of their lanes
-// (rows of 24 particles or more), the grid-stride kernels elsewhere.
-static bool seg_walk(const MeshDims& d, SegWalk* w) {
+// (rows of 24 particles or more), the grid-stride kernels elsewhere. `ctas`: the depth is halved
+// from 16 until there are so many per SM.
+static bool seg_walk(const MeshDims& d, SegWalk* w, int ctas = 4) {
   w->nkb = (d.nz + 31) / 32;
   w->kw = (d.nz + w->nkb - 1) / w->nkb;
   w->njb = (d.ny + 7) / 8;
   w->depth = 16;
-  while (w->depth > 1 && (long long)w->nkb * w->njb * d.batch * ((d.nx + w->depth - 1) / w->depth) < 4ll * sm_count())
+  while (w->depth > 1 && (long long)w->nkb * w->njb * d.batch * ((d.nx + w->depth - 1) / w->depth) <
+                             (long long)ctas * sm_count())
     w->depth >>= 1;
   w->nxc = (d.nx + w->depth - 1) / w->depth;
   return 4 * d.nz >= 3 * 32 * w->nkb;
@@ -272,7 +300,8 @@ static dim3 seg_grid(const MeshDims& d, const SegWalk& w) {
   return dim3((unsigned)(items < cap ? items : cap), d.batch);
 }
 
-// body(p, i, j, k, on) for every plane of every segment of this warp; flush() after each segment
+// body(p, i, j, k, on, i0, i1) for every plane i = i0 .. i1 - 1 of every segment of this warp; flush()
+// after each segment
 template <class Body, class Flush>
 __device__ __forceinline__ void walk_segments(const PGrid& g, const SegWalk& w, Body body, Flush flush) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -286,28 +315,72 @@ __device__ __forceinline__ void walk_segments(const PGrid& g, const SegWalk& w, 
     const bool on = lane < w.kw && k < g.nz;
     const int i1 = min(g.nx, i0 + w.depth);
     for (int i = i0; i < i1; ++i)
-      body(((unsigned)i * (unsigned)g.ny + (unsigned)j) * (unsigned)g.nz + (unsigned)k, i, j, k, on);
+      body(((unsigned)i * (unsigned)g.ny + (unsigned)j) * (unsigned)g.nz + (unsigned)k, i, j, k, on, i0, i1);
     flush();
   }
 }
 
-__device__ __forceinline__ void cic_at(const float* __restrict__ pos, int absolute, const PGrid& g, unsigned p, int i,
-                                       int j, int k, Cic1& cx, Cic1& cy, Cic1& cz) {
-  const float px = __ldcs(pos + 3ull * p), py = __ldcs(pos + 3ull * p + 1), pz = __ldcs(pos + 3ull * p + 2);
+__device__ __forceinline__ float3 position_at(const float* __restrict__ pos, unsigned p) {
+  return make_float3(__ldcs(pos + 3ull * p), __ldcs(pos + 3ull * p + 1), __ldcs(pos + 3ull * p + 2));
+}
+
+__device__ __forceinline__ void cic_at(const float3& x, int absolute, const PGrid& g, int i, int j, int k, Cic1& cx,
+                                       Cic1& cy, Cic1& cz) {
   if (absolute) {
-    cx = cic_abs(px, g.nx);
-    cy = cic_abs(py, g.ny);
-    cz = cic_abs(pz, g.nz);
+    cx = cic_abs(x.x, g.nx);
+    cy = cic_abs(x.y, g.ny);
+    cz = cic_abs(x.z, g.nz);
   } else {
-    cx = cic_rel(i, px, g.nx);
-    cy = cic_rel(j, py, g.ny);
-    cz = cic_rel(k, pz, g.nz);
+    cx = cic_rel(i, x.x, g.nx);
+    cy = cic_rel(j, x.y, g.ny);
+    cz = cic_rel(k, x.z, g.nz);
   }
 }
 
-// CIC paint. Bound by the atomics' path (L2 at 75% with the grid-stride kernel). 216 x 144 x 324
-// particles in absolute positions: 279 us grid-stride, 269 with the x merge, 239 with the
-// vector atomics of deposit_plane_merged.
+// CIC paint. Bound by the atomics' path (L2) on particles that left their neighbours, by loads in flight on
+// those that move together. Which of the two a set is cannot be told before it is painted, so
+// neither kernel may lose on one of them:
+//   * k_paint_pairs, the grid-stride walk of k_paint with vector atomics for pairs of cells from
+//     four such lanes of a warp on (rows of whole groups of four cells, 16-byte aligned mesh);
+//   * k_paint_walk, the segment walk, whose x merge saves a quarter of the atomics of particles
+//     that move together, with the next plane's position on its way and 16 CTAs per SM to cover
+//     the serial planes. On small meshes it starts too few warps and leaves lanes idle.
+// k_paint, k_paint_pairs, k_paint_walk; smooth displacements, and uniform positions:
+//   64^3    7.5, 7.2, 7.6 us and 14.5, 10.2, 10.0    144^3  30.3, 31.0, 35 and 112, 75, 73
+//   100^3  15.0, 15.0, 18.0 and 40.2, 27.1, 28       192^3  65, 70, 62 and 267, 171, 168
+//   128^3  23.2, 23.5, 25.1 and 81, 53, 52           256^3  144, 157, 134 and 650, 436, 418
+// The line is at 3 x 2^21 cells (176^3: 50, 53, 55 smooth, 204, 133, 131 uniform); 243^3, which has
+// no pairs, takes the walk for its x merge (130 and 118 us smooth, 542 and 535 uniform).
+constexpr int kPairLanes = 4;
+constexpr long long kPaintWalkCells = 3ll << 21;
+
+__global__ void __launch_bounds__(256) k_paint_pairs(const float* __restrict__ pos, int absolute,
+                                                     const float* __restrict__ weights, float weight,
+                                                     float* __restrict__ mesh, PGrid g) {
+  const long long b = blockIdx.y;
+  pos += b * g.np * 3;
+  mesh += b * g.np;
+  if (weights) weights += b * g.np;
+  const unsigned lane = threadIdx.x & 31;
+  for (unsigned p0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); p0 < g.np; p0 += gridDim.x * blockDim.x) {
+    const unsigned p = p0 + lane;
+    const bool on = p < g.np;
+    Cic1 cx = {0, 0, 0.f, 0.f}, cy = cx, cz = cx;
+    float w = 0.f;
+    if (on) {
+      cic_setup(pos + 3ull * p, p, absolute, g, cx, cy, cz);
+      w = weights ? weights[p] * weight : weight;
+    }
+    const int yo0 = cy.i0 * g.nz, yo1 = cy.i1 * g.nz;
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+      const float wx = (a ? cx.w1 : cx.w0) * w, w0 = wx * cy.w0, w1 = wx * cy.w1;
+      deposit_plane_merged<true, kPairLanes>(mesh, on, (a ? cx.i1 : cx.i0) * g.yz, yo0, yo1, cz.i0, cz.i1, w0 * cz.w0,
+                                             w0 * cz.w1, w1 * cz.w0, w1 * cz.w1);
+    }
+  }
+}
+
 template <bool VEC>
 __global__ void __launch_bounds__(256) k_paint_walk(const float* __restrict__ pos, int absolute,
                                                     const float* __restrict__ weights, float weight,
@@ -320,20 +393,24 @@ __global__ void __launch_bounds__(256) k_paint_walk(const float* __restrict__ po
   carry.valid = false;
   carry.xo = carry.yo0 = carry.yo1 = carry.z0 = carry.z1 = 0;
   carry.w00 = carry.w01 = carry.w10 = carry.w11 = 0.f;
+  float3 next = make_float3(0.f, 0.f, 0.f);
   walk_segments(
       g, walk,
-      [&](unsigned p, int i, int j, int k, bool on) {
+      [&](unsigned p, int i, int j, int k, bool on, int i0, int i1) {
+        if (on && i == i0) next = position_at(pos, p);
+        const float3 x = next;
+        if (on && i + 1 < i1) next = position_at(pos, p + (unsigned)g.yz);
         Cic1 cx = {0, 0, 0.f, 0.f}, cy = cx, cz = cx;
         float w = 0.f;
         if (on) {
-          cic_at(pos, absolute, g, p, i, j, k, cx, cy, cz);
+          cic_at(x, absolute, g, i, j, k, cx, cy, cz);
           w = weights ? weights[p] * weight : weight;
         }
-        deposit_carried<VEC>(mesh, g, cx, cy, cz, w, carry, on);
+        deposit_carried<VEC, VEC>(mesh, g, cx, cy, cz, w, carry, on);
       },
       [&] {
         deposit_plane_merged<VEC>(mesh, carry.valid, carry.xo, carry.yo0, carry.yo1, carry.z0, carry.z1, carry.w00,
-                             carry.w01, carry.w10, carry.w11);
+                                  carry.w01, carry.w10, carry.w11);
         carry.valid = false;
       });
 }
@@ -350,10 +427,10 @@ __global__ void __launch_bounds__(256) k_readout_force_walk(const float* __restr
   out += b * g.np * 3;
   walk_segments(
       g, walk,
-      [&](unsigned p, int i, int j, int k, bool on) {
+      [&](unsigned p, int i, int j, int k, bool on, int, int) {
         if (!on) return;
         Cic1 cx, cy, cz;
-        cic_at(pos, absolute, g, p, i, j, k, cx, cy, cz);
+        cic_at(position_at(pos, p), absolute, g, i, j, k, cx, cy, cz);
         float fx, fy, fz;
         gather_force_mesh(force, g, cx, cy, cz, fx, fy, fz);
         __stcs(out + 3ull * p + 0, fx);
@@ -1061,14 +1138,17 @@ __global__ void k_axpy(float* __restrict__ y, const float* __restrict__ x, float
 cudaError_t cic_paint(const float* pos, int absolute, const float* weights, float weight, float* mesh,
                       const MeshDims& d, cudaStream_t s) {
   SegWalk w;
-  if (seg_walk(d, &w)) {
-    if (d.nz % 4 == 0 && (uintptr_t)mesh % 16 == 0)
+  const dim3 grid = particle_grid_dims(d.cells(), d.batch, 256, 16);
+  const bool pairs = d.nz % 4 == 0 && (uintptr_t)mesh % 16 == 0;
+  if (d.cells() * d.batch >= kPaintWalkCells && seg_walk(d, &w, 16)) {
+    if (pairs)
       k_paint_walk<true><<<seg_grid(d, w), 256, 0, s>>>(pos, absolute, weights, weight, mesh, make_pgrid(d), w);
     else
       k_paint_walk<false><<<seg_grid(d, w), 256, 0, s>>>(pos, absolute, weights, weight, mesh, make_pgrid(d), w);
+  } else if (pairs) {
+    k_paint_pairs<<<grid, 256, 0, s>>>(pos, absolute, weights, weight, mesh, make_pgrid(d));
   } else {
-    k_paint<<<particle_grid_dims(d.cells(), d.batch, 256, 16), 256, 0, s>>>(pos, absolute, weights, weight, mesh,
-                                                                            make_pgrid(d));
+    k_paint<<<grid, 256, 0, s>>>(pos, absolute, weights, weight, mesh, make_pgrid(d));
   }
   note_launch();
   return cudaGetLastError();
