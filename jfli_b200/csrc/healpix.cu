@@ -485,8 +485,13 @@ __device__ __forceinline__ double shell_position(const float* __restrict__ disp,
   return v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
 }
 
+// CTAs per SM. The rbf weights take 96 registers, two CTAs, unless bounded; with three (80, 32 bytes
+// spilled) 128^3 particles at nside 256 258 -> 229 us, with four (64) 262.
+template <int scheme>
+constexpr int kShellCtas = scheme == 1 ? 4 : (scheme == 2 ? 3 : 2);
+
 template <int scheme, bool any>
-__global__ void __launch_bounds__(256, scheme == 1 ? 4 : 2) k_healpix_paint_shells(const float* __restrict__ disp, int absolute,
+__global__ void __launch_bounds__(256, kShellCtas<scheme>) k_healpix_paint_shells(const float* __restrict__ disp, int absolute,
                                                               const float* __restrict__ weights, float weight, PGrid g,
                                                               double3 cell, double3 obs, ShellSet shells, int nside,
                                                               HealpixTables tb, float* __restrict__ maps, float sigma) {
