@@ -420,15 +420,19 @@ __global__ void __launch_bounds__(kLegendreThreads, kLegendreCtas<RP>) k_sht_syn
 // CTAs do not fill the SMs for long and end on the serial chain of their first m, unless
 // several maps go together. a_lm with three refinements, 2 against 8 pairs: nside 512 5.1 and
 // 4.4 ms, nside 256 0.94 and 1.07 (two maps together 1.72 and 1.60, four 3.26 and 3.08), four of
-// nside 128 0.69 and 0.85.
+// nside 128 0.69 and 0.85. With fewer m than kLegendreFill two pairs as well: C_l at nside 512, lmax 64 648
+// and 694 us, lmax 200 758 and 806; nside 1024, lmax 200 2.69 and 2.67 ms, lmax 280 2.91 and 2.85.
+constexpr int kLegendreFill = 222;
+
 struct LegendreShape {
   int rp, threads, blocks;
 };
 
-static LegendreShape legendre_shape(int nrings, int nmaps) {
+static LegendreShape legendre_shape(int nrings, int lmax, int nmaps) {
   const int pairs = (nrings + 1) / 2;
   LegendreShape s;
-  s.rp = pairs >= 1024 || (pairs >= 512 && nmaps >= 2) ? 8 : 2;
+  const bool fills = (long long)(lmax + 1) * nmaps >= kLegendreFill;
+  s.rp = fills && (pairs >= 1024 || (pairs >= 512 && nmaps >= 2)) ? 8 : 2;
   int warps = (pairs + 32 * s.rp - 1) / (32 * s.rp);
   s.blocks = (warps + kLegendreWarps - 1) / kLegendreWarps;
   warps = (warps + s.blocks - 1) / s.blocks;
@@ -478,7 +482,7 @@ __device__ __forceinline__ double2 phase(int m, int j, int n, double phi0, doubl
   return make_double2(cs, sign * sn);
 }
 
-// Direct sums (nside > kRingFftMax):
+// Direct sums (where ring_fft does not hold):
 // F[r][m] = sum_j f_j e^{-i m phi_j}, m = 0..lmax (aliasing for m >= n is the DFT's own).
 // One block per (ring, 128 m); the ring's values staged in shared memory.
 __global__ void __launch_bounds__(kRingThreads) k_ring_analysis(const double* __restrict__ map, int nside, int lmax,
@@ -545,7 +549,7 @@ __global__ void __launch_bounds__(kRingThreads) k_ring_synthesis(const double2* 
   map[g.start + j] = coef[0].x + 2.0 * acc;
 }
 
-// Rings with 4 nside pixels or fewer, nside <= kRingFftMax, are transformed by an FP64 FFT in
+// Rings with 4 nside pixels or fewer are transformed, where ring_fft holds, by an FP64 FFT in
 // shared memory, one CTA per ring. A ring has n = 4 i pixels; its 2 i complex pairs (f_2j +
 // i f_2j+1) split into two interleaved transforms of length i, which are plain radix-4 ones
 // when i is a power of two and Bluestein convolutions of length M = 2^c >= 2 i - 1 otherwise
@@ -556,9 +560,20 @@ __global__ void __launch_bounds__(kRingThreads) k_ring_synthesis(const double2* 
 // A ring is never mixed with another one: a NaN or a huge value stays in its ring.
 //
 // 1 B200, nside 1024, lmax 3000: analysis 19.4 -> 0.44 ms, synthesis 20.0 -> 0.42 ms against direct
-// sums (npix x lmax terms), which still serve larger nside, whose convolutions (M = 4096 and
-// more, three arrays) do not fit two CTAs per SM.
+// sums (npix x lmax terms). Those still serve larger nside, whose convolutions (M = 4096 and
+// more, three arrays) leave one CTA per SM or none, and few coefficients (ring_fft): a warp of the
+// sums has one per lane, so that their cost goes up every 32. FFT and direct sums, analysis and
+// synthesis, in us: lmax 16, nside 256 26, 25 and 27, 17, 700 307, 131 and 325, 103, 1024 301, 320 and
+// 333, 217; lmax 32, nside 384 77, 74 and 82, 46, 1024 303, 456 and 334, 305; lmax 64, nside 16 5.7, 3.3 and
+// 6.3, 3.5, 64 6.8, 8.0 and 7.4, 5.1, 384 77, 103 and 82, 72, 700 307, 294 and 325, 229.
 constexpr int kRingFftMax = 1024;
+
+// Short rings are bound by the FFT's barriers, belts that are no power of two are convolutions.
+static bool ring_fft(int nside, int lmax) {
+  const bool convolved = (nside & (nside - 1)) != 0;
+  const int least = nside < 64 ? 96 : (!convolved ? 32 : (nside <= 512 ? 64 : 96));
+  return nside <= kRingFftMax && lmax >= least;
+}
 constexpr int kRingFftThreads = 256;
 
 struct RingFft {
@@ -830,7 +845,7 @@ cudaError_t sht_ring_analysis(const double* map, int nside, int lmax, double* F,
   const int nrings = 4 * nside - 1;
   double2* out = reinterpret_cast<double2*>(F);
   cudaError_t e;
-  if (nside <= kRingFftMax) {
+  if (ring_fft(nside, lmax)) {
     const size_t smem = ring_fft_smem(nside);
     e = cudaFuncSetAttribute(k_ring_fft_analysis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -850,7 +865,7 @@ cudaError_t sht_ring_synthesis(const double* G, int nside, int lmax, double* map
   const int nrings = 4 * nside - 1;
   const double2* in = reinterpret_cast<const double2*>(G);
   cudaError_t e;
-  if (nside <= kRingFftMax) {
+  if (ring_fft(nside, lmax)) {
     const size_t smem = ring_fft_smem(nside);
     e = cudaFuncSetAttribute(k_ring_fft_synthesis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -880,7 +895,7 @@ static cudaError_t analysis_launch(const LegendreShape& sh, const double* F, con
 
 cudaError_t sht_analysis(const double* F, const double* z, int nrings, int lmax, double weight, double* alm,
                          cudaStream_t s, int nmaps) {
-  const LegendreShape sh = legendre_shape(nrings, nmaps);
+  const LegendreShape sh = legendre_shape(nrings, lmax, nmaps);
   if (sh.blocks > 1) {  // the blocks of one m add to alm
     const cudaError_t e = cudaMemsetAsync(alm, 0, sizeof(double2) * (size_t)alm_offset(lmax + 1, lmax) * nmaps, s);
     if (e != cudaSuccess) return e;
@@ -891,7 +906,7 @@ cudaError_t sht_analysis(const double* F, const double* z, int nrings, int lmax,
 
 cudaError_t sht_synthesis(const double* alm, const double* z, int nrings, int lmax, double* G, cudaStream_t s,
                           int nmaps) {
-  const LegendreShape sh = legendre_shape(nrings, nmaps);
+  const LegendreShape sh = legendre_shape(nrings, lmax, nmaps);
   const dim3 grid(lmax + 1, sh.blocks, nmaps);
   const double2* a = reinterpret_cast<const double2*>(alm);
   double2* out = reinterpret_cast<double2*>(G);
