@@ -155,21 +155,8 @@ struct XCarry {
   bool valid;
 };
 
-// Deposit, for every lane of a full warp, the 2 (y) x 2 (z) corners of one x plane, with
-// the z lane merge of deposit_lane_merged: when lane L's upper-z pair of cells is lane
-// L+1's lower-z pair (same x and y cells, next z cell), lane L hands its two upper-z
-// weights to lane L+1, which adds them to its own lower-z deposits. Lanes with `on` false
-// deposit nothing and take part in no merge. Cell offsets are unique per cell, so equal
-// offsets mean equal cells.
-//
-// A lane that merges with neither neighbour has two adjacent cells of its own per y row: with VEC
-// (rows of a multiple of 4 cells, mesh 16-byte aligned) they go out as one 16-byte vector
-// atomic with zeros beside them (deposit_pair), unless they lie in two aligned groups of four. On
-// particles that left their neighbours the paint is bound by the atomics' path: the particle
-// pass of 256^3 347 -> 344 us over 40 steps (385 with vectors for every lane, merged or not, as the
-// merged rows' 4-byte atomics coalesce; 364 with 8-byte atomics at even cells); figures of the
-// paint at its kernels. A warp with lanes of both kinds issues both: with LEAST > 0 it does so
-// only from that many lanes of the one kind on.
+// Weights a, b of the two z cells z0, z1 of a row: one 16-byte atomic with zeros beside them (VEC: rows
+// of a multiple of 4 cells, mesh 16-byte aligned) unless they lie in two aligned groups of four.
 template <bool VEC>
 __device__ __forceinline__ void deposit_pair(float* row, int z0, int z1, float a, float b) {
   const int q = z0 & 3;
@@ -183,6 +170,19 @@ __device__ __forceinline__ void deposit_pair(float* row, int z0, int z1, float a
   }
 }
 
+// Deposit, for every lane of a full warp, the 2 (y) x 2 (z) corners of one x plane, with
+// the z lane merge of deposit_lane_merged: when lane L's upper-z pair of cells is lane
+// L+1's lower-z pair (same x and y cells, next z cell), lane L hands its two upper-z
+// weights to lane L+1, which adds them to its own lower-z deposits. Lanes with `on` false
+// deposit nothing and take part in no merge. Cell offsets are unique per cell, so equal
+// offsets mean equal cells.
+//
+// A lane that merges with neither neighbour has two adjacent cells of its own per y row: with VEC
+// they go out by deposit_pair. On particles that left their neighbours the paint is bound by the
+// atomics' path: the particle pass of 256^3 347 -> 344 us over 40 steps (385 with vectors for every lane, merged or not, as the
+// merged rows' 4-byte atomics coalesce; 364 with 8-byte atomics at even cells); figures of the
+// paint at its kernels. A warp with lanes of both kinds issues both: with LEAST > 0 it does so
+// only from that many lanes of the one kind on.
 template <bool VEC, int LEAST = 0>
 __device__ __forceinline__ void deposit_plane_merged(float* rho, bool on, int xo, int yo0, int yo1, int z0, int z1,
                                                      float w00, float w01, float w10, float w11) {
