@@ -66,18 +66,18 @@ def device_table(values, device="cuda", dtype=np.float32) -> torch.Tensor:
     no copy; a new one belongs to that capture alone."""
     global _tables_captured
     a = np.ascontiguousarray(np.asarray(values, dtype=dtype))
-    dev = torch.device(device)
-    stream = capturing = None
+    dev = device if isinstance(device, torch.device) else torch.device(device)
+    index = stream = capturing = None
     if dev.type == "cuda":
         here = torch.cuda.current_device()
-        dev = torch.device("cuda", here if dev.index is None else dev.index)
-        stream = torch._C._cuda_getCurrentRawStream(dev.index)
-        if dev.index == here:
-            capturing = torch.cuda.is_current_stream_capturing()
+        index = here if dev.index is None else dev.index
+        stream = torch._C._cuda_getCurrentRawStream(index)
+        if index == here:
+            capturing = torch._C._cuda_isCurrentStreamCapturing()
         else:
-            with torch.cuda.device(dev):
-                capturing = torch.cuda.is_current_stream_capturing()
-    key = (a.tobytes(), a.shape, a.dtype.str, str(dev))
+            with torch.cuda.device(index):
+                capturing = torch._C._cuda_isCurrentStreamCapturing()
+    key = (a.tobytes(), a.shape, a.dtype.str, index)
     with _tables_lock:
         e = _TABLES.get(key)
         if e is not None:
@@ -86,7 +86,7 @@ def device_table(values, device="cuda", dtype=np.float32) -> torch.Tensor:
                 _tables_captured += not e.captured
                 e.captured = True
             elif stream is not None and stream not in e.streams:
-                s = torch.cuda.current_stream(dev)
+                s = torch.cuda.current_stream(index)
                 s.wait_event(e.event)
                 e.tensor.record_stream(s)
                 e.streams.add(stream)
@@ -95,10 +95,10 @@ def device_table(values, device="cuda", dtype=np.float32) -> torch.Tensor:
         if stream is None:
             e = _Table(t.to(dev), None, None)
         else:
-            t = t.pin_memory().to(dev, non_blocking=True)
+            t = t.pin_memory().to(torch.device("cuda", index), non_blocking=True)
             if capturing:
                 return t
-            e = _Table(t, torch.cuda.current_stream(dev).record_event(), {stream})
+            e = _Table(t, torch.cuda.current_stream(index).record_event(), {stream})
         _TABLES[key] = e
         if len(_TABLES) - _tables_captured > _TABLES_MOST:  # the oldest that no graph reads goes
             del _TABLES[next(k for k, v in _TABLES.items() if not v.captured)]
