@@ -296,7 +296,8 @@ __device__ __forceinline__ void unkick_row(float* __restrict__ disp, bool undrif
 }
 
 constexpr int kAdjBrickY = 8, kAdjBrickZ = 32;
-constexpr int kUnkickCtas = 2;  // resident per SM (128 registers)
+constexpr int kUnkickCtas = 2;        // resident per SM (128 registers)
+constexpr int kUnkickStrideCtas = 3;  // of the grid-stride form (80)
 
 // How walk_columns cuts the columns. Up to 2^22 cells the meshes that are gathered from and painted
 // are in L2, and equal ranges of planes, one per resident CTA, leave no last round (0). Larger
@@ -341,13 +342,14 @@ __device__ __forceinline__ void walk_columns(const PGrid& g, int depth, Run run)
 // walks 8 (y) x 32 (z) columns of Lagrangian cells along x, each warp on one z row (the z merge
 // of the deposit needs consecutive z in a warp), so that the rows and planes whose particles
 // share CIC corners gather and deposit on one SM close in time (as the forward particle
-// pass). Otherwise a grid-stride walk.
+// pass). Otherwise a grid-stride walk, which needs fewer registers: bounded like the column walk,
+// with two CTAs per SM, it took 10.3 us for 48^3 against 9.1 with three (72^3 23.7 and 24.2).
 //
 // Bound by L1 (gathers and atomics of 16 bytes a lane). 128^3: 88 us with pieces of 8 planes over
 // 1184 CTAs (2.3 rounds of the resident ones), 78 with equal ranges, 76.7 with the next row's
 // loads ahead of this one (128 registers, two CTAs per SM), 67 with the x merge of VecCarry.
-template <bool kVec4>
-__global__ void __launch_bounds__(kAdjThreads, kUnkickCtas) k_adj_unkick_paint(
+template <bool kVec4, bool kWalk>
+__global__ void __launch_bounds__(kAdjThreads, kWalk ? kUnkickCtas : kUnkickStrideCtas) k_adj_unkick_paint(
     float* __restrict__ disp, int undrift, float* __restrict__ vel, const float* __restrict__ lam_x,
     float* __restrict__ lam_v, const float* __restrict__ force, float kick, float drift, float* __restrict__ ubar,
     double* __restrict__ partials, PGrid g, int depth) {
@@ -359,8 +361,8 @@ __global__ void __launch_bounds__(kAdjThreads, kUnkickCtas) k_adj_unkick_paint(
   force += b * g.np * 4;
   ubar += b * g.np * (kVec4 ? 4 : 3);
   double sk = 0.0, sd = 0.0;
-  __shared__ float4 rowbuf[kVec4 ? kAdjBrickY : 1][4][24];  // per warp: disp, vel, lam_x, lam_v of one z row
-  if (kVec4 && blockDim.x == kAdjBrickY * kAdjBrickZ && g.nz % kAdjBrickZ == 0 && g.ny % kAdjBrickY == 0) {
+  __shared__ float4 rowbuf[kWalk ? kAdjBrickY : 1][4][24];  // per warp: disp, vel, lam_x, lam_v of one z row
+  if (kWalk) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const bool staged = ((reinterpret_cast<uintptr_t>(disp) | reinterpret_cast<uintptr_t>(vel) |
                           reinterpret_cast<uintptr_t>(lam_x) | reinterpret_cast<uintptr_t>(lam_v)) & 15) == 0;
@@ -380,7 +382,7 @@ __global__ void __launch_bounds__(kAdjThreads, kUnkickCtas) k_adj_unkick_paint(
         const unsigned p = ((unsigned)i * (unsigned)g.ny + (unsigned)j) * (unsigned)g.nz + (unsigned)k;
         if (staged)
           unkick_row<kVec4>(disp, undrift != 0, vel, lam_x, lam_v, force, kick, drift, ubar, g, p - (unsigned)lane,
-                            i, j, k, lane, rowbuf[kVec4 ? w : 0], sk, sd, row, i + 1 < i1,
+                            i, j, k, lane, rowbuf[kWalk ? w : 0], sk, sd, row, i + 1 < i1,
                             carry);
         else
           unkick_particle<kVec4>(disp, undrift != 0, vel, lam_x, lam_v, force, kick, drift, ubar, g, p, i, j, k, sk,
@@ -614,8 +616,11 @@ static dim3 adj_grid(const MeshDims& d) { return particle_grid_dims(d.cells(), d
 
 // The grid of the float4 un-kick, whose partials sum_adjoint_partials adds up: its resident CTAs.
 // No larger than adj_grid, the grid of the other form, all of whose partials the caller sums.
+static bool unkick_walks(const MeshDims& d) { return d.nz % kAdjBrickZ == 0 && d.ny % kAdjBrickY == 0; }
+
 static dim3 unkick_grid(const MeshDims& d) {
-  const long long resident = max(1ll, (long long)kUnkickCtas * sm_count() / d.batch);
+  const int ctas = unkick_walks(d) ? kUnkickCtas : kUnkickStrideCtas;
+  const long long resident = max(1ll, (long long)ctas * sm_count() / d.batch);
   dim3 grid = adj_grid(d);
   if (resident < grid.x) grid.x = (unsigned)resident;
   return grid;
@@ -667,12 +672,16 @@ cudaError_t adjoint_unkick_paint(const float* disp, float* vel, const float* lam
   const int undrift = undrift_disp != nullptr;
   cudaError_t e = cudaMemsetAsync(ubar, 0, sizeof(float) * (vec4 ? 4 : 3) * (size_t)d.cells() * d.batch, s);
   if (e != cudaSuccess) return e;
-  if (vec4)
-    k_adj_unkick_paint<true><<<unkick_grid(d), kAdjThreads, 0, s>>>(dp, undrift, vel, lam_x, lam_v, force, kick, drift,
-                                                                    ubar, partials, make_pgrid(d), walk_depth(d));
+  if (vec4 && unkick_walks(d))
+    k_adj_unkick_paint<true, true><<<unkick_grid(d), kAdjThreads, 0, s>>>(dp, undrift, vel, lam_x, lam_v, force, kick,
+                                                                          drift, ubar, partials, make_pgrid(d),
+                                                                          walk_depth(d));
+  else if (vec4)
+    k_adj_unkick_paint<true, false><<<unkick_grid(d), kAdjThreads, 0, s>>>(dp, undrift, vel, lam_x, lam_v, force, kick,
+                                                                           drift, ubar, partials, make_pgrid(d), 0);
   else
-    k_adj_unkick_paint<false><<<adj_grid(d), kAdjThreads, 0, s>>>(dp, undrift, vel, lam_x, lam_v, force, kick, drift, ubar,
-                                                                  partials, make_pgrid(d), 0);
+    k_adj_unkick_paint<false, false><<<adj_grid(d), kAdjThreads, 0, s>>>(dp, undrift, vel, lam_x, lam_v, force, kick,
+                                                                         drift, ubar, partials, make_pgrid(d), 0);
   note_launch();
   return cudaGetLastError();
 }
