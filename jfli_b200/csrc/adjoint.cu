@@ -436,7 +436,6 @@ cudaError_t paint_vec4(const float* disp, const float* u, float* ubar, const Mes
 __global__ void k_div_fd(const float* __restrict__ u, float alpha, const float* __restrict__ w, float beta,
                          long long cell_stride, long long comp_stride, int accumulate, float* __restrict__ out,
                          PGrid g) {
-  grid_release();
   grid_wait();
   const long long b = blockIdx.y;
   u += b * g.np * (cell_stride == 4 ? 4 : 3);
@@ -480,7 +479,6 @@ constexpr int kDivCtas = 5;  // resident per SM
 __global__ void __launch_bounds__(kAdjThreads, kDivCtas) k_div_march(const float4* __restrict__ u, float alpha,
                                                                      int accumulate, float* __restrict__ out, PGrid g,
                                                                      int depth) {
-  grid_release();
   grid_wait();
   __shared__ float ys[2][kAdjBrickY + 4][kAdjBrickZ];
   __shared__ float zs[2][kAdjBrickY][kAdjBrickZ + 4];
@@ -632,7 +630,6 @@ size_t adjoint_partials_count(const MeshDims& d) { return (size_t)2 * adj_grid(d
 // slice, then a shared-memory tree in a fixed order (deterministic).
 __global__ void __launch_bounds__(256) k_sum_partials(const double* __restrict__ partials, int nctas,
                                                       double* __restrict__ out) {
-  grid_release();
   grid_wait();
   __shared__ double sk[256], sd[256];
   const double* p = partials + 2ll * nctas * blockIdx.x;

@@ -675,7 +675,6 @@ constexpr int kForceMeshThreads = 256;
 
 __global__ void __launch_bounds__(kForceMeshThreads) k_force_mesh4(const float* __restrict__ pot,
                                                                    float* __restrict__ F, float scale, PGrid g) {
-  grid_release();
   grid_wait();
   const long long b = blockIdx.y;
   pot += b * g.np;
@@ -1113,7 +1112,6 @@ __global__ void k_lpt_combine(const float* __restrict__ f1, const float* __restr
 
 // Zero n floats (16-byte stores where the pointer allows; the tail element by element).
 __global__ void k_zero(float* __restrict__ y, long long n) {
-  grid_release();
   grid_wait();
   const long long n4 = ((reinterpret_cast<uintptr_t>(y) & 15) == 0) ? n / 4 : 0;
   float4* y4 = reinterpret_cast<float4*>(y);

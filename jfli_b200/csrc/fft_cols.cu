@@ -54,7 +54,6 @@ __global__ void __launch_bounds__(ColCfg<N>::T) k_cols_reg(float2* __restrict__ 
   float2* ybuf = sm + N;
   data += (long long)blockIdx.y * bstride;
   const int tid = threadIdx.x;
-  grid_release();
   grid_wait();
   for (int m = tid; m < N; m += T) tw[m] = twg[m];
   __syncthreads();
@@ -82,6 +81,7 @@ __global__ void __launch_bounds__(ColCfg<N>::T) k_cols_reg(float2* __restrict__ 
 #pragma unroll
   for (int t = 0; t < P; ++t) u[t] = ybuf[(kb * P + t) * W + c];
   RegDFT<P, SIGN, Q>::run(u, tw);
+  grid_release();
   const int col = c0 + c;
   if (col < g.ncols) {
     float2* dst = data + col_base(g, col) + (long long)kb * g.stride;

@@ -53,7 +53,6 @@ __global__ void __launch_bounds__(PlaneCfg<NY>::T) k_planes_forward(const float*
   using C = PlaneCfg<NY>;
   constexpr int N = C::N, HZ = C::HZ, PZ = C::PZ, QZ = C::QZ, PY = C::PY, QY = C::QY, T = C::T, RS = C::RS, YS = C::YS;
   extern __shared__ float2 sm[];
-  grid_release();
   grid_wait();
   const PlaneSmem<NY> s(sm, twzg, tw2g, twyg);
   float2* tile = s.tile;
@@ -138,6 +137,7 @@ __global__ void __launch_bounds__(PlaneCfg<NY>::T) k_planes_forward(const float*
       tile[(kb * PY + t) * RS + c] = (kb == 0) ? v[it][0] : cmul(v[it][kb], twid<-1>(s.twy, t * kb));
   }
   __syncthreads();
+  grid_release();
   // y, stage 2, to memory
   for (int w = tid; w < HZ * QY; w += T) {
     const int c = w % HZ, kb = w / HZ;
@@ -160,7 +160,6 @@ __global__ void __launch_bounds__(PlaneCfg<NY>::T) k_planes_inverse(const float2
   using C = PlaneCfg<NY>;
   constexpr int N = C::N, HZ = C::HZ, PZ = C::PZ, QZ = C::QZ, PY = C::PY, QY = C::QY, T = C::T, RS = C::RS, YS = C::YS;
   extern __shared__ float2 sm[];
-  grid_release();
   grid_wait();
   const PlaneSmem<NY> s(sm, twzg, tw2g, twyg);
   float2* tile = s.tile;
@@ -226,6 +225,7 @@ __global__ void __launch_bounds__(PlaneCfg<NY>::T) k_planes_inverse(const float2
     }
   }
   __syncthreads();
+  grid_release();
   // z, stage 2, to memory
   for (int w = tid; w < NY * QZ; w += T) {
     const int kb = w % QZ, r = w / QZ;

@@ -108,7 +108,6 @@ __global__ void __launch_bounds__(ColCfg<N>::T) k_x_op_tma(const __grid_constant
   const int batch = blockIdx.y;
   const int tid = threadIdx.x;
   const int c0 = blockIdx.x * W;
-  grid_release();
   if (tid == 0) mbar_init(&bar, 1);
   grid_wait();
   if (tid == 0) {
@@ -157,6 +156,7 @@ __global__ void __launch_bounds__(ColCfg<N>::T) k_x_op_tma(const __grid_constant
 #pragma unroll
   for (int k1 = 0; k1 < P; ++k1) ybuf[(k1 * Q + kb) * W + c] = (k1 == 0) ? u[0] : cmul(u[k1], twid<1>(tw, kb * k1));
   __syncthreads();
+  grid_release();
   // inverse stage 2' into the tile
   for (int w = tid; w < W * P; w += T) {
     const int cc = w % W, k1 = w / W;

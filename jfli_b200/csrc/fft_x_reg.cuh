@@ -17,7 +17,6 @@ __global__ void __launch_bounds__(ColCfg<N>::T) k_x_op_reg(float2* __restrict__ 
   const int batch = blockIdx.y;
   data += (long long)batch * bstride;
   const int tid = threadIdx.x;
-  grid_release();
   grid_wait();
   for (int m = tid; m < N; m += T) tw[m] = twg[m];
   op.prologue(opsm, batch);  // ends with __syncthreads()
@@ -63,6 +62,7 @@ __global__ void __launch_bounds__(ColCfg<N>::T) k_x_op_reg(float2* __restrict__ 
     for (int k1 = 0; k1 < P; ++k1)
       ybuf[(k1 * Q + kb) * W + c] = (k1 == 0) ? u[0] : cmul(u[k1], twid<1>(tw, kb * k1));
     __syncthreads();
+    grid_release();
     // inverse stage 2': items (c, k1), k1 < P
     for (int w = tid; w < W * P; w += T) {
       const int cc = w % W, k1 = w / W;

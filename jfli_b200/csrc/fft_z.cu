@@ -169,7 +169,6 @@ __global__ void __launch_bounds__(RowCfg<N>::T) k_rfft_z_reg(const float* in, fl
   out += (long long)blockIdx.y * out_b;
   if (clear) clear += (long long)blockIdx.y * in_b;
   const int tid = threadIdx.x;
-  grid_release();
   grid_wait();
   for (int m = tid; m < N; m += T) tw[m] = twg[m];
   for (int m = tid; m <= N; m += T) tw2[m] = twg2[m];
@@ -218,6 +217,7 @@ __global__ void __launch_bounds__(RowCfg<N>::T) k_rfft_z_reg(const float* in, fl
     const float2 o = make_float2(0.5f * d.y, -0.5f * d.x);
     return cadd(e, cmul(w, o));
   };
+  grid_release();
   constexpr int H = N / 2 + 1;
   for (int w = tid; w < R * H; w += T) {
     const int rr = w / H;
@@ -256,7 +256,6 @@ __global__ void __launch_bounds__(RowCfg<N>::T) k_irfft_z_reg(const float2* __re
   const int row0 = blockIdx.x * R;
   const int have = min(R, nrows - row0) * (N + 1);  // rows past the last are not read
   const float2* src = in + (long long)row0 * (N + 1);
-  grid_release();
   grid_wait();
   if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
     for (int w = tid; w < have / 2; w += T) copy_async<16>(xbuf + 2 * w, src + 2 * w);
@@ -303,6 +302,7 @@ __global__ void __launch_bounds__(RowCfg<N>::T) k_irfft_z_reg(const float2* __re
 #pragma unroll
   for (int t = 0; t < P; ++t) u[t] = ybuf[r * S + t * YS + kb];
   RegDFT<P, 1, Q>::run(u, tw);
+  grid_release();
   if (row < nrows) {
     float2* dst = reinterpret_cast<float2*>(out) + (long long)row * N + kb;
 #pragma unroll
