@@ -153,7 +153,7 @@ def maps2alm(maps, lmax: int | None = None, iter: int = 3):
     packed a_lm."""
     nside = _nside_of(int(maps.shape[-1]))
     lmax = 3 * nside - 1 if lmax is None else int(lmax)
-    step = max(1, _BATCH_BYTES // (16 * (4 * nside - 1) * (lmax + 1)))
+    step = min(max(1, _BATCH_BYTES // (16 * (4 * nside - 1) * (lmax + 1))), 65535)  # maps per launch
     alms = []
     for first in range(0, len(maps), step):
         md = _device_map(maps[first:first + step])
