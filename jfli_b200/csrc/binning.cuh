@@ -35,7 +35,7 @@ struct BinCursor {
   __device__ __forceinline__ bool holds(float x) const { return bin >= 0 && x >= lo && x < hi; }
   // move to x's bin; the next one up is tried before the search
   __device__ __forceinline__ void move(float x, const float* edges, int nedges) {
-    if (bin >= 0 && x >= hi && (bin + 1 == nedges || x < edges[bin + 1]))
+    if (bin >= 0 && bin < nedges && x >= hi && (bin + 1 == nedges || x < edges[bin + 1]))
       ++bin;
     else
       bin = digitize(x, edges, nedges);
