@@ -1,4 +1,4 @@
-// Binned FP64 sums of the power-spectrum kernels (fft.cu, poles.cu).
+// Binned FP64 sums of the power-spectrum kernels (PkTile in kspace_ops.cuh for fft_pk.cu, poles.cu).
 //
 // A thread walks modes whose |k| changes slowly (successive kz columns at one kx, or
 // successive ky at one kz), keeps the sums of the current bin in registers and adds them to
@@ -32,15 +32,16 @@ struct BinCursor {
   int bin = -1;  // -1: none yet
   float lo, hi;
 
-  __device__ __forceinline__ bool holds(float x) const { return bin >= 0 && x >= lo && x < hi; }
+  // The last bin has no upper edge (NaN): it holds infinity too, and move never looks past it.
+  __device__ __forceinline__ bool holds(float x) const { return bin >= 0 && x >= lo && !(x >= hi); }
   // move to x's bin; the next one up is tried before the search
   __device__ __forceinline__ void move(float x, const float* edges, int nedges) {
-    if (bin >= 0 && bin < nedges && x >= hi && (bin + 1 == nedges || x < edges[bin + 1]))
+    if (bin >= 0 && x >= hi && (bin + 1 == nedges || x < edges[bin + 1]))
       ++bin;
     else
       bin = digitize(x, edges, nedges);
     lo = bin > 0 ? edges[bin - 1] : -INFINITY;
-    hi = bin < nedges ? edges[bin] : INFINITY;
+    hi = bin < nedges ? edges[bin] : NAN;
   }
 };
 
