@@ -98,7 +98,6 @@ template <int N, class Op>
 __global__ void __launch_bounds__(ColCfg<N>::T) k_x_op_tma(const __grid_constant__ CUtensorMap map, ColGeom g,
                                                            const float2* __restrict__ twg, Op op) {
   constexpr int P = Split<N>::P, Q = Split<N>::Q, W = ColCfg<N>::W, T = ColCfg<N>::T;
-  static_assert(Op::kInverse, "the TMA x pass writes the inverse-transformed tile back");
   extern __shared__ __align__(128) unsigned char smraw[];
   float2* tile = reinterpret_cast<float2*>(smraw);
   float2* ybuf = tile + N * W;
@@ -150,7 +149,6 @@ __global__ void __launch_bounds__(ColCfg<N>::T) k_x_op_tma(const __grid_constant
     for (int ka = 0; ka < P; ++ka) u[ka] = op.apply(u[ka], kb + Q * ka, ky, kz, opsm, batch);
   }
   __syncthreads();
-  op.epilogue(opsm, batch, blockIdx.x, gridDim.x);
   // inverse stage 1': t' = kb holds x'[t' + Q m'] = u[m'], m' < P
   RegDFT<P, 1, Q>::run(u, tw);
 #pragma unroll

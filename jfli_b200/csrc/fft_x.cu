@@ -12,8 +12,8 @@ namespace jfli {
 
 // ---------------------------------------------------------------------------------
 // x pass with a k-space operator. Columns are (ky, kz) pairs, c = ky*hz + kz, and the
-// transform runs over kx with stride ny*hz. Op decides what happens between the
-// forward and the (optional) inverse transform.
+// transform runs over kx with stride ny*hz. Op is applied between the forward and the
+// inverse transform.
 // ---------------------------------------------------------------------------------
 template <class Op>
 __global__ void __launch_bounds__(kFftThreads) k_fft_x_op(float2* __restrict__ data, ColGeom g, FftPlan pl, Op op,
@@ -46,14 +46,11 @@ __global__ void __launch_bounds__(kFftThreads) k_fft_x_op(float2* __restrict__ d
     }
   }
   __syncthreads();
-  op.epilogue(opsm, batch, blockIdx.x, gridDim.x);
-  if (Op::kInverse) res = tile_fft<1>(res, res == bufa ? bufb : bufa, g.w, wl, pl, tw);
-  if (Op::kStore) {
-    for (int idx = threadIdx.x; idx < E; idx += blockDim.x) {
-      const int e = idx >> wl;
-      const int c = c0 + (idx & (g.w - 1));
-      if (c < g.ncols) data[(long long)c + (long long)e * g.stride] = res[idx];
-    }
+  res = tile_fft<1>(res, res == bufa ? bufb : bufa, g.w, wl, pl, tw);
+  for (int idx = threadIdx.x; idx < E; idx += blockDim.x) {
+    const int e = idx >> wl;
+    const int c = c0 + (idx & (g.w - 1));
+    if (c < g.ncols) data[(long long)c + (long long)e * g.stride] = res[idx];
   }
 }
 
@@ -121,22 +118,20 @@ static cudaError_t x_op_tma(float2* data, const MeshDims& d, const Op& op, bool*
 template <class Op>
 static cudaError_t x_op(float2* data, const MeshDims& d, const Op& op, cudaStream_t s, bool mixed) {
   const ColGeom g = x_geom(d);
-  if constexpr (Op::kInverse) {
-    if (x_pass_mode() == 1) {
-      bool done = false;
-      cudaError_t e = cudaSuccess;
-      switch (g.n) {
-#define JFLI_CASE(N_)                              \
-  case N_:                                         \
-    e = x_op_tma<N_, Op>(data, d, op, &done, s);   \
+  if (x_pass_mode() == 1) {
+    bool done = false;
+    cudaError_t e = cudaSuccess;
+    switch (g.n) {
+#define JFLI_CASE(N_)                            \
+  case N_:                                       \
+    e = x_op_tma<N_, Op>(data, d, op, &done, s); \
     break;
-        JFLI_REG_SIZES(JFLI_CASE)
+      JFLI_REG_SIZES(JFLI_CASE)
 #undef JFLI_CASE
-        default:
-          break;
-      }
-      if (e != cudaSuccess || done) return e;
+      default:
+        break;
     }
+    if (e != cudaSuccess || done) return e;
   }
   switch (g.n) {
 #define JFLI_CASE(N_) \

@@ -54,34 +54,24 @@ __global__ void __launch_bounds__(ColCfg<N>::T) k_x_op_reg(float2* __restrict__ 
     for (int ka = 0; ka < P; ++ka) u[ka] = op.apply(u[ka], kb + Q * ka, ky, kz, opsm, batch);
   }
   __syncthreads();
-  op.epilogue(opsm, batch, blockIdx.x, gridDim.x);
-  if (Op::kInverse) {
-    // inverse stage 1': t' = kb holds x'[t' + Q m'] = u[m'], m' < P
-    RegDFT<P, 1, Q>::run(u, tw);
+  // inverse stage 1': t' = kb holds x'[t' + Q m'] = u[m'], m' < P
+  RegDFT<P, 1, Q>::run(u, tw);
 #pragma unroll
-    for (int k1 = 0; k1 < P; ++k1)
-      ybuf[(k1 * Q + kb) * W + c] = (k1 == 0) ? u[0] : cmul(u[k1], twid<1>(tw, kb * k1));
-    __syncthreads();
-    grid_release();
-    // inverse stage 2': items (c, k1), k1 < P
-    for (int w = tid; w < W * P; w += T) {
-      const int cc = w % W, k1 = w / W;
-      const int col2 = c0 + cc;
-      float2 v[Q];
+  for (int k1 = 0; k1 < P; ++k1) ybuf[(k1 * Q + kb) * W + c] = (k1 == 0) ? u[0] : cmul(u[k1], twid<1>(tw, kb * k1));
+  __syncthreads();
+  grid_release();
+  // inverse stage 2': items (c, k1), k1 < P
+  for (int w = tid; w < W * P; w += T) {
+    const int cc = w % W, k1 = w / W;
+    const int col2 = c0 + cc;
+    float2 v[Q];
 #pragma unroll
-      for (int t = 0; t < Q; ++t) v[t] = ybuf[(k1 * Q + t) * W + cc];
-      RegDFT<Q, 1, P>::run(v, tw);
-      if (col2 < g.ncols) {
-        float2* dst = data + col2 + (long long)k1 * g.stride;
+    for (int t = 0; t < Q; ++t) v[t] = ybuf[(k1 * Q + t) * W + cc];
+    RegDFT<Q, 1, P>::run(v, tw);
+    if (col2 < g.ncols) {
+      float2* dst = data + col2 + (long long)k1 * g.stride;
 #pragma unroll
-        for (int k2 = 0; k2 < Q; ++k2) dst[(long long)(P * k2) * g.stride] = v[k2];
-      }
-    }
-  } else if (Op::kStore) {
-    if (col < g.ncols) {
-      float2* dst = data + col + (long long)kb * g.stride;
-#pragma unroll
-      for (int ka = 0; ka < P; ++ka) dst[(long long)(Q * ka) * g.stride] = u[ka];
+      for (int k2 = 0; k2 < Q; ++k2) dst[(long long)(P * k2) * g.stride] = v[k2];
     }
   }
 }

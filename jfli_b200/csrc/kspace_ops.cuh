@@ -19,8 +19,6 @@ __device__ __forceinline__ float k_rad_per_cell(int i, int n) {
 // Poisson potential: pot_k = delta_k * (-1/k^2) * norm, k = 0 -> 0.
 // Follows JaxPM `invlaplace_kernel` (reference call site pm/solvers.py:22 via pm_forces).
 struct PoissonOp {
-  static constexpr bool kInverse = true;
-  static constexpr bool kStore = true;
   int nx, ny, nz;
   float norm;
   static size_t smem_bytes(const PoissonOp& op) { return sizeof(float) * op.nx; }
@@ -38,7 +36,6 @@ struct PoissonOp {
     const float g = (kk == 0.f) ? 0.f : -1.f / kk;
     return cscale(v, g * norm);
   }
-  __device__ void epilogue(float*, int, int, int) const {}
 };
 
 // PGD short-range potential (reference pm/correction.py:177-189), optionally mixed with the
@@ -48,8 +45,6 @@ struct PoissonOp {
 // is a reversible step's kick plus SharpeningKernel's velocity boost at the same positions
 // (reference pm/solvers.py:292-318, pm/correction.py:214-333).
 struct PgdOp {
-  static constexpr bool kInverse = true;
-  static constexpr bool kStore = true;
   int nx, ny, nz;
   float norm, kl2, ks4;
   float c0 = 0.f, c1 = 1.f;
@@ -69,7 +64,6 @@ struct PgdOp {
     const float range = expf(-kl2 / kk) * expf(-(kk * kk) / ks4);
     return cscale(v, (-1.f / kk) * (c0 + c1 * range) * norm);
   }
-  __device__ void epilogue(float*, int, int, int) const {}
 };
 
 // Linear interpolation with end extrapolation on a tabulated P(k), the behaviour of
@@ -112,8 +106,6 @@ __device__ __forceinline__ float interp_table_d(float x, const float* xp, const 
 // field_k *= sqrt(P(|k|) * M / V) * norm, |k| in h/Mpc. `zero_mode_one` reproduces the
 // k = 0 guard of infer/dist.py:68.
 struct IcOp {
-  static constexpr bool kInverse = true;
-  static constexpr bool kStore = true;
   int nx, ny, nz;
   const float* ktab;
   const float* ptab;
@@ -202,7 +194,6 @@ struct IcOp {
     if (zero_mode_one && kmag == 0.f) pk = 1.f;
     return cscale(v, sqrtf(pk) * norm);
   }
-  __device__ void epilogue(float*, int, int, int) const {}
 };
 
 // Power spectrum histogram (reference _src/power/_compute.py:23-119): |delta_k|^2 with
@@ -379,8 +370,6 @@ constexpr int kMaxAdjPoles = 8;
 // 1) each, of a complex per-bin factor c; the Hermitian part of c w(k) is the multiplier:
 // Re(c) (w(k) + w(partner)) / 2 + i Im(c) (w(k) - w(partner)) / 2.
 struct PkAdjOp {
-  static constexpr bool kInverse = true;
-  static constexpr bool kStore = true;
   int nx, ny, nz;
   const float* kedges;
   const float* weights;  // nedges + 1
@@ -430,7 +419,6 @@ struct PkAdjOp {
     if (!cplx) return cscale(v, w * norm);
     return make_float2((v.x * w - v.y * wo) * norm, (v.x * wo + v.y * w) * norm);
   }
-  __device__ void epilogue(float*, int, int, int) const {}
 };
 
 }  // namespace jfli
