@@ -402,7 +402,7 @@ int jfli_born_flat(void* stream, const float* maps, int nplanes, int n0, int n1,
  *   jfli_sht_ring_analysis:  F[r][m] = sum_j map_j e^{-i m phi_j},  m = 0..lmax
  *   jfli_sht_ring_synthesis: map_j = Re G[r][0] + 2 sum_{m=1..lmax} Re(G[r][m] e^{i m phi_j})
  * FP64 FFTs of each ring (any ring length) up to nside 1024, direct FP64 sums (phases exact
- * every 64 terms) above. nside <= 4096, lmax <= 8191. */
+ * every 64 terms) above and for few m (lmax < 32 to 96, by nside). nside <= 4096, lmax <= 8191. */
 int jfli_sht_ring_analysis(void* stream, const double* map, int nside, int lmax, double* F, char* err,
                            size_t errlen);
 int jfli_sht_ring_synthesis(void* stream, const double* G, int nside, int lmax, double* map, char* err,

@@ -83,6 +83,8 @@ inline int reg_col_w(int n, bool first = false) {
 // gradient of a 108^3 or 144^3 run through 12 to 20 steps moves by 5e-5 to 4e-4 of its norm, where
 // repeats of one build differ by 2e-6 to 7e-5 (atomics). In the solves of the steps and of the
 // reverse sweep, where the atomics reorder the density anyway, it moves by no more than that.
+// The LPT adjoint places no particle and takes the register passes (its phi1 then rounds apart from
+// the forward call's, 3e-7).
 inline int reg_fft_length(int n, bool mixed) {
   if (mixed) return n;
   switch (n) {

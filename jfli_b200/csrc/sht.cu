@@ -181,11 +181,12 @@ struct RingPairs {
 // two of four 4.3 and 3.6; with the tables per super-tile 3.6 and 3.4).
 constexpr int kLegendreThreads = 32 * kLegendreWarps;
 template <int RP>
-constexpr int kLegendreCtas = RP == 8 ? 3 : 6;  // resident per SM (168 and 80 registers)
+constexpr int kLegendreCtas = RP == 8 ? 3 : 6;  // resident per SM by registers (168 and 80)
 
 // Analysis: a thread's sums over its pairs go through shared memory, 16 l at a time per warp: a
 // lane stores one value per l and afterwards adds up half a row (the lanes of one l), so the
 // reduction over a warp's rings costs four instructions per l.
+// Its rows, part and tables take 44 KB with four warps, so that five CTAs of RP = 2 fit an SM.
 template <int RP>
 __global__ void __launch_bounds__(kLegendreThreads, kLegendreCtas<RP>) k_sht_analysis(const double2* __restrict__ F,
                                                                    const double* __restrict__ z, int nrings, int lmax,
@@ -442,7 +443,10 @@ static LegendreShape legendre_shape(int nrings, int lmax, int nmaps) {
 
 // ---- ring transforms along phi ------------------------------------------------------
 // RING geometry of ring r (0 = northernmost, i = r + 1): pixel count, first pixel, and the
-// longitude of the first pixel centre (Gorski et al. 2005).
+// longitude of the first pixel centre, by which the transforms have phi. In the belt it is half a
+// pixel from the painters' pixel centres (Gorski et al. 2005; ring_info_tab) on every ring, 0 where
+// they have pi / (4 nside) and the other way around: C_l of a painted map falls short from l ~
+// nside on (tests/test_sht_longitudes.py).
 struct RingPhi {
   long long start;
   int n;

@@ -532,7 +532,7 @@ class SphericalDensity(AbstractField):
                    batch_size=None) -> PowerSpectrum:
         """C_ell of each map, auto or cross with mesh2 (reference fields/lightcone.py:632-674):
         healpy's anafast algorithm in this library's GPU engine (ring transforms and
-        Legendre stages in FP64)."""
+        Legendre stages in FP64), with a known defect from l ~ nside on (jfli_b200/sht.py)."""
         from .power import angular_cl_spherical, angular_cls_spherical
 
         d1 = self.array

@@ -12,6 +12,9 @@ library's FP64 kernels:
   `jfli_sht_alm2map`, `jfli_sht_ring_synthesis`);
 * healpy's default iterative refinement (iter=3): a += map2alm(map - alm2map(a));
 * C_l = (Re a_l0 b_l0* + 2 sum_{m>0} Re a_lm b_lm*) / (2l + 1) (`jfli_sht_alm2cl`).
+Known defect: the longitudes of the belt rings are half a pixel off those of the painters' maps
+(ring_geometry), so that C_l of a painted map falls short from l ~ nside on: of a single harmonic
+(l, m) at nside 16 it keeps 0.98 of its power at (4, 3), 0.89 at (12, 8), 0.50 at (20, 16), 0.04 at (30, 28).
 lambda_lm are the orthonormal associated Legendre functions with the Condon-Shortley
 phase (three-term recursion in l at fixed m, lambda_mm formed in log space).
 """
@@ -25,7 +28,9 @@ import torch
 
 
 def ring_geometry(nside: int):
-    """(z, n_pix, phi0, start) per ring, RING ordering, north to south."""
+    """(z, n_pix, phi0, start) per ring, RING ordering, north to south. phi0 in the belt is half a
+    pixel from the painters' pixel centres on every ring (0 where they have pi / (4 nside), and
+    the other way around), as in the kernels."""
     nr = 4 * nside - 1
     z = np.empty(nr)
     npr = np.empty(nr, np.int64)

@@ -31,7 +31,8 @@ import numpy as np
 
 
 def ring_geometry(nside: int):
-    """(z, n_pix, phi0, start) per ring, RING ordering, north to south."""
+    """(z, n_pix, phi0, start) per ring, RING ordering, north to south (phi0 of the belt as the kernels
+    have it, half a pixel from pix2ang's centres)."""
     nr = 4 * nside - 1
     z = np.empty(nr)
     npr = np.empty(nr, np.int64)
