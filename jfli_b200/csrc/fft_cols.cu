@@ -76,12 +76,12 @@ __global__ void __launch_bounds__(ColCfg<N>::T) k_cols_reg(float2* __restrict__ 
       ybuf[(kb * P + t) * W + c] = (kb == 0) ? u[0] : cmul(u[kb], twid<SIGN>(tw, t * kb));
   }
   __syncthreads();
+  grid_release();
   const int c = tid % W, kb = tid / W;
   float2 u[P];
 #pragma unroll
   for (int t = 0; t < P; ++t) u[t] = ybuf[(kb * P + t) * W + c];
   RegDFT<P, SIGN, Q>::run(u, tw);
-  grid_release();
   const int col = c0 + c;
   if (col < g.ncols) {
     float2* dst = data + col_base(g, col) + (long long)kb * g.stride;

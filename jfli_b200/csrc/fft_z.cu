@@ -296,13 +296,13 @@ __global__ void __launch_bounds__(RowCfg<N>::T) k_irfft_z_reg(const float2* __re
       ybuf[r * S + t * YS + kb] = (kb == 0) ? u1[it][0] : cmul(u1[it][kb], conjf2(RowSmem<N>::kStaged ? tws[(kb - 1) * P + t] : tw[t * kb]));
   }
   __syncthreads();
+  grid_release();
   const int kb = tid % Q, r = tid / Q;
   const int row = row0 + r;
   float2 u[P];
 #pragma unroll
   for (int t = 0; t < P; ++t) u[t] = ybuf[r * S + t * YS + kb];
   RegDFT<P, 1, Q>::run(u, tw);
-  grid_release();
   if (row < nrows) {
     float2* dst = reinterpret_cast<float2*>(out) + (long long)row * N + kb;
 #pragma unroll

@@ -26,7 +26,7 @@
 namespace jfli {
 
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;"); }
 
 // Whether a pass over `cells` cells (of all meshes of a batch) starts before its predecessor has
 // ended: below 2^24, where a pass takes 3 to 30 us and the meshes of a step are in L2. Above,
